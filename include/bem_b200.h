@@ -128,8 +128,8 @@ int bem_boundary_matrices_vk(const void* geom, float k, void* v_out, void* k_out
                              float k_coeff, bem_stream_t stream);
 
 /* Batched fused assembly: many problems (meshes of any size, each with its
- * own wavenumber) in one persistent launch whose CTAs drain a single queue of
- * (problem, 32 test triangles, trial-tile chunk) work items, plus one launch
+ * own wavenumber) in one persistent launch whose warps drain a single queue of
+ * (problem, run of triangle pairs) work items, plus one launch
  * per touching-pair type over all problems.  `problems` is a HOST array;
  * every v_out / k_out must be non-NULL (nv x nv complex64, overwritten with V
  * and mass_coeff M + k_coeff K).  Workspace: bem_batch_workspace_bytes.
@@ -181,7 +181,7 @@ int bem_assembly_status(bem_stream_t stream);
 /* Launch-shape knobs of the assembly kernels, set by the autotuner
  * (0 = automatic).  Process-wide. */
 enum {
-  BEM_TUNE_ASSEMBLY_CHUNK = 1,      /* trial tiles (16 triangles) per work item */
+  BEM_TUNE_ASSEMBLY_CHUNK = 1,      /* trial blocks (32 triangles) per work item */
   BEM_TUNE_ASSEMBLY_CTAS_PER_SM = 2, /* persistent CTAs per SM (<= occupancy limit) */
   BEM_TUNE_TC_PROMOTE = 3,           /* tensor-core matvec: K blocks (64 reals) accumulated in tensor
                                         memory before the partial sum leaves it (0: automatic) */

@@ -8,8 +8,8 @@ batch runner changes how the work reaches the GPU:
   problem's matrices are released before the next wave), so a batch larger
   than HBM streams through it;
 * the assembly of a whole wave is ONE persistent launch of the regular-pair
-  kernel (CTAs drain a single queue of (problem, test group, trial chunk)
-  items, so a 320-triangle mesh and a 20 480-triangle mesh share the GPU
+  kernel (its warps drain a single queue of (problem, run of triangle
+  pairs) items, so a 320-triangle mesh and a 20 480-triangle mesh share the GPU
   without launch-per-problem overhead) plus one launch per touching-pair
   type (``bem_batch_matrices_vk``);
 * the solves of a wave run concurrently, one CUDA stream per worker thread,

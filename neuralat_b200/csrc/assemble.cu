@@ -14,21 +14,21 @@
 //   * one pass evaluates each quadrature-point pair once for BOTH operators
 //     (shared r, rsqrt and sincos), with the 6-point rule's constant weights
 //     folded into immediate FMA operands;
-//   * V and K together (regular_sym_kernel): each unordered pair once, a
-//     CTA owns one 16-triangle test tile (lane & 15) and sweeps the trial
-//     tiles at or after it, two trial triangles per warp, tiles
-//     double-buffered by bulk copies, two CTAs per SM; one operator alone
-//     (regular_vk_kernel): a CTA owns 32 test triangles (one per lane) x one
-//     16-triangle trial tile, the 8 warps broadcasting their trial triangles
-//     from shared memory;
-//   * pair blocks go to a shared-memory "corner" slab (test corner x trial
-//     corner) and are reduced on chip onto the tile's distinct vertices, so
-//     each matrix entry receives ~0.8 vector atomics per triangle pair instead
-//     of the reference's 18 scalar atomics;
+//   * V and K together (regular_strip_vk_kernel): each unordered pair once, a
+//     warp walks a 32-triangle test block (one triangle per lane) along the
+//     trial triangles and sums their columns in registers (strip.cuh); one
+//     operator alone (regular_vk_kernel): a CTA owns 32 test triangles (one
+//     per lane) x one 16-triangle trial tile, the 8 warps broadcasting their
+//     trial triangles from shared memory, and pair blocks go to a
+//     shared-memory "corner" slab (test corner x trial corner);
+//   * both reduce the corners on chip onto distinct vertices, so each matrix
+//     entry receives about one vector atomic per triangle pair instead of the
+//     reference's 18 scalar atomics;
 //   * touching pairs are masked out of the regular pass and integrated by
 //     separate Sauter-Schwab kernels (coincident pairs in FP64), one warp per
 //     pair over a precomputed pair list (no O(T^2) adjacency scan).
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -36,6 +36,7 @@
 
 #include "async_copy.cuh"
 #include "bem_common.cuh"
+#include "strip.cuh"
 
 namespace bemb {
 
@@ -298,27 +299,29 @@ __global__ void __launch_bounds__(kRegThreads, 2)
 //   V_ji = V_ij^T,
 //   K_ij uses the trial plane of j (dn_j(p) = n_j . (c_j - x_p)),
 //   K_ji uses the plane of i at the trial points (dn_i(q) = n_i . (c_i - y_q)),
-// both from the same r, sincos and kernel values.  A work item is one test
-// tile (16 triangles, test triangle = lane & 15) against a chunk of trial
-// tiles at or after it; on the test tile itself only pairs j > i.  Each of
-// the 8 warps takes two trial triangles (one per half-warp); the test points
-// are staged structure-of-arrays in shared memory.  The slabs fit two CTAs
-// per SM, so one CTA's reduction and barriers overlap the other's evaluation.
+// both from the same r, sincos and kernel values, on a warp's strip walk
+// (strip.cuh).
+//
+// Bound by the FP32 pipe.  The rule is symmetric, w_q phi_b(q) = common(q) +
+// own(q) [b = own vertex of q], so with g_b and h_b the values at the two
+// points of vertex b the trial sums are
+//   t_b = own_1 (g_b + rho h_b) + common_1 sum_c (g_c + sigma h_c),
+// and likewise over the test points: one sum per own vertex and one common
+// sum, combined when a column is flushed.  About 37 FP32-pipe operations per
+// point pair against 42 for weights applied point by point.  The arithmetic
+// runs on packed pairs (the two points of a trial vertex): the same rounding
+// as scalar operations in fewer issued instructions.
+//
+// Measured on B200 with 20 480 triangles: 13.3 ms (both operators; FP32 pipe
+// 61 % of its cycles, issue 61 %), of which 1.6 ms are the column reductions,
+// against 19.0 ms for 16 x 16-triangle tiles whose 3 x 3 blocks all went
+// through shared memory between block barriers.  Two CTAs of four warps per SM
+// with everything unrolled (no spills) take 14.6 ms for the whole assembly;
+// three CTAs at 168 registers 15.1 ms, four at 128 registers 18.2 ms (spills).
 // ---------------------------------------------------------------------------
-constexpr int kSymThreads = 16 * kTile;         // 256: warp w takes trial triangles 2w, 2w + 1
-constexpr int kSymTest = kTile;                 // test triangles per CTA (one tile)
-constexpr int kSymCorners = 3 * kSymTest;       // 48
-
-struct SymSmem {
-  float2 slotV[kSymCorners][kSlotStride];
-  float2 slotK[kSymCorners][kSlotStride];
-  float2 slotM[kSymCorners][kSlotStride];  // K_ji^T, indexed like slotK
-  float xs[18][kSymTest];                  // test quadrature points, [coordinate][tl]
-  TriRec trial[2][kTile];                  // trial tile records, double-buffered
-  TileRec tileJ[2];
-  TileRec tileI;
-  uint64_t tile_full[2];                   // bulk-copy completion of each trial buffer
-};
+constexpr float kRho = (float)(tri6_w_own(3) / tri6_w_own(0));
+constexpr float kSigma = (float)(tri6_w_common(3) / tri6_w_common(0));
+constexpr float kTau = (float)(tri6_w_common(0) / tri6_w_own(0));
 
 // A bounded wait of the assembly kernels expired somewhere in this process
 // (read and cleared by bem_assembly_status).  The waits themselves check the
@@ -326,283 +329,151 @@ struct SymSmem {
 // one geometry does not affect assemblies of other geometries.
 __device__ int g_asm_err;
 
-// Thread 0: bulk-copy trial tile jt (records and vertex table) into buffer b.
-__device__ __forceinline__ void sym_fetch_tile(SymSmem& sm, const GeomView& g, int jt, int b) {
-  const int ntri = min(kTile, g.nt - jt * kTile);
-  const uint32_t rec_bytes = (uint32_t)(ntri * sizeof(TriRec));
-  mbar_expect_tx(&sm.tile_full[b], rec_bytes + (uint32_t)sizeof(TileRec));
-  bulk_load(sm.trial[b], &g.rec[jt * kTile], rec_bytes, &sm.tile_full[b]);
-  bulk_load(&sm.tileJ[b], &g.tiles[jt], (uint32_t)sizeof(TileRec), &sm.tile_full[b]);
-}
+using VkWarp = StripWarp<18, false>;
 
-// aV, aK as pair_block; aM[3a+b] = sum_pq C_ap C_bq dn_i(q) Gk(r_pq) = K_ji[b][a].
-// The arithmetic runs on packed FP32 pairs: the complex accumulations as
-// (re, im) pairs and the distance computation for two trial points at once,
-// with the same operations and rounding as the scalar form (bit-identical),
-// in about half the issued instructions; rsqrt and sin/cos stay scalar.
-__device__ __forceinline__ void pair_block_sym(const float (*xs)[kSymTest], int tl, const float (&yq)[18],
-                                               const float (&dq)[6], float njx, float njy, float njz, float cjx,
-                                               float cjy, float cjz, float k, float2 (&aV)[9], float2 (&aK)[9],
-                                               float2 (&aM)[9]) {
+struct VkStrip {
+  float k, v_scale, k_scale;
+  float2* V;
+  float2* K;
+  // sums of the open columns: own-vertex part [3 a + b] and common part [b]
+  // of V_ij, K_ij and K_ji^T
+  float2 eV[9], eK[9], eM[9], cV[3], cK[3], cM[3];
+
+  __device__ __forceinline__ void clear() {
 #pragma unroll
-  for (int e = 0; e < 9; e++) {
-    aV[e] = make_float2(0.f, 0.f);
-    aK[e] = make_float2(0.f, 0.f);
-    aM[e] = make_float2(0.f, 0.f);
+    for (int e = 0; e < 9; e++) eV[e] = eK[e] = eM[e] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int b = 0; b < 3; b++) cV[b] = cK[b] = cM[b] = make_float2(0.f, 0.f);
   }
-  // trial points in pairs (2h, 2h + 1), one float2 per coordinate
-  float2 Yx[3], Yy[3], Yz[3];
+
+  __device__ __forceinline__ void load(VkWarp& sw, const StripTest& t, const GeomView& g, int lane) {
+    const TriRec& r = g.rec[min(t.grp * kBlock + lane, g.nt - 1)];
 #pragma unroll
-  for (int h = 0; h < 3; h++) {
-    Yx[h] = make_float2(yq[6 * h], yq[6 * h + 3]);
-    Yy[h] = make_float2(yq[6 * h + 1], yq[6 * h + 4]);
-    Yz[h] = make_float2(yq[6 * h + 2], yq[6 * h + 5]);
+    for (int e = 0; e < 18; e++) sw.xs[e][lane] = r.qp[e];
   }
-  const float2 kk = make_float2(k, -k);
+
+  __device__ __forceinline__ void pair(const VkWarp& sw, const StripTest& t, const TriRec& rj, const BmRec&, float w,
+                                       int lane) {
+    const float4* r4 = (const float4*)&rj;
+    const float4 q0 = r4[0], q1 = r4[1], q2 = r4[2], q3 = r4[3], q4 = r4[4], q5 = r4[5];
+    // the points of trial vertex b: orbit 1 and orbit 2
+    const float2 yx[3] = {{q0.x, q2.y}, {q0.w, q3.x}, {q1.z, q3.w}};
+    const float2 yy[3] = {{q0.y, q2.z}, {q1.x, q3.y}, {q1.w, q4.x}};
+    const float2 yz[3] = {{q0.z, q2.w}, {q1.y, q3.z}, {q2.x, q4.y}};
+    const float njx = q4.z, njy = q4.w, njz = q5.x, cjx = q5.y, cjy = q5.z, cjz = q5.w;
+    float2 dq[3];  // n_i . (c_i - y_q)
+    float dr[3];   // rho times the second orbit's
 #pragma unroll
-  for (int p = 0; p < 6; p++) {
-    const float px = xs[3 * p][tl], py = xs[3 * p + 1][tl], pz = xs[3 * p + 2][tl];
-    const float dn = njx * (cjx - px) + njy * (cjy - py) + njz * (cjz - pz);
-    // the rule is symmetric: phi_b(q) = a_q + (1 - 3 a_q) [b = own vertex of
-    // q], so each point adds its own-vertex excess to one trial sum and its
-    // common weight to c*, which all three sums receive at the end
-    float2 tV[3], tK[3], uK[3];
-    float2 cV = make_float2(0.f, 0.f), cK = cV, cU = cV;
+    for (int b = 0; b < 3; b++)
+      dq[b] = f2_fma(f2(t.nx), f2_sub(f2(t.cx), yx[b]),
+                     f2_fma(f2(t.ny), f2_sub(f2(t.cy), yy[b]), f2_mul(f2(t.nz), f2_sub(f2(t.cz), yz[b]))));
 #pragma unroll
-    for (int b = 0; b < 3; b++) {
-      tV[b] = make_float2(0.f, 0.f);
-      tK[b] = make_float2(0.f, 0.f);
-      uK[b] = make_float2(0.f, 0.f);
-    }
+    for (int b = 0; b < 3; b++) dr[b] = kRho * dq[b].y;
+    const float2 k2 = f2(k), nk2 = f2(-k);
 #pragma unroll
-    for (int h = 0; h < 3; h++) {
-      const float2 dx = f2_sub(Yx[h], f2(px)), dy = f2_sub(Yy[h], f2(py)), dz = f2_sub(Yz[h], f2(pz));
-      const float2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
-      const float2 rinv = make_float2(fminf(rsqrtf(r2.x), 1.0f / kEps), fminf(rsqrtf(r2.y), 1.0f / kEps));
-      float2 r = f2_mul(r2, rinv);
-      r.x = fmaxf(r.x, kEps);
-      r.y = fmaxf(r.y, kEps);
-      const float2 kr = f2_mul(f2(k), r);
-      const float2 rinv2 = f2_mul(rinv, rinv);
-      float sc[2][2];  // [point][sin, cos]
-      __sincosf(kr.x, &sc[0][0], &sc[0][1]);
-      __sincosf(kr.y, &sc[1][0], &sc[1][1]);
+    for (int o = 0; o < 2; o++) {  // orbit of the test points
+      const float so = w * (float)(o == 0 ? tri6_w_own(0) * tri6_w_own(0) : tri6_w_own(3) * tri6_w_own(0));
+      const float sc = w * (float)(o == 0 ? tri6_w_common(0) * tri6_w_own(0) : tri6_w_common(3) * tri6_w_own(0));
+      const float2 so2 = f2(so), sc2 = f2(sc);
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int q = 2 * h + j;
-        const float ri = j == 0 ? rinv.x : rinv.y, ri2 = j == 0 ? rinv2.x : rinv2.y;
-        const float2 gv = f2_mul(make_float2(sc[j][1], sc[j][0]), f2(ri));                  // (c, s) / r
-        const float2 gk = f2_mul(f2_fma(kk, make_float2(sc[j][0], sc[j][1]), gv), f2(ri2));  // (c + kr s, s - kr c) / r^3
-        const float2 mk = f2_mul(f2(dq[q]), gk);
-        const int b = tri6_own(q);
-        const float2 wo = f2((float)tri6_w_own(q)), wc = f2((float)tri6_w_common(q));
-        tV[b] = f2_fma(wo, gv, tV[b]);
-        tK[b] = f2_fma(wo, gk, tK[b]);
-        uK[b] = f2_fma(wo, mk, uK[b]);
-        cV = f2_fma(wc, gv, cV);
-        cK = f2_fma(wc, gk, cK);
-        cU = f2_fma(wc, mk, cU);
+      for (int a = 0; a < 3; a++) {
+        const float px = sw.xs[9 * o + 3 * a][lane], py = sw.xs[9 * o + 3 * a + 1][lane],
+                    pz = sw.xs[9 * o + 3 * a + 2][lane];
+        const float dn = njx * (cjx - px) + njy * (cjy - py) + njz * (cjz - pz);
+        float2 tV[3], tK[3], tM[3];
+        float2 sVr, sVi, sKr, sKi, sMr, sMi;  // sums over the vertices, per orbit
+        float2 ri[3], kr[3], s[3], c[3];
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          const float2 dx = f2_sub(yx[b], f2(px)), dy = f2_sub(yy[b], f2(py)), dz = f2_sub(yz[b], f2(pz));
+          float2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+          r2.x = fmaxf(r2.x, kEps * kEps);  // r >= 1e-3, to a rounding
+          r2.y = fmaxf(r2.y, kEps * kEps);
+          ri[b] = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+          kr[b] = f2_mul(k2, f2_mul(r2, ri[b]));
+        }
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          __sincosf(kr[b].x, &s[b].x, &c[b].x);
+          __sincosf(kr[b].y, &s[b].y, &c[b].y);
+        }
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          const float2 ri2 = f2_mul(ri[b], ri[b]);
+          const float2 gr = f2_mul(c[b], ri[b]), gi = f2_mul(s[b], ri[b]);  // e^{ikr} / r
+          const float2 hr = f2_mul(f2_fma(k2, s[b], gr), ri2), hi = f2_mul(f2_fma(nk2, c[b], gi), ri2);  // (1 - ikr) e^{ikr} / r^3
+          tV[b] = make_float2(fmaf(kRho, gr.y, gr.x), fmaf(kRho, gi.y, gi.x));
+          tK[b] = make_float2(fmaf(kRho, hr.y, hr.x), fmaf(kRho, hi.y, hi.x));
+          tM[b] = make_float2(fmaf(dr[b], hr.y, dq[b].x * hr.x), fmaf(dr[b], hi.y, dq[b].x * hi.x));
+          sVr = b ? f2_add(sVr, gr) : gr;
+          sVi = b ? f2_add(sVi, gi) : gi;
+          sKr = b ? f2_add(sKr, hr) : hr;
+          sKi = b ? f2_add(sKi, hi) : hi;
+          sMr = b ? f2_fma(dq[b], hr, sMr) : f2_mul(dq[b], hr);
+          sMi = b ? f2_fma(dq[b], hi, sMi) : f2_mul(dq[b], hi);
+        }
+        const float2 sV = make_float2(fmaf(kSigma, sVr.y, sVr.x), fmaf(kSigma, sVi.y, sVi.x));
+        const float2 sK = make_float2(fmaf(kSigma, sKr.y, sKr.x), fmaf(kSigma, sKi.y, sKi.x));
+        const float2 sM = make_float2(fmaf(kSigma, sMr.y, sMr.x), fmaf(kSigma, sMi.y, sMi.x));
+        const float2 sod = f2(so * dn), scd = f2(sc * dn), tau = f2(kTau);
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          const float2 v = f2_fma(tau, sV, tV[b]), kk = f2_fma(tau, sK, tK[b]), m = f2_fma(tau, sM, tM[b]);
+          eV[3 * a + b] = f2_fma(so2, v, eV[3 * a + b]);
+          cV[b] = f2_fma(sc2, v, cV[b]);
+          eK[3 * a + b] = f2_fma(sod, kk, eK[3 * a + b]);
+          cK[b] = f2_fma(scd, kk, cK[b]);
+          eM[3 * a + b] = f2_fma(so2, m, eM[3 * a + b]);
+          cM[b] = f2_fma(sc2, m, cM[b]);
+        }
       }
     }
-#pragma unroll
-    for (int b = 0; b < 3; b++) {
-      tV[b] = f2_fma(f2(1.f), cV, tV[b]);
-      tK[b] = f2_fma(f2(1.f), cK, tK[b]);
-      uK[b] = f2_fma(f2(1.f), cU, uK[b]);
-    }
+  }
+
+  template <int B>
+  __device__ __forceinline__ void take(VkWarp& sw, int i, int lane) {
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      const float wa = (float)(tri6_w(p) * tri6_phi(p, a));
-      const float2 wa2 = f2(wa), wk2 = f2(wa * dn);
-#pragma unroll
-      for (int b = 0; b < 3; b++) {
-        aV[3 * a + b] = f2_fma(wa2, tV[b], aV[3 * a + b]);
-        aK[3 * a + b] = f2_fma(wk2, tK[b], aK[3 * a + b]);
-        aM[3 * a + b] = f2_fma(wa2, uK[b], aM[3 * a + b]);
-      }
+      const float2 v = f2_add(eV[3 * a + B], cV[B]), kk = f2_add(eK[3 * a + B], cK[B]);
+      sw.col4[i][32 * a + lane] = make_float4(v.x, v.y, kk.x, kk.y);
+      sw.col2[i][32 * a + lane] = f2_add(eM[3 * a + B], cM[B]);
+      eV[3 * a + B] = eK[3 * a + B] = eM[3 * a + B] = make_float2(0.f, 0.f);
     }
-  }
-}
-
-// `uses` counts the trial tiles this CTA has processed (buffer = uses & 1,
-// mbarrier parity = (uses >> 1) & 1).
-__device__ __forceinline__ void regular_sym_item(SymSmem& sm, const GeomView& g, float k, float2* __restrict__ V,
-                                                 float2* __restrict__ K, float v_scale, float k_scale, int grp,
-                                                 int jt_begin, int jt_end, unsigned& uses) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tl = lane & 15;               // test triangle of this lane
-  const int tt = 2 * warp + (lane >> 4);  // trial triangle of this half-warp
-  const int nt = g.nt, nv = g.nv;
-  const int ti = grp * kSymTest + tl;
-  const bool valid_i = ti < nt;
-  const TriRec& ri = g.rec[valid_i ? ti : nt - 1];
-  const float area_i = ri.area;
-  const float nix = ri.n[0], niy = ri.n[1], niz = ri.n[2], cix = ri.c[0], ciy = ri.c[1], ciz = ri.c[2];
-  const int iv0 = ri.v[0], iv1 = ri.v[1], iv2 = ri.v[2];
-
-  __syncthreads();  // the previous item is done with tileI, xs and both trial buffers
-  if (tid == 0) sym_fetch_tile(sm, g, jt_begin, uses & 1);
-  copy_words(&sm.tileI, &g.tiles[grp], sizeof(TileRec), tid, kSymThreads);
-  for (int e = tid; e < 18 * kSymTest; e += kSymThreads) {
-    const int c = e / kSymTest, l = e - c * kSymTest;
-    const int t = min(grp * kSymTest + l, nt - 1);
-    sm.xs[c][l] = g.rec[t].qp[c];
+    cV[B] = cK[B] = cM[B] = make_float2(0.f, 0.f);
   }
 
-  for (int jt = jt_begin; jt < jt_end; jt++, uses++) {
-    const int bf = uses & 1;
-    __syncthreads();  // the previous tile's gather is done with the slots and with buffer bf ^ 1
-    if (tid == 0 && jt + 1 < jt_end) sym_fetch_tile(sm, g, jt + 1, bf ^ 1);
-    if (!mbar_wait(&sm.tile_full[bf], (uses >> 1) & 1u, g.err)) {
-      // expired (this geometry's status word raised): record it process-wide
-      // too, and let the copy land before the buffer is reused
-      if (tid == 0) atomicExch(&g_asm_err, 1);
-      mbar_wait_drain(&sm.tile_full[bf], (uses >> 1) & 1u);
-    }
-    const TriRec* trial = sm.trial[bf];
-    const TileRec& tileJ = sm.tileJ[bf];
-    const int ntriJ = min(kTile, nt - jt * kTile);
-
-    // ---- compute: half-warp h of warp w takes trial triangle 2w + h ----
-    const int tj = jt * kTile + tt;
-    float aa = 0.f;
-    if (tt < ntriJ) {
-      const TriRec& rj = trial[tt];
-      const int j0 = rj.v[0], j1 = rj.v[1], j2 = rj.v[2];
-      const bool touching = (iv0 == j0) | (iv0 == j1) | (iv0 == j2) | (iv1 == j0) | (iv1 == j1) | (iv1 == j2) |
-                            (iv2 == j0) | (iv2 == j1) | (iv2 == j2);
-      // on the test tile itself each unordered pair once (j > i)
-      const bool once = jt > grp || tj > ti;
-      aa = (valid_i && !touching && once) ? area_i * rj.area : 0.f;
-    }
-    const bool any = __any_sync(0xffffffffu, aa != 0.f);  // every lane, before the half-warp branch
-    if (tt < ntriJ && any) {
-      const TriRec& rj = trial[tt];
-      float yq[18];
-#pragma unroll
-      for (int e = 0; e < 18; e++) yq[e] = rj.qp[e];
-      float dq[6];
-#pragma unroll
-      for (int q = 0; q < 6; q++)
-        dq[q] = nix * (cix - yq[3 * q]) + niy * (ciy - yq[3 * q + 1]) + niz * (ciz - yq[3 * q + 2]);
-      float2 aV[9], aK[9], aM[9];
-      pair_block_sym(sm.xs, tl, yq, dq, rj.n[0], rj.n[1], rj.n[2], rj.c[0], rj.c[1], rj.c[2], k, aV, aK, aM);
-      const float sv = aa * v_scale, sk = aa * k_scale;
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-          sm.slotV[3 * tl + a][3 * tt + b] = make_float2(aV[3 * a + b].x * sv, aV[3 * a + b].y * sv);
-          sm.slotK[3 * tl + a][3 * tt + b] = make_float2(aK[3 * a + b].x * sk, aK[3 * a + b].y * sk);
-          sm.slotM[3 * tl + a][3 * tt + b] = make_float2(aM[3 * a + b].x * sk, aM[3 * a + b].y * sk);
-        }
-    } else if (tt < ntriJ) {
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-          sm.slotV[3 * tl + a][3 * tt + b] = make_float2(0.f, 0.f);
-          sm.slotK[3 * tl + a][3 * tt + b] = make_float2(0.f, 0.f);
-          sm.slotM[3 * tl + a][3 * tt + b] = make_float2(0.f, 0.f);
-        }
-    }
-    __syncthreads();
-
-    // ---- reduce corner slots onto distinct vertices: (A, B) and (B, A) ----
-    // Pass 1, in place: for every trial corner column, the row of test
-    // vertex A's first corner gets the sum over A's test corners (the corner
-    // rows of different vertices are disjoint).  Pass 2: entry (A, B) is the
-    // sum over B's trial corners along that row.  Short independent chains
-    // instead of one (corner x corner) loop per entry.
-    const TileRec& TI = sm.tileI;
-    const int nI = TI.nlv, nJ = tileJ.nlv;
-    const int ncol = 3 * ntriJ;
-    const float rcol = 1.f / (float)ncol, rJ = 1.f / (float)(nJ > 0 ? nJ : 1);
-    for (int e = tid; e < nI * ncol; e += kSymThreads) {
-      const int a = div_by(e, ncol, rcol);
-      const int col = e - a * ncol;
-      const int ca0 = TI.lv_ptr[a], ca1 = TI.lv_ptr[a + 1];
-      const int rep = TI.lv_corner[ca0];
-      float2 v = sm.slotV[rep][col], kk = sm.slotK[rep][col], mm = sm.slotM[rep][col];
-#pragma unroll 4
-      for (int ca = ca0 + 1; ca < ca1; ca++) {
-        const int row = TI.lv_corner[ca];
-        const float2 v1 = sm.slotV[row][col], k1 = sm.slotK[row][col], m1 = sm.slotM[row][col];
-        v.x += v1.x;
-        v.y += v1.y;
-        kk.x += k1.x;
-        kk.y += k1.y;
-        mm.x += m1.x;
-        mm.y += m1.y;
-      }
-      sm.slotV[rep][col] = v;
-      sm.slotK[rep][col] = kk;
-      sm.slotM[rep][col] = mm;
-    }
-    __syncthreads();
-    for (int e = tid; e < nI * nJ; e += kSymThreads) {
-      const int a = div_by(e, nJ, rJ);
-      const int b = e - a * nJ;
-      const int rep = TI.lv_corner[TI.lv_ptr[a]];
-      const int cb0 = tileJ.lv_ptr[b], cb1 = tileJ.lv_ptr[b + 1];
-      float2 acc_v = make_float2(0.f, 0.f), acc_k = make_float2(0.f, 0.f), acc_m = make_float2(0.f, 0.f);
-#pragma unroll 4
-      for (int cb = cb0; cb < cb1; cb++) {
-        const int col = tileJ.lv_corner[cb];
-        const float2 v1 = sm.slotV[rep][col], k1 = sm.slotK[rep][col], m1 = sm.slotM[rep][col];
-        acc_v.x += v1.x;
-        acc_v.y += v1.y;
-        acc_k.x += k1.x;
-        acc_k.y += k1.y;
-        acc_m.x += m1.x;
-        acc_m.y += m1.y;
-      }
-      const int A = TI.vid[a], B = tileJ.vid[b];
-      if (acc_v.x != 0.f || acc_v.y != 0.f || acc_k.x != 0.f || acc_k.y != 0.f || acc_m.x != 0.f ||
-          acc_m.y != 0.f) {
-        atomicAdd(&V[(size_t)A * nv + B], acc_v);
-        atomicAdd(&V[(size_t)B * nv + A], acc_v);
-        atomicAdd(&K[(size_t)A * nv + B], acc_k);
-        atomicAdd(&K[(size_t)B * nv + A], acc_m);
-      }
-    }
+  __device__ __forceinline__ void store(const GeomView& g, int A, int B, const float4& s4, const float2& s2) const {
+    if (s4.x == 0.f && s4.y == 0.f && s4.z == 0.f && s4.w == 0.f && s2.x == 0.f && s2.y == 0.f) return;
+    const size_t ab = (size_t)A * g.nv + B, ba = (size_t)B * g.nv + A;
+    const float2 v = make_float2(s4.x * v_scale, s4.y * v_scale);
+    atomicAdd(&V[ab], v);
+    atomicAdd(&V[ba], v);
+    atomicAdd(&K[ab], make_float2(s4.z * k_scale, s4.w * k_scale));
+    atomicAdd(&K[ba], make_float2(s2.x * k_scale, s2.y * k_scale));
   }
-}
+};
 
-// Splits units [pos, end) of one problem at test-tile boundaries.
-__device__ __forceinline__ void regular_sym_units(SymSmem& sm, const GeomView& g, float k, float2* V, float2* K,
-                                                  float v_scale, float k_scale, long long pos, long long end,
-                                                  unsigned& uses) {
-  while (pos < end) {  // uniform over the block
-    const int grp = tile_group_of(pos, g.ntiles);
-    const long long base = tile_units_before(grp, g.ntiles);
-    const long long gend = base + (g.ntiles - grp);
-    const long long stop = end < gend ? end : gend;
-    const int jt0 = grp + (int)(pos - base);
-    regular_sym_item(sm, g, k, V, K, v_scale, k_scale, grp, jt0, jt0 + (int)(stop - pos), uses);
-    pos = stop;
-  }
-}
-
-// The (test tile, trial tile >= it) units in order (tile_units_before).
-// Items are equal runs of `chunk` consecutive units (a run crossing a test
-// tile is split), dealt round-robin to a persistent grid: every CTA gets the
-// same amount of work.
-__global__ void __launch_bounds__(kSymThreads, 2)
-    regular_sym_kernel(GeomView g, float k, float2* __restrict__ V, float2* __restrict__ K, float v_scale,
-                       float k_scale, long long chunk, long long n_units, int n_items) {
+// One problem: equal runs of `chunk` steps, one or more per warp of a
+// persistent grid (every warp gets the same amount of work).
+__global__ void __launch_bounds__(kStripThreads, 2)
+    regular_strip_vk_kernel(const __grid_constant__ GeomView g, float k, float2* __restrict__ V, float2* __restrict__ K, float v_scale,
+                            float k_scale, long long chunk, long long n_steps, long long n_items) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SymSmem& sm = *reinterpret_cast<SymSmem*>(smem_raw);
-  if (threadIdx.x == 0) {
-    mbar_init(&sm.tile_full[0], 1);
-    mbar_init(&sm.tile_full[1], 1);
-    mbar_init_fence();
-  }
+  VkWarp& sw = reinterpret_cast<VkWarp*>(smem_raw)[threadIdx.x >> 5];
+  strip_init(sw);
+  VkStrip pol;
+  pol.k = k;
+  pol.v_scale = v_scale;
+  pol.k_scale = k_scale;
+  pol.V = V;
+  pol.K = K;
+  pol.clear();
+  StripTest test;
   unsigned uses = 0;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const long long pos = (long long)item * chunk;
-    const long long end = pos + chunk < n_units ? pos + chunk : n_units;
-    regular_sym_units(sm, g, k, V, K, v_scale, k_scale, pos, end, uses);
+  const long long warps = (long long)gridDim.x * kStripWarps;
+  for (long long item = (long long)blockIdx.x * kStripWarps + (threadIdx.x >> 5); item < n_items; item += warps) {
+    const long long pos = item * chunk;
+    strip_walk(sw, test, g, pol, pos, pos + chunk < n_steps ? pos + chunk : n_steps, uses, &g_asm_err);
   }
 }
 
@@ -902,16 +773,16 @@ __global__ void __launch_bounds__(128)
 
 // ---------------------------------------------------------------------------
 // Batched assembly: many problems (meshes of uneven size, wavenumbers) in one
-// persistent launch.  Regular work items of all problems (runs of used
-// (test group, trial tile) units, each unordered pair once) form one queue
-// that CTAs drain with an atomic counter (dynamic load balance); touching
+// persistent launch.  Regular work items of all problems (runs of strip
+// steps, each unordered pair once) form one queue that warps drain with an
+// atomic counter (dynamic load balance); touching
 // pairs of all problems are concatenated per type.
 // ---------------------------------------------------------------------------
 struct BatchProblem {
   GeomView g;
   float k;
-  int chunk, n_chunks;      // units per item, items
-  long long n_units;        // used (test group, trial tile) units
+  int chunk;                // steps per item
+  long long n_steps;        // steps of the problem's strip walk
   float2* V;
   float2* K;
   long long item_begin;   // prefix sum of regular items
@@ -936,32 +807,34 @@ __device__ __forceinline__ int find_problem(const BatchProblem* probs, int np, l
   return lo;
 }
 
-// Each unordered regular pair of every problem once (the symmetric item of
-// regular_sym_kernel); items are runs of `chunk` units of one problem.
-__global__ void __launch_bounds__(kSymThreads, 2)
-    regular_sym_batch_kernel(BatchHeader* __restrict__ hdr, const BatchProblem* __restrict__ probs, float v_scale,
-                             float k_scale) {
+// Each unordered regular pair of every problem once; items are runs of
+// `chunk` steps of one problem's strip walk, drawn by the warps.
+__global__ void __launch_bounds__(kStripThreads, 2)
+    regular_strip_vk_batch_kernel(BatchHeader* __restrict__ hdr, const BatchProblem* __restrict__ probs, float v_scale,
+                                  float k_scale) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SymSmem& sm = *reinterpret_cast<SymSmem*>(smem_raw);
-  __shared__ long long s_item;
-  if (threadIdx.x == 0) {
-    mbar_init(&sm.tile_full[0], 1);
-    mbar_init(&sm.tile_full[1], 1);
-    mbar_init_fence();
-  }
+  VkWarp& sw = reinterpret_cast<VkWarp*>(smem_raw)[threadIdx.x >> 5];
+  strip_init(sw);
   const int np = hdr->nproblems;
   const long long total = hdr->total_items;
+  VkStrip pol;
+  pol.v_scale = v_scale;
+  pol.k_scale = k_scale;
+  pol.clear();
+  StripTest test;
   unsigned uses = 0;
   for (;;) {
-    __syncthreads();  // everyone has read s_item of the previous round
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&hdr->next_item, 1ull);
-    __syncthreads();
-    const long long item = s_item;
+    long long item = 0;
+    if ((threadIdx.x & 31) == 0) item = (long long)atomicAdd(&hdr->next_item, 1ull);
+    item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= total) break;
     const BatchProblem& P = probs[find_problem(probs, np, item, -1)];
+    pol.k = P.k;
+    pol.V = P.V;
+    pol.K = P.K;
+    test.grp = -1;  // another problem's block may have the same number
     const long long pos = (item - P.item_begin) * P.chunk;
-    const long long end = pos + P.chunk < P.n_units ? pos + P.chunk : P.n_units;
-    regular_sym_units(sm, P.g, P.k, P.V, P.K, v_scale, k_scale, pos, end, uses);
+    strip_walk(sw, test, P.g, pol, pos, pos + P.chunk < P.n_steps ? pos + P.chunk : P.n_steps, uses, &g_asm_err);
   }
 }
 
@@ -1056,31 +929,41 @@ int launch_singular(const GeomView& g, float k, float2* V, float2* K, float v_sc
 
 }  // namespace
 
-// V and/or (mass_coeff M + k_coeff K), both overwritten.
-int launch_regular_sym(const GeomView& g, float k, float2* V, float2* K, float v_scale, float k_scale,
-                       cudaStream_t s) {
-  const int smem = (int)sizeof(SymSmem);
-  static std::atomic<bool> attr_set{false};
-  if (!attr_set.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(regular_sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr_set.store(true, std::memory_order_release);
+namespace {
+// Persistent grid of a strip kernel (shared-memory attribute set once).
+template <typename KernelT>
+int strip_grid(KernelT kernel, std::atomic<bool>& attr, int most_per_sm, long long* grid) {
+  const int smem = (int)(kStripWarps * sizeof(VkWarp));
+  if (!attr.load(std::memory_order_acquire)) {
+    BEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr.store(true, std::memory_order_release);
   }
   int occ = 0;
-  BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, regular_sym_kernel, kSymThreads, smem));
-  const int grid = sm_count() * (occ > 0 ? occ : 1);
-  const long long n_units = (long long)g.ntiles * (g.ntiles + 1) / 2;
-  // 8 equal items per CTA (a tuned chunk overrides)
-  long long chunk = (n_units + 8LL * grid - 1) / (8LL * grid);
-  if (chunk < 1) chunk = 1;
-  if (g_tune_chunk > 0) chunk = g_tune_chunk;
-  const long long n_items = (n_units + chunk - 1) / chunk;
-  (regular_sym_kernel<<<grid < n_items ? grid : (int)n_items, kSymThreads, smem, s>>>(g, k, V, K, v_scale, k_scale,
-                                                                                       chunk, n_units, (int)n_items),
+  BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kStripThreads, smem));
+  if (most_per_sm > 0 && most_per_sm < occ) occ = most_per_sm;
+  *grid = (long long)sm_count() * (occ > 0 ? occ : 1);
+  return BEM_OK;
+}
+
+int launch_strip_vk(const GeomView& g, float k, float2* V, float2* K, float v_scale, float k_scale, cudaStream_t s) {
+  static std::atomic<bool> attr{false};
+  long long grid = 0;
+  int rc = strip_grid(regular_strip_vk_kernel, attr, 0, &grid);
+  if (rc) return rc;
+  const long long n_steps = strip_steps(g.nblocks), warps = grid * kStripWarps;
+  long long chunk = (n_steps + warps - 1) / warps;
+  if (chunk < 2) chunk = 2;
+  if (g_tune_chunk > 0) chunk = 32LL * g_tune_chunk;
+  const long long n_items = (n_steps + chunk - 1) / chunk, blocks = (n_items + kStripWarps - 1) / kStripWarps;
+  (regular_strip_vk_kernel<<<(unsigned)(grid < blocks ? grid : blocks), kStripThreads, kStripWarps * sizeof(VkWarp), s>>>(
+       g, k, V, K, v_scale, k_scale, chunk, n_steps, n_items),
    count_launch());
   BEM_CUDA_TRY(cudaGetLastError());
   return BEM_OK;
 }
+}  // namespace
 
+// V and/or (mass_coeff M + k_coeff K), both overwritten.
 int assemble_vk(const GeomView& g, float k, float2* V, float2* Kout, float mass_coeff, float k_coeff, cudaStream_t s) {
   const size_t bytes = sizeof(float2) * (size_t)g.nv * g.nv;
   if (V) BEM_CUDA_TRY(cudaMemsetAsync(V, 0, bytes, s));
@@ -1089,7 +972,7 @@ int assemble_vk(const GeomView& g, float k, float2* V, float2* Kout, float mass_
   const float k_scale = -kInv4Pi * k_coeff;  // K = -(...)/(4 pi)
   int rc;
   if (V && Kout) {
-    if ((rc = launch_regular_sym(g, k, V, Kout, v_scale, k_scale, s))) return rc;
+    if ((rc = launch_strip_vk(g, k, V, Kout, v_scale, k_scale, s))) return rc;
     return launch_singular<true, true>(g, k, V, Kout, v_scale, k_scale, mass_coeff, s);
   } else if (V) {
     if ((rc = launch_regular<true, false>(g, k, V, nullptr, v_scale, 0.f, s))) return rc;
@@ -1200,12 +1083,10 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
                       float mass_coeff, float k_coeff, void* ws, size_t ws_bytes, cudaStream_t s) {
   if (np <= 0) return BEM_ERR_INVALID_ARGUMENT;
   if (!ws || ws_bytes < batch_workspace_bytes(np)) return BEM_ERR_WORKSPACE;
-  const int smem = (int)sizeof(SymSmem);
   static std::atomic<bool> attr{false};
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(regular_sym_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr.store(true, std::memory_order_release);
-  }
+  long long grid = 0;
+  const int rc = strip_grid(regular_strip_vk_batch_kernel, attr, g_tune_ctas_per_sm, &grid);
+  if (rc) return rc;
   // host descriptors
   const size_t hbytes = al256b(sizeof(BatchHeader)), pbytes = sizeof(BatchProblem) * (size_t)np;
   if (!t_stage.ev) BEM_CUDA_TRY(cudaEventCreateWithFlags(&t_stage.ev, cudaEventDisableTiming));
@@ -1219,7 +1100,11 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
   BatchProblem* hp = (BatchProblem*)((char*)t_stage.buf + hbytes);
   std::memset(hh, 0, sizeof(BatchHeader));
   hh->nproblems = np;
-  long long items = 0, pairs[3] = {0, 0, 0};
+  long long items = 0, pairs[3] = {0, 0, 0}, steps = 0;
+  for (int p = 0; p < np; p++) steps += strip_steps(views[p].nblocks);
+  // about 8 items per warp, at most 16 trial blocks each
+  int chunk = (int)std::min<long long>(512, std::max<long long>(4, steps / (8 * grid * kStripWarps)));
+  if (g_tune_chunk > 0) chunk = (int)std::min<long long>(32LL * g_tune_chunk, 1 << 30);
   const size_t elem = sizeof(float2);
   for (int p = 0; p < np; p++) {
     const GeomView& g = views[p];
@@ -1230,14 +1115,12 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
     BatchProblem& P = hp[p];
     P.g = g;
     P.k = ks[p];
-    P.n_units = (long long)g.ntiles * (g.ntiles + 1) / 2;
-    int chunk = g_tune_chunk > 0 ? g_tune_chunk : (g.ntiles / 8 < 1 ? 1 : (g.ntiles / 8 > 64 ? 64 : g.ntiles / 8));
+    P.n_steps = strip_steps(g.nblocks);
     P.chunk = chunk;
-    P.n_chunks = (int)((P.n_units + chunk - 1) / chunk);
     P.V = Vs[p];
     P.K = Ks[p];
     P.item_begin = items;
-    items += P.n_chunks;
+    items += (P.n_steps + chunk - 1) / chunk;
     P.pair_begin[0] = pairs[0];
     P.pair_begin[1] = pairs[1];
     P.pair_begin[2] = pairs[2];
@@ -1252,13 +1135,10 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
   BEM_CUDA_TRY(cudaMemcpyAsync(ws, t_stage.buf, hbytes + pbytes, cudaMemcpyHostToDevice, s));
   BEM_CUDA_TRY(cudaEventRecord(t_stage.ev, s));
   const float v_scale = kInv4Pi, k_scale = -kInv4Pi * k_coeff;
-  int occ = 0;
-  BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, regular_sym_batch_kernel, kSymThreads, smem));
-  if (g_tune_ctas_per_sm > 0 && g_tune_ctas_per_sm < occ) occ = g_tune_ctas_per_sm;
-  const long long grid = (long long)sm_count() * (occ > 0 ? occ : 1);
+  const long long blocks = (items + kStripWarps - 1) / kStripWarps;
   if (items > 0)
-    (regular_sym_batch_kernel<<<(unsigned)(grid < items ? grid : items), kSymThreads, smem, s>>>(dh, dp, v_scale,
-                                                                                                 k_scale),
+    (regular_strip_vk_batch_kernel<<<(unsigned)(grid < blocks ? grid : blocks), kStripThreads,
+                                     kStripWarps * sizeof(VkWarp), s>>>(dh, dp, v_scale, k_scale),
      count_launch());
   const int wpb = 4;
   if (pairs[0])

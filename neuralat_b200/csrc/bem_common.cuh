@@ -71,6 +71,15 @@ __device__ __forceinline__ float2 f2_mul(float2 a, float2 b) {
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+__device__ __forceinline__ float2 f2_add(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 __device__ __forceinline__ float2 f2_sub(float2 a, float2 b) {
   float2 d;
   asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
@@ -94,7 +103,7 @@ struct __align__(16) TriRec {
   float area;
   int v[3];
   float h;  // n . v0 (plane offset)
-  float pad;
+  int leave;  // sorted order: bit b set if the next triangle of the block does not hold v[b] in slot b
 };
 static_assert(sizeof(TriRec) == 128, "TriRec must be 128 bytes");
 
@@ -117,13 +126,30 @@ struct __align__(16) TileRec {
   int nlv;                       // number of distinct vertices in the tile
   int ntri;                      // triangles in the tile (last tile may be short)
   int pad0, pad1;
-  int vid[kTileCorners];         // global vertex id of each local vertex (ascending)
+  int vid[kTileCorners];         // global vertex id of each local vertex
   uint8_t corner_lv[kTileCorners];     // local vertex of corner (3*t + a)
   uint8_t lv_ptr[kTileCorners + 4];    // CSR: corners of local vertex l are lv_corner[lv_ptr[l]..lv_ptr[l+1])
   uint8_t lv_corner[kTileCorners];
   uint8_t pad2[12];
 };
 static_assert(sizeof(TileRec) % 16 == 0, "TileRec alignment");
+
+// Blocks of 32 sorted triangles, ordered within the block as paths over shared
+// edges, with the local vertices of each triangle permuted (in the sorted
+// records only) so that a vertex kept from one triangle to the next stays in
+// its slot.  Corner 32 a + t is slot a of the block's triangle t.
+constexpr int kBlock = 32;
+constexpr int kBlockCorners = 3 * kBlock;
+struct __align__(16) BlockRec {
+  int nlv;                         // distinct vertices
+  int most;                        // most corners of one vertex
+  int pad[2];
+  int vid[kBlockCorners];          // global vertex id of each local vertex
+  uint8_t ptr[kBlockCorners + 4];  // corners of local vertex l: corner[ptr[l]..ptr[l+1])
+  uint8_t corner[kBlockCorners];
+  uint8_t pad2[12];
+};
+static_assert(sizeof(BlockRec) % 16 == 0, "BlockRec alignment");
 
 // Header at the start of the geometry workspace.  All offsets in bytes from
 // the start of the workspace.
@@ -144,19 +170,23 @@ struct GeomHeader {
   uint64_t off_normals;    // float[nt*3]
   uint64_t off_curls;      // float[nt*9]   rows: n x grad(phi_b)
   uint64_t off_bmrec;      // BmRec[nt] in sorted order
+  uint64_t off_slots;      // int[nt]  sorted position -> local vertex of each slot (2 bits each) and leave bits
+  uint64_t off_blocks;     // BlockRec[nblocks]
   uint64_t bytes;
 };
-constexpr uint32_t kGeomMagic = 0x42454D33u;  // "BEM3"
+constexpr uint32_t kGeomMagic = 0x42454D34u;  // "BEM4"
 
 // Device-side view of a built geometry.
 struct GeomView {
-  int nv, nt, ntiles, n_edge, n_vert;
+  int nv, nt, ntiles, nblocks, n_edge, n_vert;
   const float* vertices;
   const int* triangles;
   const int* perm;
+  const int* slots;        // sorted position -> input-order local vertex of slot a in bits 2a, 2a + 1
   const TriRec* rec;       // sorted order
   const TriRec* rec_orig;  // input order
   const TileRec* tiles;
+  const BlockRec* blocks;
   const int2* edge_pairs;
   const int2* vert_pairs;
   const float* normals;

@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kGenThreads, 2)
     const bool valid_i = ti < nt;
     const TriRec& ri = g.rec[valid_i ? ti : nt - 1];
     const int oi = g.perm[valid_i ? ti : nt - 1];
+    const int oslots = g.slots[valid_i ? ti : nt - 1];  // the sorted records permute the local vertices
     float xv[9];
 #pragma unroll
     for (int a = 0; a < 3; a++)
@@ -145,7 +146,7 @@ __global__ void __launch_bounds__(kGenThreads, 2)
     float ci[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, nip[3] = {0, 0, 0};
     if (kCurl) {
 #pragma unroll
-      for (int e = 0; e < 9; e++) ci[e] = curls[9 * oi + e];
+      for (int e = 0; e < 9; e++) ci[e] = curls[9 * oi + 3 * ((oslots >> (2 * (e / 3))) & 3) + e % 3];
 #pragma unroll
       for (int e = 0; e < 3; e++) nip[e] = normals[3 * oi + e];
     }
@@ -165,7 +166,10 @@ __global__ void __launch_bounds__(kGenThreads, 2)
       for (int e = tid; e < ntriJ * 9; e += kGenThreads) {
         const int t = e / 9, c = e - 9 * t;
         sm.tverts[t][c] = g.vertices[3 * sm.trial[t].v[c / 3] + c % 3];
-        if (kCurl) sm.tcurl[t][c] = curls[9 * g.perm[jt * kTile + t] + c];
+        if (kCurl) {
+          const int slot = (g.slots[jt * kTile + t] >> (2 * (c / 3))) & 3;
+          sm.tcurl[t][c] = curls[9 * g.perm[jt * kTile + t] + 3 * slot + c % 3];
+        }
       }
       if (kCurl)
         for (int e = tid; e < ntriJ * 3; e += kGenThreads)

@@ -34,11 +34,13 @@ inline uint32_t part1by2(uint32_t v) {
 }
 
 struct HostGeom {
-  int nv = 0, nt = 0, ntiles = 0;
+  int nv = 0, nt = 0, ntiles = 0, nblocks = 0;
   std::vector<float> vertices;
   std::vector<int> triangles;
   std::vector<int> perm;
+  std::vector<int> slots;
   std::vector<TileRec> tiles;
+  std::vector<BlockRec> blocks;
   std::vector<int2> edge_pairs, vert_pairs;
   int max_valence = 0;
   GeomHeader hdr{};
@@ -90,7 +92,9 @@ int analyse(const float* d_vertices, int nv, const int* d_triangles, int nt, cud
   }
   t_last_valid = false;
   t_stage_ok = false;
-  t_last = HostGeom{};
+  t_last.edge_pairs.clear();  // the vectors keep their capacity from mesh to mesh
+  t_last.vert_pairs.clear();
+  t_last.max_valence = 0;
   t_last.nv = nv;
   t_last.nt = nt;
   t_last.vertices.assign((const float*)t_download.p, (const float*)t_download.p + 3 * (size_t)nv);
@@ -100,6 +104,163 @@ int analyse(const float* d_vertices, int nv, const int* d_triangles, int nt, cud
   t_last_valid = true;
   *out = &t_last;
   return BEM_OK;
+}
+
+// Vertex in slot a of the triangle at sorted position s.
+inline int slot_vertex(const HostGeom& g, int s, int a) {
+  return g.triangles[3 * (size_t)g.perm[s] + ((g.slots[s] >> (2 * a)) & 3)];
+}
+
+// Cuts the sorted triangles into blocks of 32 that share as many vertices as
+// possible: a block grows from the first free triangle in Morton order, each
+// time by the triangle across one of its edges that brings no new vertex, then
+// by the one with the fewest free neighbours (so that no islands stay behind),
+// the oldest first (so that it stays round).  Blocks of a closed mesh hold
+// about 26 vertices (31 with plain runs of the Morton order), which is what a
+// column flush of the strip kernels costs.
+void grow_blocks(HostGeom& g, const std::vector<int>& nbr) {
+  const int nt = g.nt;
+  std::vector<int> order(g.perm), mark(g.nv, -1);
+  std::vector<uint8_t> state(nt, 0);  // 0 free, 1 in the list of candidates, 2 taken
+  std::vector<int> cand;
+  int next = 0, done = 0;
+  for (int blk = 0; done < nt; blk++) {
+    cand.clear();
+    for (int n = 0; n < kBlock && done < nt; n++) {
+      int best = -1, best_score = -1;
+      for (size_t c = 0; c < cand.size(); c++) {
+        const int* v = &g.triangles[3 * (size_t)cand[c]];
+        int score = (mark[v[0]] == blk) + (mark[v[1]] == blk) + (mark[v[2]] == blk);
+        score *= 4;
+        for (int e = 0; e < 3; e++) {
+          const int j = nbr[3 * (size_t)cand[c] + e];
+          score += j < 0 || state[j] == 2;
+        }
+        if (score > best_score) {
+          best_score = score;
+          best = (int)c;
+        }
+      }
+      int tri;
+      if (best >= 0) {
+        tri = cand[best];
+        cand.erase(cand.begin() + best);
+      } else {
+        while (state[order[next]] == 2) next++;
+        tri = order[next];
+      }
+      state[tri] = 2;
+      g.perm[done++] = tri;
+      for (int a = 0; a < 3; a++) mark[g.triangles[3 * (size_t)tri + a]] = blk;
+      for (int e = 0; e < 3; e++) {
+        const int j = nbr[3 * (size_t)tri + e];
+        if (j >= 0 && state[j] == 0) {
+          state[j] = 1;
+          cand.push_back(j);
+        }
+      }
+    }
+    for (int c : cand) state[c] = 0;
+  }
+}
+
+// Orders the triangles of every 32-triangle block of the sorted order as
+// paths over shared edges (nbr: up to three edge neighbours per triangle) and
+// chooses the slots of each triangle's vertices and its leave bits (BlockRec).
+// From a triangle the path goes on to the neighbour with the fewest
+// neighbours left, so that few triangles end up alone.
+void path_order(HostGeom& g, const std::vector<int>& nbr) {
+  const int nt = g.nt;
+  g.slots.assign(nt, 0);
+  std::vector<int> place(nt);  // sorted position of a triangle
+  for (int s = 0; s < nt; s++) place[g.perm[s]] = s;
+  for (int b0 = 0; b0 < nt; b0 += kBlock) {
+    const int n = std::min(kBlock, nt - b0);
+    int tri[kBlock], left[kBlock], near[kBlock][3];
+    bool used[kBlock];
+    for (int i = 0; i < n; i++) {
+      tri[i] = g.perm[b0 + i];
+      used[i] = false;
+      left[i] = 0;
+      for (int e = 0; e < 3; e++) {
+        const int j = nbr[3 * (size_t)tri[i] + e];
+        const int p = j < 0 ? -1 : place[j] - b0;
+        near[i][e] = p >= 0 && p < n ? p : -1;
+        left[i] += near[i][e] >= 0;
+      }
+    }
+    int last = -1, prev[3] = {-1, -1, -1};  // the path's last triangle, the vertices in its slots
+    for (int s = 0; s < n; s++) {
+      int best = -1;
+      if (last >= 0)
+        for (int e = 0; e < 3; e++) {
+          const int i = near[last][e];
+          if (i >= 0 && !used[i] && (best < 0 || left[i] < left[best] || (left[i] == left[best] && i < best))) best = i;
+        }
+      if (best < 0)  // a new path
+        for (int i = 0; i < n; i++)
+          if (!used[i] && (best < 0 || left[i] < left[best])) best = i;
+      used[best] = true;
+      for (int e = 0; e < 3; e++)
+        if (near[best][e] >= 0) left[near[best][e]]--;
+      // shared vertices keep their slots, the others fill the free ones in order
+      const int* v = &g.triangles[3 * (size_t)tri[best]];
+      int slot[3] = {-1, -1, -1};  // local vertex in each slot
+      bool kept[3] = {false, false, false};
+      for (int a = 0; a < 3; a++)
+        for (int c = 0; c < 3; c++)
+          if (prev[a] == v[c]) {
+            slot[a] = c;
+            kept[c] = true;
+          }
+      int leave = 0;
+      for (int a = 0; a < 3; a++)
+        if (slot[a] < 0) {
+          leave |= 1 << a;
+          int c = 0;
+          while (kept[c]) c++;
+          slot[a] = c;
+          kept[c] = true;
+        }
+      if (s > 0) g.slots[b0 + s - 1] |= leave << 8;
+      g.slots[b0 + s] = slot[0] | (slot[1] << 2) | (slot[2] << 4);
+      g.perm[b0 + s] = tri[best];
+      for (int a = 0; a < 3; a++) prev[a] = v[slot[a]];
+      last = best;
+    }
+    g.slots[b0 + n - 1] |= 7 << 8;
+  }
+}
+
+// Vertex table of `ntri` triangles from sorted position s0: the distinct
+// vertices in order of appearance (vid, returns their number), the corners of
+// each (ptr, corner; corner a of triangle t is st t + sa a) and, unless null,
+// each corner's local vertex.  stamp / local: scratch, one entry per vertex
+// (`tag` differs from call to call).
+int local_vertices(const HostGeom& g, int s0, int ntri, int st, int sa, int tag, std::vector<int>& stamp,
+                   std::vector<int>& local, int* vid, uint8_t* ptr, uint8_t* corner, uint8_t* corner_lv) {
+  int n = 0, lv[kBlockCorners], fill[kBlockCorners + 1] = {0};
+  for (int c = 0; c < 3 * ntri; c++) {
+    const int v = slot_vertex(g, s0 + c / 3, c % 3);
+    if (stamp[v] != tag) {
+      stamp[v] = tag;
+      local[v] = n;
+      vid[n++] = v;
+    }
+    lv[c] = local[v];
+    fill[lv[c] + 1]++;
+  }
+  for (int l = 0; l < n; l++) {
+    fill[l + 1] += fill[l];
+    ptr[l] = (uint8_t)fill[l];
+  }
+  ptr[n] = (uint8_t)(3 * ntri);
+  for (int c = 0; c < 3 * ntri; c++) {
+    const int at = st * (c / 3) + sa * (c % 3);
+    corner[fill[lv[c]]++] = (uint8_t)at;
+    if (corner_lv) corner_lv[at] = (uint8_t)lv[c];
+  }
+  return n;
 }
 
 int analyse_host(HostGeom& g) {
@@ -141,41 +302,19 @@ int analyse_host(HostGeom& g) {
     uint64_t code = part1by2(q[0]) | (part1by2(q[1]) << 1) | (part1by2(q[2]) << 2);
     key[i] = (code << 32) | (uint32_t)i;
   }
-  std::sort(key.begin(), key.end());
-  g.perm.resize(nt);
-  for (int s2 = 0; s2 < nt; s2++) g.perm[s2] = (int)(key[s2] & 0xffffffffu);
-
-  // 16-triangle tiles with local vertex tables.
-  g.ntiles = (nt + kTile - 1) / kTile;
-  g.tiles.assign(g.ntiles, TileRec{});
-  for (int t = 0; t < g.ntiles; t++) {
-    TileRec& tr = g.tiles[t];
-    std::memset(&tr, 0, sizeof(TileRec));
-    int ntri = std::min(kTile, nt - t * kTile);
-    tr.ntri = ntri;
-    int ids[kTileCorners];
-    int nc = 3 * ntri;
-    for (int c = 0; c < nc; c++) ids[c] = g.triangles[3 * (size_t)g.perm[t * kTile + c / 3] + c % 3];
-    int uniq[kTileCorners];
-    std::copy(ids, ids + nc, uniq);
-    std::sort(uniq, uniq + nc);
-    int nl = (int)(std::unique(uniq, uniq + nc) - uniq);
-    tr.nlv = nl;
-    for (int l = 0; l < nl; l++) tr.vid[l] = uniq[l];
-    int count[kTileCorners] = {0};
-    for (int c = 0; c < nc; c++) {
-      int l = (int)(std::lower_bound(uniq, uniq + nl, ids[c]) - uniq);
-      tr.corner_lv[c] = (uint8_t)l;
-      count[l]++;
-    }
-    tr.lv_ptr[0] = 0;
-    for (int l = 0; l < nl; l++) tr.lv_ptr[l + 1] = (uint8_t)(tr.lv_ptr[l] + count[l]);
-    int fill[kTileCorners] = {0};
-    for (int c = 0; c < nc; c++) {
-      int l = tr.corner_lv[c];
-      tr.lv_corner[tr.lv_ptr[l] + fill[l]++] = (uint8_t)c;
+  // three counting passes over the 30-bit code (stable: equal codes keep the input order)
+  {
+    std::vector<uint64_t> other(nt);
+    for (int shift = 32; shift < 62; shift += 10) {
+      int start[1025] = {0};
+      for (int i = 0; i < nt; i++) start[((key[i] >> shift) & 1023) + 1]++;
+      for (int d = 0; d < 1024; d++) start[d + 1] += start[d];
+      for (int i = 0; i < nt; i++) other[start[(key[i] >> shift) & 1023]++] = key[i];
+      key.swap(other);
     }
   }
+  g.perm.resize(nt);
+  for (int s2 = 0; s2 < nt; s2++) g.perm[s2] = (int)(key[s2] & 0xffffffffu);
 
   // Vertex stars and touching pairs (exact, no neighbour cap).
   std::vector<int> vptr(nv + 1, 0), vtri(3 * (size_t)nt);
@@ -190,24 +329,60 @@ int analyse_host(HostGeom& g) {
       for (int a = 0; a < 3; a++) vtri[fill[g.triangles[3 * (size_t)i + a]]++] = i;
   }
   std::vector<int> seen(nt, -1);
+  std::vector<int> nbr(3 * (size_t)nt, -1);  // triangles across an edge (three at most are used)
+  std::vector<int> touch, shared(nt, 0);  // triangles meeting i in the order of its stars, vertices shared with each
+  g.edge_pairs.reserve(3 * (size_t)nt);
+  g.vert_pairs.reserve(10 * (size_t)nt);
   for (int i = 0; i < nt; i++) {
     const int* ti = &g.triangles[3 * (size_t)i];
+    touch.clear();
     seen[i] = i;
     for (int a = 0; a < 3; a++)
       for (int p = vptr[ti[a]]; p < vptr[ti[a] + 1]; p++) {
-        int j = vtri[p];
-        if (seen[j] == i) continue;
-        seen[j] = i;
-        const int* tj = &g.triangles[3 * (size_t)j];
-        int common = 0;
-        for (int x = 0; x < 3; x++)
-          for (int y = 0; y < 3; y++) common += (ti[x] == tj[y]);
-        if (common >= 3) return BEM_ERR_DEGENERATE;  // duplicated triangle
-        if (common == 2)
-          g.edge_pairs.push_back(make_int2(i, j));
-        else
-          g.vert_pairs.push_back(make_int2(i, j));
+        const int j = vtri[p];
+        if (j == i) continue;
+        if (seen[j] != i) {
+          seen[j] = i;
+          shared[j] = 0;
+          touch.push_back(j);
+        }
+        shared[j]++;
       }
+    int edges = 0;
+    for (int j : touch) {
+      if (shared[j] >= 3) return BEM_ERR_DEGENERATE;  // duplicated triangle
+      if (shared[j] == 2) {
+        g.edge_pairs.push_back(make_int2(i, j));
+        if (edges < 3) nbr[3 * (size_t)i + edges++] = j;
+      } else {
+        g.vert_pairs.push_back(make_int2(i, j));
+      }
+    }
+  }
+
+  grow_blocks(g, nbr);
+  path_order(g, nbr);
+
+  // 16-triangle tiles with local vertex tables.
+  g.ntiles = (nt + kTile - 1) / kTile;
+  g.tiles.assign(g.ntiles, TileRec{});
+  std::vector<int> stamp(nv, -1), local(nv);
+  for (int t = 0; t < g.ntiles; t++) {
+    TileRec& tr = g.tiles[t];
+    std::memset(&tr, 0, sizeof(TileRec));
+    int ntri = std::min(kTile, nt - t * kTile);
+    tr.ntri = ntri;
+    tr.nlv = local_vertices(g, t * kTile, ntri, 3, 1, t, stamp, local, tr.vid, tr.lv_ptr, tr.lv_corner, tr.corner_lv);
+  }
+  // the same for the 32-triangle blocks (corner a of triangle t at 32 a + t)
+  g.nblocks = (nt + kBlock - 1) / kBlock;
+  g.blocks.assign(g.nblocks, BlockRec{});
+  for (int t = 0; t < g.nblocks; t++) {
+    BlockRec& br = g.blocks[t];
+    const int ntri = std::min(kBlock, nt - t * kBlock);
+    br.nlv = local_vertices(g, t * kBlock, ntri, 1, kBlock, g.ntiles + t, stamp, local, br.vid, br.ptr, br.corner,
+                            nullptr);
+    for (int l = 0; l < br.nlv; l++) br.most = std::max(br.most, br.ptr[l + 1] - br.ptr[l]);
   }
 
   // workspace layout
@@ -230,7 +405,9 @@ int analyse_host(HostGeom& g) {
   h.off_vertices = take(sizeof(float) * 3 * (size_t)nv);
   h.off_triangles = take(sizeof(int) * 3 * (size_t)nt);
   h.off_perm = take(sizeof(int) * (size_t)nt);
+  h.off_slots = take(sizeof(int) * (size_t)nt);
   h.off_tiles = take(sizeof(TileRec) * (size_t)g.ntiles);
+  h.off_blocks = take(sizeof(BlockRec) * (size_t)g.nblocks);
   h.off_edge_pairs = take(sizeof(int2) * (size_t)std::max(1, h.n_edge));
   h.off_vert_pairs = take(sizeof(int2) * (size_t)std::max(1, h.n_vert));
   h.off_trirec = take(sizeof(TriRec) * (size_t)nt);
@@ -244,7 +421,8 @@ int analyse_host(HostGeom& g) {
 
 // FP64 per-triangle records; launched over sorted positions.
 __global__ void geom_records_kernel(int nt, const float* __restrict__ verts, const int* __restrict__ tris,
-                                    const int* __restrict__ perm, TriRec* __restrict__ rec_sorted,
+                                    const int* __restrict__ perm, const int* __restrict__ slots,
+                                    TriRec* __restrict__ rec_sorted,
                                     TriRec* __restrict__ rec_orig, float* __restrict__ normals,
                                     float* __restrict__ curls, BmRec* __restrict__ bm) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -284,9 +462,21 @@ __global__ void geom_records_kernel(int nt, const float* __restrict__ verts, con
   r.v[1] = id[1];
   r.v[2] = id[2];
   r.h = (float)dot3(n, p[0]);
-  r.pad = 0.f;
-  rec_sorted[s] = r;
+  r.leave = 0;
   rec_orig[i] = r;
+  // the sorted record holds local vertex slot[a] in slot a
+  const int code = slots[s];
+  const int slot[3] = {code & 3, (code >> 2) & 3, (code >> 4) & 3};
+  TriRec rs = r;
+  rs.leave = (code >> 8) & 7;
+  for (int a = 0; a < 3; a++) {
+    rs.v[a] = id[slot[a]];
+    for (int c = 0; c < 3; c++) {
+      rs.qp[3 * a + c] = r.qp[3 * slot[a] + c];
+      rs.qp[9 + 3 * a + c] = r.qp[9 + 3 * slot[a] + c];
+    }
+  }
+  rec_sorted[s] = rs;
   normals[3 * i] = r.n[0];
   normals[3 * i + 1] = r.n[1];
   normals[3 * i + 2] = r.n[2];
@@ -300,16 +490,19 @@ __global__ void geom_records_kernel(int nt, const float* __restrict__ verts, con
   BmRec m;
   for (int b = 0; b < 3; b++) {
     d3 c = cross3(n, gr[b]);
-    curls[9 * i + 3 * b] = m.curl[3 * b] = (float)c.x;
-    curls[9 * i + 3 * b + 1] = m.curl[3 * b + 1] = (float)c.y;
-    curls[9 * i + 3 * b + 2] = m.curl[3 * b + 2] = (float)c.z;
+    curls[9 * i + 3 * b] = (float)c.x;
+    curls[9 * i + 3 * b + 1] = (float)c.y;
+    curls[9 * i + 3 * b + 2] = (float)c.z;
   }
+  for (int a = 0; a < 3; a++)
+    for (int c = 0; c < 3; c++) m.curl[3 * a + c] = curls[9 * i + 3 * slot[a] + c];
   // 3-point degree-2 rule: point q = 2/3 vertex q + 1/6 (each other vertex)
   for (int q = 0; q < 3; q++) {
     const double own = 2.0 / 3.0 - 1.0 / 6.0, all = 1.0 / 6.0;
-    m.qp[3 * q] = (float)(all * (p[0].x + p[1].x + p[2].x) + own * p[q].x);
-    m.qp[3 * q + 1] = (float)(all * (p[0].y + p[1].y + p[2].y) + own * p[q].y);
-    m.qp[3 * q + 2] = (float)(all * (p[0].z + p[1].z + p[2].z) + own * p[q].z);
+    const d3 pq = p[slot[q]];
+    m.qp[3 * q] = (float)(all * (p[0].x + p[1].x + p[2].x) + own * pq.x);
+    m.qp[3 * q + 1] = (float)(all * (p[0].y + p[1].y + p[2].y) + own * pq.y);
+    m.qp[3 * q + 2] = (float)(all * (p[0].z + p[1].z + p[2].z) + own * pq.z);
   }
   m.pad[0] = m.pad[1] = 0.f;
   bm[s] = m;
@@ -355,14 +548,17 @@ int geom_view(const void* geom, GeomView* v, GeomHeader* out_hdr) {
   v->nv = h.nv;
   v->nt = h.nt;
   v->ntiles = h.ntiles;
+  v->nblocks = (h.nt + kBlock - 1) / kBlock;
   v->n_edge = h.n_edge;
   v->n_vert = h.n_vert;
   v->vertices = (const float*)(b + h.off_vertices);
   v->triangles = (const int*)(b + h.off_triangles);
   v->perm = (const int*)(b + h.off_perm);
+  v->slots = (const int*)(b + h.off_slots);
   v->rec = (const TriRec*)(b + h.off_trirec);
   v->rec_orig = (const TriRec*)(b + h.off_trirec_orig);
   v->tiles = (const TileRec*)(b + h.off_tiles);
+  v->blocks = (const BlockRec*)(b + h.off_blocks);
   v->edge_pairs = (const int2*)(b + h.off_edge_pairs);
   v->vert_pairs = (const int2*)(b + h.off_vert_pairs);
   v->normals = (const float*)(b + h.off_normals);
@@ -407,6 +603,8 @@ extern "C" int bem_geometry_build(const float* vertices, int nv, const int* tria
     std::memcpy(st + h.off_vertices, g.vertices.data(), sizeof(float) * 3 * (size_t)nv);
     std::memcpy(st + h.off_triangles, g.triangles.data(), sizeof(int) * 3 * (size_t)nt);
     std::memcpy(st + h.off_perm, g.perm.data(), sizeof(int) * (size_t)nt);
+    std::memcpy(st + h.off_slots, g.slots.data(), sizeof(int) * (size_t)nt);
+    std::memcpy(st + h.off_blocks, g.blocks.data(), sizeof(BlockRec) * (size_t)g.nblocks);
     std::memcpy(st + h.off_tiles, g.tiles.data(), sizeof(TileRec) * (size_t)g.ntiles);
     if (h.n_edge) std::memcpy(st + h.off_edge_pairs, g.edge_pairs.data(), sizeof(int2) * h.n_edge);
     if (h.n_vert) std::memcpy(st + h.off_vert_pairs, g.vert_pairs.data(), sizeof(int2) * h.n_vert);
@@ -416,7 +614,7 @@ extern "C" int bem_geometry_build(const float* vertices, int nv, const int* tria
   char* b = (char*)geom;
   (geom_records_kernel<<<(nt + 127) / 128, 128, 0, s>>>(
       nt, (const float*)(b + h.off_vertices), (const int*)(b + h.off_triangles), (const int*)(b + h.off_perm),
-      (TriRec*)(b + h.off_trirec), (TriRec*)(b + h.off_trirec_orig), (float*)(b + h.off_normals),
+      (const int*)(b + h.off_slots), (TriRec*)(b + h.off_trirec), (TriRec*)(b + h.off_trirec_orig), (float*)(b + h.off_normals),
       (float*)(b + h.off_curls), (BmRec*)(b + h.off_bmrec)), count_launch());
   BEM_CUDA_TRY(cudaGetLastError());
   BEM_CUDA_TRY(cudaStreamSynchronize(s));  // the staging buffer serves the next build of this thread

@@ -1,0 +1,252 @@
+// Strip sweep of regular triangle pairs, shared by the V/K and the
+// Burton-Miller assembly.
+//
+// The sorted triangles come in blocks of 32 whose members are ordered as
+// paths over shared edges (geometry.cu).  A warp owns one test block (a test
+// triangle per lane) and walks along a trial block: all lanes meet the same
+// trial triangle at the same time, consecutive trial triangles keep their
+// shared vertices in the same local slots, so the 3 x 3 blocks of a pair are
+// summed in registers, by trial slot, until the slot's vertex leaves the path.
+// Only then (about 1.2 columns per trial triangle instead of 3) the column is
+// reduced over the block's test corners in the warp's own shared memory and
+// added to the matrices.  Nothing is shared between warps: no block barrier,
+// and a warp's reduction overlaps the other warps' arithmetic.
+//
+#pragma once
+
+#include "async_copy.cuh"
+#include "bem_common.cuh"
+
+namespace bemb {
+
+constexpr int kStripThreads = 128;
+constexpr int kStripWarps = kStripThreads / 32;
+constexpr int kStripZero = kBlockCorners;  // index of a column entry that stays zero
+
+// One warp's shared memory: the trial block being walked and the next one
+// (bulk copies), ROWS values per test triangle (structure of arrays), and two
+// columns of corner values (three complex numbers per test corner).
+template <int ROWS, bool BM>
+struct StripWarp {
+  TriRec trial[2][kBlock];
+  BmRec trial_bm[BM ? 2 : 1][BM ? kBlock : 1];
+  float xs[ROWS][32];
+  float4 col4[2][kBlockCorners + 1];
+  float2 col2[2][kBlockCorners + 1];
+  uint64_t full[2];
+};
+
+// The warp's position: test block `grp`, its lane's triangle and the lane's
+// entry of the block's vertex table.
+struct StripTest {
+  int grp = -1;
+  bool valid;
+  float area, nx, ny, nz, cx, cy, cz;
+  int v0, v1, v2;
+  int nlv, most;   // distinct vertices of the block, most corners of one vertex
+  int vid;         // vertex `lane` (or -1), its corners as bytes (8 at most), their number
+  unsigned c_lo, c_hi;
+  int corners;
+};
+
+__device__ __forceinline__ void strip_load_test(StripTest& t, const GeomView& g, int grp) {
+  const int lane = threadIdx.x & 31;
+  t.grp = grp;
+  const int ti = grp * kBlock + lane;
+  t.valid = ti < g.nt;
+  const TriRec& r = g.rec[t.valid ? ti : g.nt - 1];
+  t.area = r.area;
+  t.nx = r.n[0];
+  t.ny = r.n[1];
+  t.nz = r.n[2];
+  t.cx = r.c[0];
+  t.cy = r.c[1];
+  t.cz = r.c[2];
+  t.v0 = r.v[0];
+  t.v1 = r.v[1];
+  t.v2 = r.v[2];
+  const BlockRec& b = g.blocks[grp];
+  t.nlv = b.nlv;
+  t.most = b.most < 8 ? b.most : 8;
+  t.vid = -1;
+  t.corners = 0;
+  t.c_lo = t.c_hi = kStripZero * 0x01010101u;
+  if (lane < b.nlv) {
+    const int p0 = b.ptr[lane];
+    t.corners = b.ptr[lane + 1] - p0;
+    t.vid = b.vid[lane];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (i < t.corners) {
+        const unsigned c = b.corner[p0 + i];
+        const int sh = 8 * (i & 3);
+        if (i < 4)
+          t.c_lo = (t.c_lo & ~(0xffu << sh)) | (c << sh);
+        else
+          t.c_hi = (t.c_hi & ~(0xffu << sh)) | (c << sh);
+      }
+  }
+}
+
+// Lane 0: bulk-copy trial block jb into buffer b.
+template <int ROWS, bool BM>
+__device__ __forceinline__ void strip_fetch(StripWarp<ROWS, BM>& sw, const GeomView& g, int jb, int b) {
+  const int ntri = min(kBlock, g.nt - jb * kBlock);
+  const uint32_t rb = (uint32_t)(ntri * sizeof(TriRec)), mb = BM ? (uint32_t)(ntri * sizeof(BmRec)) : 0u;
+  mbar_expect_tx(&sw.full[b], rb + mb);
+  bulk_load(sw.trial[b], &g.rec[jb * kBlock], rb, &sw.full[b]);
+  if (BM) bulk_load(sw.trial_bm[BM ? b : 0], &g.bm[jb * kBlock], mb, &sw.full[b]);
+}
+
+template <int ROWS, bool BM>
+__device__ __forceinline__ void strip_init(StripWarp<ROWS, BM>& sw) {
+  if ((threadIdx.x & 31) == 0) {
+    mbar_init(&sw.full[0], 1);
+    mbar_init(&sw.full[1], 1);
+    mbar_init_fence();
+    for (int i = 0; i < 2; i++) {
+      sw.col4[i][kStripZero] = make_float4(0.f, 0.f, 0.f, 0.f);
+      sw.col2[i][kStripZero] = make_float2(0.f, 0.f);
+    }
+  }
+  __syncwarp();
+}
+
+// The two columns in col4/col2 (corner a of lane t at 32 a + t; trial vertices
+// b0 and b1, b1 < 0 if there is one column only) summed over the test corners
+// of each distinct vertex A of the block, handed to store(A, b, sum4, sum2).
+// Two at a time, since the sums are short chains of shared-memory loads.
+// Lane l takes vertices l, l + 32, ...; the first 8 corners of vertex `lane`
+// sit in registers, what lies beyond (blocks with more than 32 vertices,
+// vertices with more than 8 corners in one block) is read from the block's
+// table.
+template <int ROWS, bool BM, typename F>
+__device__ __forceinline__ void strip_reduce(StripWarp<ROWS, BM>& sw, const StripTest& t, const GeomView& g, int b0,
+                                             int b1, F&& store) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();  // the columns are complete
+  float4 s4[2];
+  float2 s2[2];
+  auto clear = [&]() {
+    s4[0] = s4[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    s2[0] = s2[1] = make_float2(0.f, 0.f);
+  };
+  auto add = [&](int c) {
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const float4 x = sw.col4[i][c];
+      const float2 y = sw.col2[i][c];
+      s4[i].x += x.x;
+      s4[i].y += x.y;
+      s4[i].z += x.z;
+      s4[i].w += x.w;
+      s2[i].x += y.x;
+      s2[i].y += y.y;
+    }
+  };
+  clear();
+  unsigned lo = t.c_lo, hi = t.c_hi;
+  for (int i = 0; i < t.most; i += 2) {  // unused places point at the zero entry
+    add(lo & 0xff);
+    add((lo >> 8) & 0xff);
+    lo = __funnelshift_r(lo, hi, 16);
+    hi >>= 16;
+  }
+  if (t.corners > 8) {
+    const BlockRec& b = g.blocks[t.grp];
+    for (int i = b.ptr[lane] + 8; i < b.ptr[lane + 1]; i++) add(b.corner[i]);
+  }
+  if (t.vid >= 0) {
+    store(t.vid, b0, s4[0], s2[0]);
+    if (b1 >= 0) store(t.vid, b1, s4[1], s2[1]);
+  }
+  for (int l = lane + 32; l < t.nlv; l += 32) {
+    const BlockRec& b = g.blocks[t.grp];
+    clear();
+    for (int i = b.ptr[l]; i < b.ptr[l + 1]; i++) add(b.corner[i]);
+    store(b.vid[l], b0, s4[0], s2[0]);
+    if (b1 >= 0) store(b.vid[l], b1, s4[1], s2[1]);
+  }
+  __syncwarp();  // the columns may be overwritten
+}
+
+// Walks steps [pos, end) of one problem: step 32 u + t is trial triangle t of
+// unit u, the units being (test block, trial block at or after it) in order
+// (tile_units_before).  `uses` counts the trial blocks this warp has fetched
+// (buffer uses & 1, mbarrier parity (uses >> 1) & 1).  Pol provides
+//   load(sw, t, g, lane)                  the test block's rows of sw.xs,
+//   pair(sw, t, rec, bm record, weight)   adds the pair's blocks,
+//   take<B>(sw, i, lane)                  moves trial slot B's column into
+//                                         sw.col4[i] / sw.col2[i] and clears it,
+//   store(g, A, B, sum4, sum2)            adds the sums of vertices (A, B).
+template <int ROWS, bool BM, typename Pol>
+__device__ __forceinline__ void strip_walk(StripWarp<ROWS, BM>& sw, StripTest& test, const GeomView& g, Pol& pol,
+                                           long long pos, long long end, unsigned& uses, int* process_err) {
+  const int lane = threadIdx.x & 31;
+  if (pos >= end) return;
+  const int nb = g.nblocks;
+  int grp = tile_group_of(pos >> 5, nb);
+  int jb = grp + (int)((pos >> 5) - tile_units_before(grp, nb));
+  if (lane == 0) strip_fetch(sw, g, jb, uses & 1);
+  for (; pos < end; uses++) {
+    const int t0 = (int)(pos & 31), t1 = (int)(end - pos < 32 - t0 ? t0 + (end - pos) : 32);
+    const int bf = uses & 1;
+    pos += t1 - t0;
+    int next_grp = grp, next_jb = jb + 1;
+    if (next_jb == nb) next_jb = ++next_grp;
+    __syncwarp();  // every lane is done with buffer bf ^ 1 and with xs
+    if (lane == 0 && pos < end) strip_fetch(sw, g, next_jb, bf ^ 1);
+    if (grp != test.grp) {
+      strip_load_test(test, g, grp);
+      pol.load(sw, test, g, lane);
+    }
+    if (!mbar_wait(&sw.full[bf], (uses >> 1) & 1u, g.err)) {
+      // expired (this geometry's status word raised): record it process-wide
+      // too, and let the copy land before the buffer is reused
+      if (lane == 0) atomicExch(process_err, 1);
+      mbar_wait_drain(&sw.full[bf], (uses >> 1) & 1u);
+    }
+    __syncwarp();  // xs is written
+    const int stop = min(t1, g.nt - jb * kBlock);
+    int waiting = -1;  // trial vertex of the column in col4[0], if one waits for the next
+#pragma unroll 1
+    for (int t = t0; t < stop; t++) {
+      const TriRec& rj = sw.trial[bf][t];
+      const int j0 = rj.v[0], j1 = rj.v[1], j2 = rj.v[2];
+      const bool touching = (test.v0 == j0) | (test.v0 == j1) | (test.v0 == j2) | (test.v1 == j0) | (test.v1 == j1) |
+                            (test.v1 == j2) | (test.v2 == j0) | (test.v2 == j1) | (test.v2 == j2);
+      // on the test block itself each unordered pair once
+      const bool once = jb > grp || t > lane;
+      const float w = (test.valid && !touching && once) ? test.area * rj.area : 0.f;
+      if (__any_sync(0xffffffffu, w != 0.f)) pol.pair(sw, test, rj, sw.trial_bm[BM ? bf : 0][BM ? t : 0], w, lane);
+      const bool last = t + 1 == stop;
+      const int leave = last ? 7 : rj.leave;  // slots whose vertex leaves the path
+#pragma unroll 1
+      for (int b = 0; b < 3; b++) {  // one copy of the reduction (instruction cache)
+        if (!((leave >> b) & 1)) continue;
+        const int at = waiting >= 0;
+        if (b == 0)
+          pol.template take<0>(sw, at, lane);
+        else if (b == 1)
+          pol.template take<1>(sw, at, lane);
+        else
+          pol.template take<2>(sw, at, lane);
+        const int vertex = b == 0 ? j0 : (b == 1 ? j1 : j2);
+        if (at || (last && b == 2)) {
+          strip_reduce(sw, test, g, at ? waiting : vertex, at ? vertex : -1,
+                       [&](int A, int B, const float4& s4, const float2& s2) { pol.store(g, A, B, s4, s2); });
+          waiting = -1;
+        } else {
+          waiting = vertex;
+        }
+      }
+    }
+    grp = next_grp;
+    jb = next_jb;
+  }
+}
+
+// Steps of a problem's walk.
+inline long long strip_steps(int nblocks) { return 32LL * nblocks * (nblocks + 1) / 2; }
+
+}  // namespace bemb

@@ -1,0 +1,85 @@
+"""Strip walk of the regular pairs (V/K and Burton-Miller) at the edges of its
+32-triangle blocks: meshes smaller than a block, one triangle more or less
+than a block, blocks of disjoint triangles (96 vertices), vertices with more
+corners in one block than a lane keeps in registers, against the FP64 oracle.
+
+Tolerance: 1e-5 relative Frobenius norm, the bar of every assembled matrix.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5
+
+
+def patch(count, seed):
+    """The first `count` triangles of a bumpy grid, vertices renumbered."""
+    n = 9
+    i, j = np.meshgrid(np.arange(n), np.arange(n), indexing="ij")
+    v = np.stack([0.05 * i, 0.05 * j, 0.01 * np.sin(1.3 * i + 0.7 * j)], -1).reshape(-1, 3)
+    t = []
+    for a in range(n - 1):
+        for b in range(n - 1):
+            p = a * n + b
+            t += [(p, p + n, p + 1), (p + 1, p + n, p + n + 1)]
+    t = np.array(t)[:count]
+    used, t = np.unique(t, return_inverse=True)
+    return v[used], t.reshape(-1, 3)
+
+
+def fan(count):
+    """A cone of `count` triangles around one vertex."""
+    a = 2 * np.pi * np.arange(count) / count
+    v = np.concatenate([[[0.0, 0.0, 0.05]], np.stack([0.2 * np.cos(a), 0.2 * np.sin(a), 0 * a], 1)])
+    k = np.arange(count)
+    return v, np.stack([0 * k, 1 + k, 1 + (k + 1) % count], 1)
+
+
+def soup(count, seed):
+    """Disjoint triangles."""
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-0.3, 0.3, (count, 1, 3))
+    v = (c + rng.uniform(-0.02, 0.02, (count, 3, 3))).reshape(-1, 3)
+    return v, np.arange(3 * count).reshape(-1, 3)
+
+
+MESHES = {
+    "one triangle": lambda: patch(1, 0), "two triangles": lambda: patch(2, 0), "31": lambda: patch(31, 1),
+    "32": lambda: patch(32, 2), "33": lambda: patch(33, 3), "65": lambda: patch(65, 4), "fan 40": lambda: fan(40),
+    "disjoint 33": lambda: soup(33, 5),
+}
+
+
+def rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("name", list(MESHES))
+def test_block_edges(name):
+    import torch
+
+    from neuralat_b200.bem import BEM_Solver
+    from neuralat_b200.bem.batch import assemble_batch, assemble_batch_bm
+
+    O.build()
+    v, t = MESHES[name]()
+    v, t, k = v.astype(np.float32), t.astype(np.int32), 21.7
+    s = BEM_Solver(torch.from_numpy(v).cuda(), torch.from_numpy(t).cuda())
+    v64, M = v.astype(np.float64), O.identity_matrix(v.astype(np.float64), t)
+    V, A = (x.cpu().numpy() for x in s.assemble_vk(k))
+    K = O.boundary_matrix("double", v64, t, k)
+    assert rel(V, O.boundary_matrix("single", v64, t, k)) < TOL
+    assert rel(A, 0.5 * M - K) < TOL
+    (Vb, Ab), = assemble_batch([s], [k])
+    assert rel(Vb.cpu().numpy(), V) < 1e-6 and rel(Ab.cpu().numpy(), A) < 1e-6
+    for approx, order in ((True, "_approx"), (False, "")):
+        L, R = (x.cpu().numpy() for x in s.assemble_bm(k, approx=approx))
+        assert rel(L, O.boundary_matrix("bm_lhs", v64, t, k, order) + 0.5 * M) < TOL
+        assert rel(R, O.boundary_matrix("bm_rhs", v64, t, k, order) - 0.5j / k * M) < TOL
+        (Lb, Rb), = assemble_batch_bm([s], [k], approx=approx)
+        assert rel(Lb.cpu().numpy(), L) < 1e-6 and rel(Rb.cpu().numpy(), R) < 1e-6
+    for layer in ("hypersingular", "bm_lhs"):  # the sorted records' curls in the general kernel
+        got = s.assemble_boundary_matrix(k, layer, approx=True).cpu().numpy()
+        assert rel(got, O.boundary_matrix(layer, v64, t, k, "_approx")) < TOL
