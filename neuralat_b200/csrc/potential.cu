@@ -6,11 +6,16 @@
 // src/bem/solver.py:128-147 (matrix times vector), bind.cu:23-48
 // (triangle2vertex).
 //
-// B200 design: `boundary2potential` never materialises the P x N matrices.
-// The P1 densities are first interpolated onto the 6T quadrature points
-// (one small pass), after which the listener sum is a dense, atomic-free
-// "N-body" contraction: each lane owns a listener, warps stream quadrature
-// points, and S and D share one distance and one sincos.
+// B200 design: `boundary2potential` never materialises the P x N matrices.  A
+// thread owns a listener and walks along the sorted triangles, whose order
+// keeps shared vertices in their slots (BlockRec): S and D share one distance
+// and one sincos per quadrature point, and the potentials of a vertex are
+// summed in registers until it leaves the path.  Only then they meet the
+// right-hand sides, once per path vertex (1.15 per triangle) instead of once
+// per quadrature point (6 per triangle).
+
+#include <algorithm>
+#include <atomic>
 
 #include "bem_common.cuh"
 
@@ -61,100 +66,252 @@ __global__ void potential_matrix_kernel(GeomView g, const float* __restrict__ pt
     atomicAdd(&out[(size_t)p * g.nv + r.v[b]], make_float2(acc[b].x * sc, acc[b].y * sc));
 }
 
-// Densities on quadrature points: dens[(6 j + q) * nrhs + s] =
-//   area_j w_q sum_b phi_b(q) u[v_b(j), s]   for u = neumann (slot 0) and dirichlet (slot 1).
-__global__ void b2p_density_kernel(GeomView g, const float2* __restrict__ neu, const float2* __restrict__ dir,
-                                   int nrhs, float2* __restrict__ dn_out, float2* __restrict__ dd_out) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)g.nt * 6 * nrhs;
-  if (idx >= total) return;
-  const int s = (int)(idx % nrhs);
-  const int jq = (int)(idx / nrhs);
-  const int j = jq / 6, q = jq - 6 * (jq / 6);
-  const TriRec& r = g.rec_orig[j];
-  float2 an = make_float2(0.f, 0.f), ad = make_float2(0.f, 0.f);
+// Sums of one listener's potentials over the path, per trial slot: S phi_b and
+// D phi_b, (re, im), without the sign of the double layer.
+struct ListenSums {
+  float2 s[3], d[3];
+};
+
+// Adds one triangle.  The rule's symmetry as in the assembly: with g_b, h_b
+// the values at the two points of vertex b, the sum for b is
+// own_1 (g_b + rho h_b + tau sum_c (g_c + sigma h_c)).
+__device__ __forceinline__ void listen_triangle(const TriRec& r, float px, float py, float pz, float k,
+                                                ListenSums& acc) {
+  constexpr float kRho = (float)(tri6_w_own(3) / tri6_w_own(0)), kSigma = (float)(tri6_w_common(3) / tri6_w_common(0)),
+                  kTau = (float)(tri6_w_common(0) / tri6_w_own(0));
+  const float4* r4 = (const float4*)&r;
+  const float4 q0 = r4[0], q1 = r4[1], q2 = r4[2], q3 = r4[3], q4 = r4[4], q5 = r4[5];
+  const float2 yx[3] = {{q0.x, q2.y}, {q0.w, q3.x}, {q1.z, q3.w}};
+  const float2 yy[3] = {{q0.y, q2.z}, {q1.x, q3.y}, {q1.w, q4.x}};
+  const float2 yz[3] = {{q0.z, q2.w}, {q1.y, q3.z}, {q2.x, q4.y}};
+  const float dn = q4.z * (q5.y - px) + q4.w * (q5.z - py) + q5.x * (q5.w - pz);  // n . (y - x) on the plane
+  const float2 k2 = f2(k), nk2 = f2(-k);
+  float2 tS[3], tD[3], sSr, sSi, sDr, sDi;
 #pragma unroll
   for (int b = 0; b < 3; b++) {
-    const float f = (float)tri6_phi(q, b);
-    if (neu) {
-      const float2 u = neu[(size_t)r.v[b] * nrhs + s];
-      an.x = fmaf(f, u.x, an.x);
-      an.y = fmaf(f, u.y, an.y);
-    }
-    if (dir) {
-      const float2 u = dir[(size_t)r.v[b] * nrhs + s];
-      ad.x = fmaf(f, u.x, ad.x);
-      ad.y = fmaf(f, u.y, ad.y);
-    }
-  }
-  const float w = (float)tri6_w(q) * r.area * kInv4Pi;
-  dn_out[idx] = make_float2(-an.x * w, -an.y * w);  // -S applied to neumann
-  dd_out[idx] = make_float2(ad.x * w, ad.y * w);
-}
-
-constexpr int kB2PThreads = 256;
-
-// out[p, s] += sum_{jq in chunk} G(x_p, y_jq) dn[jq, s] + D(x_p, y_jq) dd[jq, s]
-// (the -1, the weights and 1/(4 pi) are inside dn/dd).  Block = 32 listeners
-// (lanes) x one chunk of quadrature points split over 8 warps; kB2PRhs
-// right-hand sides per pass (8, or 16 for more than 8 right-hand sides: the
-// distances and sin/cos are computed once per pass).
-template <int kB2PRhs>
-__global__ void __launch_bounds__(kB2PThreads)
-    b2p_eval_kernel(GeomView g, const float* __restrict__ pts, int np, float k, const float2* __restrict__ dn,
-                    const float2* __restrict__ dd, int nrhs, int rhs0, int chunk, float2* __restrict__ out) {
-  __shared__ float2 red[kB2PThreads / 32][32][kB2PRhs];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p = blockIdx.x * 32 + lane;
-  const bool valid = p < np;
-  const float px = valid ? pts[3 * p] : 0.f, py = valid ? pts[3 * p + 1] : 0.f, pz = valid ? pts[3 * p + 2] : 0.f;
-  const int nq = 6 * g.nt;
-  const int q0 = blockIdx.y * chunk, q1 = min(q0 + chunk, nq);
-  const int ns = min(kB2PRhs, nrhs - rhs0);
-  float2 acc[kB2PRhs];
-#pragma unroll
-  for (int s = 0; s < kB2PRhs; s++) acc[s] = make_float2(0.f, 0.f);
-  for (int jq = q0 + warp; jq < q1; jq += kB2PThreads / 32) {
-    const int j = jq / 6, q = jq - 6 * j;
-    const TriRec& r = g.rec_orig[j];
-    const float dx = r.qp[3 * q] - px, dy = r.qp[3 * q + 1] - py, dz = r.qp[3 * q + 2] - pz;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    const float rinv = fminf(rsqrtf(r2), 1.0f / kEps);
-    const float rr = fmaxf(r2 * rinv, kEps);
+    const float2 dx = f2_sub(yx[b], f2(px)), dy = f2_sub(yy[b], f2(py)), dz = f2_sub(yz[b], f2(pz));
+    float2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+    r2.x = fmaxf(r2.x, kEps * kEps);  // r >= 1e-3, to a rounding
+    r2.y = fmaxf(r2.y, kEps * kEps);
+    const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+    const float2 kr = f2_mul(k2, f2_mul(r2, ri)), ri2 = f2_mul(ri, ri);
     // hardware sin/cos: the FP32 phase k r carries a relative error of ~2^-24,
     // which the hardware evaluation keeps (a few 1e-6 rad at k r ~ 100)
-    float sn, cs;
-    __sincosf(k * rr, &sn, &cs);
-    const float gr = cs * rinv, gi = sn * rinv;
-    const float dnv = dx * r.n[0] + dy * r.n[1] + dz * r.n[2];
-    const float f = -dnv * rinv * rinv;
-    const float kr = k * rr;
-    const float dr = (cs + kr * sn) * rinv * f, di = (sn - kr * cs) * rinv * f;
-    const float2* pn = dn + (size_t)jq * nrhs + rhs0;
-    const float2* pd = dd + (size_t)jq * nrhs + rhs0;
+    float2 sn, cs;
+    __sincosf(kr.x, &sn.x, &cs.x);
+    __sincosf(kr.y, &sn.y, &cs.y);
+    const float2 gr = f2_mul(cs, ri), gi = f2_mul(sn, ri);
+    const float2 hr = f2_mul(f2_fma(k2, sn, gr), ri2), hi = f2_mul(f2_fma(nk2, cs, gi), ri2);
+    tS[b] = make_float2(fmaf(kRho, gr.y, gr.x), fmaf(kRho, gi.y, gi.x));
+    tD[b] = make_float2(fmaf(kRho, hr.y, hr.x), fmaf(kRho, hi.y, hi.x));
+    sSr = b ? f2_add(sSr, gr) : gr;
+    sSi = b ? f2_add(sSi, gi) : gi;
+    sDr = b ? f2_add(sDr, hr) : hr;
+    sDi = b ? f2_add(sDi, hi) : hi;
+  }
+  const float2 sS = make_float2(fmaf(kSigma, sSr.y, sSr.x), fmaf(kSigma, sSi.y, sSi.x));
+  const float2 sD = make_float2(fmaf(kSigma, sDr.y, sDr.x), fmaf(kSigma, sDi.y, sDi.x));
+  const float ws = r.area * (float)(tri6_w_own(0) / (4.0 * kPi)), wd = ws * dn;
 #pragma unroll
-    for (int s = 0; s < kB2PRhs; s++) {
-      if (s < ns) {
-        const float2 a = pn[s], b = pd[s];
-        acc[s].x += gr * a.x - gi * a.y + dr * b.x - di * b.y;
-        acc[s].y += gr * a.y + gi * a.x + dr * b.y + di * b.x;
+  for (int b = 0; b < 3; b++) {
+    acc.s[b] = f2_fma(f2(ws), f2_fma(f2(kTau), sS, tS[b]), acc.s[b]);
+    acc.d[b] = f2_fma(f2(wd), f2_fma(f2(kTau), sD, tD[b]), acc.d[b]);
+  }
+}
+
+constexpr int kLsThreads = 128;  // listeners per CTA
+
+// out[p, s] += -S neumann + D dirichlet over the triangles of one run
+// (blockIdx.y), for up to M <= 4 right-hand sides: the products with the
+// vertex densities stay in the listener's own registers.
+//
+// Bound by the FP32 and sincos units (about 125 instructions for the 6 points
+// of a triangle).  Measured on B200: 1000 listeners x 5110 triangles x 1
+// right-hand side 43 us, against 165 us with the densities
+// interpolated onto the quadrature points by a pass of their own and 8 products
+// per point and right-hand side.
+template <int M>
+__global__ void __launch_bounds__(kLsThreads)
+    listen_few_kernel(GeomView g, const float* __restrict__ pts, int np, float k, const float2* __restrict__ neu,
+                      const float2* __restrict__ dir, int nrhs, int run, float2* __restrict__ out) {
+  __shared__ TriRec rec[kBlock];
+  __shared__ float4 dens[kBlock][3][M];  // (neumann, dirichlet) at the triangle's vertices
+  const int tid = threadIdx.x, p = blockIdx.x * kLsThreads + tid;
+  const float* x = pts + 3 * (size_t)min(p, np - 1);
+  const float px = x[0], py = x[1], pz = x[2];
+  const int t0 = blockIdx.y * run, t1 = min(t0 + run, g.nt);
+  ListenSums acc;
+#pragma unroll
+  for (int b = 0; b < 3; b++) acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
+  float2 sum[M];
+#pragma unroll
+  for (int s = 0; s < M; s++) sum[s] = make_float2(0.f, 0.f);
+  for (int c0 = t0; c0 < t1; c0 += kBlock) {
+    const int n = min(kBlock, t1 - c0);
+    __syncthreads();
+    for (int e = tid; e < 8 * n; e += kLsThreads) ((float4*)rec)[e] = ((const float4*)&g.rec[c0])[e];
+    for (int e = tid; e < 3 * M * n; e += kLsThreads) {
+      const int t = e / (3 * M), b = (e / M) % 3, s = e % M;
+      const size_t at = (size_t)g.rec[c0 + t].v[b] * nrhs + s;
+      const float2 zero = make_float2(0.f, 0.f);
+      const float2 a = neu && s < nrhs ? neu[at] : zero, u = dir && s < nrhs ? dir[at] : zero;
+      dens[t][b][s] = make_float4(a.x, a.y, u.x, u.y);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int t = 0; t < n; t++) {
+      listen_triangle(rec[t], px, py, pz, k, acc);
+      const int leave = c0 + t + 1 == t1 ? 7 : rec[t].leave;
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        if (!((leave >> b) & 1)) continue;
+        const float2 sv = acc.s[b], dv = acc.d[b];
+#pragma unroll
+        for (int s = 0; s < M; s++) {
+          const float4 w = dens[t][b][s];
+          sum[s].x -= sv.x * w.x - sv.y * w.y + dv.x * w.z - dv.y * w.w;
+          sum[s].y -= sv.x * w.y + sv.y * w.x + dv.x * w.w + dv.y * w.z;
+        }
+        acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
       }
     }
   }
+  if (p < np) {
 #pragma unroll
-  for (int s = 0; s < kB2PRhs; s++) red[warp][lane][s] = acc[s];
-  __syncthreads();
-  if (warp == 0 && valid) {
-    for (int s = 0; s < ns; s++) {
-      float2 t = make_float2(0.f, 0.f);
+    for (int s = 0; s < M; s++)
+      if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], sum[s]);
+  }
+}
+
+// The same for 8 J right-hand sides at a time (from rhs0 on): a thread writes
+// its listener's path vertices as rows of a shared-memory tile; every
+// kLsRows rows the CTA multiplies the tile (128 listeners x kLsRows vertices,
+// S and D) with the densities of those vertices, a thread holding 8 listeners
+// x J right-hand sides.  The tile stores Im also negated, and the densities
+// stand twice, as the packed arithmetic takes them.
+//
+// Bound by the FP32 unit: per path vertex 16 operations per right-hand side
+// and listener, besides the 125 instructions per triangle.  Measured on B200:
+// 4096 listeners x 20 480 triangles x 64 right-hand sides 2.86 ms (one
+// pass), against 21.2 ms with 8 products per quadrature point and right-hand
+// side in four passes.
+constexpr int kLsRows = 16;
+
+template <int J>
+struct ListenSmem {
+  float w[kLsRows][6][kLsThreads];  // Re S, Im S, -Im S, Re D, Im D, -Im D
+  float4 dens[kLsRows][2][8 * J];   // (re, re, im, im) of neumann and dirichlet
+  TriRec rec[kBlock];
+  int vertex[kLsRows];
+};
+
+template <int J>
+__global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
+    listen_many_kernel(GeomView g, const float* __restrict__ pts, int np, float k, const float2* __restrict__ neu,
+                       const float2* __restrict__ dir, int nrhs, int rhs0, int run, float2* __restrict__ out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ListenSmem<J>& sm = *reinterpret_cast<ListenSmem<J>*>(smem_raw);
+  const int tid = threadIdx.x;
+  const int cg = tid & 7, lg = tid >> 3;  // right-hand sides cg + 8 j, listeners 4 lg + 64 h + 0..3
+  const float* x = pts + 3 * (size_t)min((int)blockIdx.x * kLsThreads + tid, np - 1);
+  const float px = x[0], py = x[1], pz = x[2];
+  const int t0 = blockIdx.y * run, t1 = min(t0 + run, g.nt);
+  float2 ar[4][J], ai[4][J];  // listener pairs x right-hand sides
 #pragma unroll
-      for (int w = 0; w < kB2PThreads / 32; w++) {
-        t.x += red[w][lane][s].x;
-        t.y += red[w][lane][s].y;
+  for (int l = 0; l < 4; l++)
+#pragma unroll
+    for (int j = 0; j < J; j++) ar[l][j] = ai[l][j] = make_float2(0.f, 0.f);
+  ListenSums acc;
+#pragma unroll
+  for (int b = 0; b < 3; b++) acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
+  int rows = 0;
+  for (int c0 = t0; c0 < t1; c0 += kBlock) {
+    const int n = min(kBlock, t1 - c0);
+    __syncthreads();  // everyone is done with the previous records
+    for (int e = tid; e < 8 * n; e += kLsThreads) ((float4*)sm.rec)[e] = ((const float4*)&g.rec[c0])[e];
+    __syncthreads();
+    for (int t = 0; t < n;) {
+      // ---- walk until the tile is full or the records end ----
+#pragma unroll 1
+      for (; t < n && rows + 3 <= kLsRows; t++) {
+        const TriRec& r = sm.rec[t];
+        listen_triangle(r, px, py, pz, k, acc);
+        const int leave = c0 + t + 1 == t1 ? 7 : r.leave;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          if (!((leave >> b) & 1)) continue;
+          const float2 sv = acc.s[b], dv = acc.d[b];
+          sm.w[rows][0][tid] = sv.x;
+          sm.w[rows][1][tid] = sv.y;
+          sm.w[rows][2][tid] = -sv.y;
+          sm.w[rows][3][tid] = dv.x;
+          sm.w[rows][4][tid] = dv.y;
+          sm.w[rows][5][tid] = -dv.y;
+          if (tid == 0) sm.vertex[rows] = r.v[b];
+          rows++;
+          acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
+        }
       }
-      atomicAdd(&out[(size_t)p * nrhs + rhs0 + s], t);
+      const bool last = t == n && c0 + n == t1;
+      if (!last && rows + 3 <= kLsRows) continue;  // more records first
+      __syncthreads();
+      // ---- densities of the rows' vertices, then the product ----
+      for (int e = tid; e < rows * 8 * J; e += kLsThreads) {
+        const int row = e / (8 * J), c = e - row * 8 * J;
+        const size_t at = (size_t)sm.vertex[row] * nrhs + rhs0 + c;
+        const bool in = rhs0 + c < nrhs;
+        const float2 zero = make_float2(0.f, 0.f);
+        const float2 a = neu && in ? neu[at] : zero, u = dir && in ? dir[at] : zero;
+        sm.dens[row][0][c] = make_float4(a.x, a.x, a.y, a.y);
+        sm.dens[row][1][c] = make_float4(u.x, u.x, u.y, u.y);
+      }
+      __syncthreads();
+#pragma unroll 1
+      for (int row = 0; row < rows; row++) {
+#pragma unroll
+        for (int layer = 0; layer < 2; layer++) {
+          float2 re[4], im[4], ni[4];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const float4 a = *(const float4*)&sm.w[row][3 * layer][4 * lg + 64 * h];
+            const float4 b = *(const float4*)&sm.w[row][3 * layer + 1][4 * lg + 64 * h];
+            const float4 c = *(const float4*)&sm.w[row][3 * layer + 2][4 * lg + 64 * h];
+            re[2 * h] = make_float2(a.x, a.y);
+            re[2 * h + 1] = make_float2(a.z, a.w);
+            im[2 * h] = make_float2(b.x, b.y);
+            im[2 * h + 1] = make_float2(b.z, b.w);
+            ni[2 * h] = make_float2(c.x, c.y);
+            ni[2 * h + 1] = make_float2(c.z, c.w);
+          }
+#pragma unroll
+          for (int j = 0; j < J; j++) {
+            const float4 d = sm.dens[row][layer][cg + 8 * j];
+            const float2 dr = make_float2(d.x, d.y), di = make_float2(d.z, d.w);
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+              ar[l][j] = f2_fma(ni[l], di, f2_fma(re[l], dr, ar[l][j]));
+              ai[l][j] = f2_fma(im[l], dr, f2_fma(re[l], di, ai[l][j]));
+            }
+          }
+        }
+      }
+      rows = 0;
+      __syncthreads();  // the tile may be overwritten
     }
   }
+#pragma unroll
+  for (int l = 0; l < 4; l++)
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+      const int p = blockIdx.x * kLsThreads + 4 * lg + 64 * (l >> 1) + 2 * (l & 1) + i;
+      if (p >= np) continue;
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        const int s = rhs0 + cg + 8 * j;
+        const float re = i ? ar[l][j].y : ar[l][j].x, im = i ? ai[l][j].y : ai[l][j].x;
+        if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], make_float2(-re, -im));
+      }
+    }
 }
 
 __global__ void t2v_scatter_kernel(GeomView g, const float2* __restrict__ tv, float2* __restrict__ out,
@@ -209,34 +366,80 @@ extern "C" size_t bem_boundary2potential_scratch_bytes(int nt, int nrhs) {
 }
 
 namespace bemb {
-// The densities of both layers at every quadrature point (into dn, dd: 6 nt
-// nrhs complex64 each), then the listener sums: the work of
-// bem_boundary2potential and bem_boundary2potential_noalloc, which differ
-// only in where dn and dd live.
-int b2p_enqueue(const GeomView& g, const float* points, int np, float k, const void* neumann, const void* dirichlet,
-                int nrhs, void* out, float2* dn, float2* dd, cudaStream_t s) {
-  const long long total = (long long)g.nt * 6 * nrhs;
-  (b2p_density_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(g, (const float2*)neumann,
-                                                                      (const float2*)dirichlet, nrhs, dn, dd),
+namespace {
+// Triangles per CTA so that the grid is a little below a whole number of
+// waves of `slots` CTAs: as few waves as leave at most a tenth of the last one
+// empty, and runs of at least `least` triangles (each run loads its densities
+// and adds its sums to the output) and of at most 800 or so: longer serial
+// FP32 sums cost accuracy (20 480 triangles: 2.7e-6 off the FP64 pressures
+// with 9 runs, 2.3e-6 with 27; 2.1e-6 before).
+int listen_run(int groups, int nt, long long slots, int least) {
+  long long splits = 1;
+  for (int waves = 1; waves <= 64; waves++) {
+    splits = std::max<long long>(1, waves * slots / groups);
+    if (10 * splits * groups >= 9 * waves * slots && nt <= 800 * splits) break;
+  }
+  splits = std::min<long long>(splits, 65535);
+  return (int)std::max<long long>(least, (nt + splits - 1) / splits);
+}
+
+template <int M>
+void listen_few(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
+                float2* out, int sms, cudaStream_t s) {
+  const int groups = (np + kLsThreads - 1) / kLsThreads;
+  const int run = listen_run(groups, g.nt, 8LL * sms, 4);
+  (listen_few_kernel<M><<<dim3(groups, (g.nt + run - 1) / run), kLsThreads, 0, s>>>(g, pts, np, k, neu, dir, nrhs, run,
+                                                                                 out),
    count_launch());
+}
+
+template <int J>
+int listen_many(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
+                int rhs0, float2* out, int dev, int sms, cudaStream_t s) {
+  const int smem = (int)sizeof(ListenSmem<J>);
+  static std::atomic<unsigned long long> attr{0};  // devices whose attribute is set
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (!(attr.load(std::memory_order_acquire) & bit)) {
+    BEM_CUDA_TRY(cudaFuncSetAttribute(listen_many_kernel<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr.fetch_or(bit, std::memory_order_release);
+  }
+  const int groups = (np + kLsThreads - 1) / kLsThreads;
+  const int run = listen_run(groups, g.nt, (J == 8 ? 2LL : 3LL) * sms, 12);
+  (listen_many_kernel<J><<<dim3(groups, (g.nt + run - 1) / run), kLsThreads, smem, s>>>(g, pts, np, k, neu, dir, nrhs,
+                                                                                     rhs0, run, out),
+   count_launch());
+  return BEM_OK;
+}
+}  // namespace
+
+// The work of bem_boundary2potential and bem_boundary2potential_noalloc.  Up
+// to 4 right-hand sides multiply in the listener's registers; more go through
+// the tiled product in passes of up to 64 (each pass evaluates the potentials
+// again).
+int b2p_enqueue(const GeomView& g, const float* points, int np, float k, const void* neumann, const void* dirichlet,
+                int nrhs, void* out, cudaStream_t s) {
+  const float2 *neu = (const float2*)neumann, *dir = (const float2*)dirichlet;
+  float2* o = (float2*)out;
   BEM_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float2) * (size_t)np * nrhs, s));
-  const int nq = 6 * g.nt;
-  const int ptiles = (np + 31) / 32;
-  // enough quadrature chunks to fill the GPU ~4 times
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int nchunks = (4 * sms * 4 + ptiles - 1) / ptiles;
-  int chunk = (nq + nchunks - 1) / nchunks;
-  chunk = chunk < 256 ? 256 : chunk;
-  nchunks = (nq + chunk - 1) / chunk;
-  if (nrhs <= 8) {
-    (b2p_eval_kernel<8><<<dim3(ptiles, nchunks), kB2PThreads, 0, s>>>(g, points, np, k, dn, dd, nrhs, 0, chunk,
-                                                                      (float2*)out), count_launch());
+  if (nrhs <= 4) {
+    if (nrhs == 1)
+      listen_few<1>(g, points, np, k, neu, dir, nrhs, o, sms, s);
+    else if (nrhs == 2)
+      listen_few<2>(g, points, np, k, neu, dir, nrhs, o, sms, s);
+    else
+      listen_few<4>(g, points, np, k, neu, dir, nrhs, o, sms, s);
   } else {
-    for (int r0 = 0; r0 < nrhs; r0 += 16)
-      (b2p_eval_kernel<16><<<dim3(ptiles, nchunks), kB2PThreads, 0, s>>>(g, points, np, k, dn, dd, nrhs, r0, chunk,
-                                                                         (float2*)out), count_launch());
+    for (int r0 = 0; r0 < nrhs; r0 += 64) {
+      const int left = nrhs - r0;
+      const int rc = left > 32   ? listen_many<8>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s)
+                     : left > 16 ? listen_many<4>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s)
+                     : left > 8  ? listen_many<2>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s)
+                                 : listen_many<1>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s);
+      if (rc) return rc;
+    }
   }
   BEM_CUDA_TRY(cudaGetLastError());
   return BEM_OK;
@@ -251,10 +454,9 @@ extern "C" int bem_boundary2potential(const void* geom, const float* points, int
   if (rc) return rc;
   if (np < 0 || nrhs <= 0 || (np > 0 && (!points || !out))) return BEM_ERR_INVALID_ARGUMENT;
   if (np == 0) return BEM_OK;
+  // part of the contract, although the kernels sum in registers
   if (!scratch || scratch_bytes < bem_boundary2potential_scratch_bytes(g.nt, nrhs)) return BEM_ERR_WORKSPACE;
-  float2* dn = (float2*)scratch;
-  float2* dd = dn + (size_t)g.nt * 6 * nrhs;
-  return b2p_enqueue(g, points, np, k, neumann, dirichlet, nrhs, out, dn, dd, (cudaStream_t)stream);
+  return b2p_enqueue(g, points, np, k, neumann, dirichlet, nrhs, out, (cudaStream_t)stream);
 }
 
 extern "C" int bem_triangle2vertex(const void* geom, const void* tri_values, void* out, int* counts,
@@ -280,51 +482,18 @@ extern "C" int bem_triangle2vertex(const void* geom, const void* tri_values, voi
 // must not block on the allocator (an allocation may synchronise the device
 // and miss the callback deadline), and plug-ins embedded through a plain C
 // FFI often have no device allocator of their own.  This entry point is the
-// same computation as bem_boundary2potential, with the quadrature-point
-// densities kept in a fixed array of this library's own device memory
-// instead of a caller-provided scratch buffer.
+// same computation as bem_boundary2potential without a scratch argument (the
+// kernels keep their sums in registers and shared memory).
 //
 // Contract:
-//  * the array holds 2 x kNoAllocQuadRhs complex64 values (16 MiB); every GPU
-//    that loads the library reserves it until the process exits;
-//  * requests with 6 * nt * nrhs > kNoAllocQuadRhs are rejected with
-//    BEM_ERR_WORKSPACE before any work is enqueued;
-//  * the first call on a device, with that device current, looks up the
-//    array's device address (cudaGetSymbolAddress) and caches it; make that
-//    first call before any stream capture;
-//  * all calls share the array and it keeps the last call's contents: each
-//    call overwrites every density it reads before reading it, so nothing
-//    needs clearing, but calls that overlap on the GPU (different streams,
-//    or different host threads) race on it and must be serialised by the
-//    caller;
+//  * requests with 6 * nt * nrhs > 2^20 are rejected with BEM_ERR_WORKSPACE
+//    before any work is enqueued;
+//  * calls may overlap (different streams, different host threads);
 //  * no cudaMalloc, cudaFree or allocating library routine is called.
 // ---------------------------------------------------------------------------
-#include <mutex>
-
 namespace bemb {
 namespace {
 constexpr long long kNoAllocQuadRhs = 1LL << 20;
-static __device__ __align__(256) float2 g_noalloc_density[2 * kNoAllocQuadRhs];
-std::mutex g_noalloc_mu;
-constexpr int kNoAllocMaxDevices = 64;
-float2* g_noalloc_addr[kNoAllocMaxDevices] = {};
-
-// Device address of g_noalloc_density on the current device (set-up once per
-// device; the name itself is only a host-side handle for the symbol).
-int noalloc_density(float2** out) {
-  int dev = 0;
-  BEM_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kNoAllocMaxDevices) return BEM_ERR_UNSUPPORTED;
-  std::lock_guard<std::mutex> lk(g_noalloc_mu);
-  if (!g_noalloc_addr[dev]) {
-    void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_density);
-    if (e != cudaSuccess || !p) return BEM_ERR_CUDA;
-    g_noalloc_addr[dev] = (float2*)p;
-  }
-  *out = g_noalloc_addr[dev];
-  return BEM_OK;
-}
 }  // namespace
 }  // namespace bemb
 
@@ -339,8 +508,5 @@ extern "C" int bem_boundary2potential_noalloc(const void* geom, const float* poi
   if (np < 0 || nrhs <= 0 || (np > 0 && (!points || !out))) return BEM_ERR_INVALID_ARGUMENT;
   if ((long long)6 * g.nt * nrhs > kNoAllocQuadRhs) return BEM_ERR_WORKSPACE;
   if (np == 0) return BEM_OK;
-  float2* base = nullptr;
-  if ((rc = noalloc_density(&base))) return rc;
-  return b2p_enqueue(g, points, np, k, neumann, dirichlet, nrhs, out, base, base + kNoAllocQuadRhs,
-                     (cudaStream_t)stream);
+  return b2p_enqueue(g, points, np, k, neumann, dirichlet, nrhs, out, (cudaStream_t)stream);
 }

@@ -1,0 +1,58 @@
+"""Listener evaluation at the edges of its kernels: right-hand sides around
+each variant's limit (1, 2, 4 in registers, then tiles of 8, 16, 32 and 64
+with remainders and a second pass), listeners around a CTA's 128, runs that
+end inside a block, one density only; against the FP64 oracle.
+
+Tolerance: 1e-5 relative (2-norm over the listeners, worst right-hand side):
+the FP32 phase k r <= 40 carries 40 * 2^-24 = 2.4e-6, sums of ~1e3 terms less.
+"""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5
+
+
+@pytest.fixture(scope="module")
+def solver():
+    from neuralat_b200.bem import BEM_Solver
+    from neuralat_b200.bem import meshes as M
+
+    O.build()
+    v0, t0 = M.icosphere(2, 0.1)
+    v1, t1 = M.icosphere(1, 0.07)
+    v = np.concatenate([v0 * [1.2, 0.8, 1.0], v1 + [0.3, 0.05, 0.0]]).astype(np.float32)
+    t = np.concatenate([t0, t1 + len(v0)]).astype(np.int32)[:-3]  # 397 triangles: the last block is short
+    return BEM_Solver(v, t), v.astype(np.float64), t
+
+
+@pytest.mark.parametrize("points,rhs,which", [
+    (1, 1, "both"), (127, 2, "both"), (128, 3, "both"), (129, 4, "both"), (5, 5, "both"), (129, 8, "both"),
+    (300, 9, "neumann"), (64, 16, "both"), (65, 17, "dirichlet"), (40, 33, "both"), (130, 64, "both"), (17, 70, "both"),
+    (3000, 1, "both"),
+])
+def test_listen_edges(solver, points, rhs, which):
+    import torch
+
+    s, v, t = solver
+    rng = np.random.default_rng(points * 100 + rhs)
+    x = rng.standard_normal((points, 3))
+    x = (0.6 * x / np.linalg.norm(x, axis=1, keepdims=True)).astype(np.float32)
+    g, u = ((rng.standard_normal((len(v), rhs)) + 1j * rng.standard_normal((len(v), rhs))).astype(np.complex64)
+            for _ in range(2))
+    if which == "neumann":
+        u = None
+    if which == "dirichlet":
+        g = None
+    k = 33.3
+    dev = [None if a is None else torch.from_numpy(a).cuda() for a in (g, u)]
+    got = s._b2p(k, dev[0], dev[1], torch.from_numpy(x).cuda()).cpu().numpy()
+    ref = 0
+    if g is not None:
+        ref = ref - O.potential_matrix("single", v, t, x.astype(np.float64), np.float32(k)) @ g.astype(complex)
+    if u is not None:
+        ref = ref + O.potential_matrix("double", v, t, x.astype(np.float64), np.float32(k)) @ u.astype(complex)
+    err = np.linalg.norm(got - ref, axis=0) / np.linalg.norm(ref, axis=0)
+    assert err.max() < TOL, err.max()
