@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kRegThreads, 2)
 // 61 % of its cycles, issue 61 %), of which 1.6 ms are the column reductions,
 // against 19.0 ms for 16 x 16-triangle tiles whose 3 x 3 blocks all went
 // through shared memory between block barriers.  Two CTAs of four warps per SM
-// with everything unrolled (no spills) take 14.6 ms for the whole assembly;
+// with everything unrolled (no spills) take 14.6 ms for the whole assembly,
 // three CTAs at 168 registers 15.1 ms, four at 128 registers 18.2 ms (spills).
 // ---------------------------------------------------------------------------
 constexpr float kRho = (float)(tri6_w_own(3) / tri6_w_own(0));
@@ -330,6 +330,7 @@ constexpr float kTau = (float)(tri6_w_common(0) / tri6_w_own(0));
 __device__ int g_asm_err;
 
 using VkWarp = StripWarp<18, false>;
+constexpr int kVkPanel = 8, kVkPanelItems = 64;  // strip_items
 
 struct VkStrip {
   float k, v_scale, k_scale;
@@ -453,11 +454,10 @@ struct VkStrip {
   }
 };
 
-// One problem: equal runs of `chunk` steps, one or more per warp of a
-// persistent grid (every warp gets the same amount of work).
+// One problem, its items dealt round-robin to the warps of a persistent grid.
 __global__ void __launch_bounds__(kStripThreads, 2)
     regular_strip_vk_kernel(const __grid_constant__ GeomView g, float k, float2* __restrict__ V, float2* __restrict__ K, float v_scale,
-                            float k_scale, long long chunk, long long n_steps, long long n_items) {
+                            float k_scale, StripItems P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   VkWarp& sw = reinterpret_cast<VkWarp*>(smem_raw)[threadIdx.x >> 5];
   strip_init(sw);
@@ -471,10 +471,8 @@ __global__ void __launch_bounds__(kStripThreads, 2)
   StripTest test;
   unsigned uses = 0;
   const long long warps = (long long)gridDim.x * kStripWarps;
-  for (long long item = (long long)blockIdx.x * kStripWarps + (threadIdx.x >> 5); item < n_items; item += warps) {
-    const long long pos = item * chunk;
-    strip_walk(sw, test, g, pol, pos, pos + chunk < n_steps ? pos + chunk : n_steps, uses, &g_asm_err);
-  }
+  for (long long item = (long long)blockIdx.x * kStripWarps + (threadIdx.x >> 5); item < P.items; item += warps)
+    strip_item(sw, test, g, pol, P, item, uses, &g_asm_err);
 }
 
 // ---------------------------------------------------------------------------
@@ -781,8 +779,7 @@ __global__ void __launch_bounds__(128)
 struct BatchProblem {
   GeomView g;
   float k;
-  int chunk;                // steps per item
-  long long n_steps;        // steps of the problem's strip walk
+  StripItems items;
   float2* V;
   float2* K;
   long long item_begin;   // prefix sum of regular items
@@ -807,8 +804,7 @@ __device__ __forceinline__ int find_problem(const BatchProblem* probs, int np, l
   return lo;
 }
 
-// Each unordered regular pair of every problem once; items are runs of
-// `chunk` steps of one problem's strip walk, drawn by the warps.
+// Each unordered regular pair of every problem once; the warps draw the items.
 __global__ void __launch_bounds__(kStripThreads, 2)
     regular_strip_vk_batch_kernel(BatchHeader* __restrict__ hdr, const BatchProblem* __restrict__ probs, float v_scale,
                                   float k_scale) {
@@ -833,8 +829,7 @@ __global__ void __launch_bounds__(kStripThreads, 2)
     pol.V = P.V;
     pol.K = P.K;
     test.grp = -1;  // another problem's block may have the same number
-    const long long pos = (item - P.item_begin) * P.chunk;
-    strip_walk(sw, test, P.g, pol, pos, pos + P.chunk < P.n_steps ? pos + P.chunk : P.n_steps, uses, &g_asm_err);
+    strip_item(sw, test, P.g, pol, P.items, item - P.item_begin, uses, &g_asm_err);
   }
 }
 
@@ -950,13 +945,10 @@ int launch_strip_vk(const GeomView& g, float k, float2* V, float2* K, float v_sc
   long long grid = 0;
   int rc = strip_grid(regular_strip_vk_kernel, attr, 0, &grid);
   if (rc) return rc;
-  const long long n_steps = strip_steps(g.nblocks), warps = grid * kStripWarps;
-  long long chunk = (n_steps + warps - 1) / warps;
-  if (chunk < 2) chunk = 2;
-  if (g_tune_chunk > 0) chunk = 32LL * g_tune_chunk;
-  const long long n_items = (n_steps + chunk - 1) / chunk, blocks = (n_items + kStripWarps - 1) / kStripWarps;
+  const StripItems P = strip_items(g.nv, g.nblocks, grid * kStripWarps, 2, g_tune_chunk, kVkPanel, kVkPanelItems);
+  const long long blocks = (P.items + kStripWarps - 1) / kStripWarps;
   (regular_strip_vk_kernel<<<(unsigned)(grid < blocks ? grid : blocks), kStripThreads, kStripWarps * sizeof(VkWarp), s>>>(
-       g, k, V, K, v_scale, k_scale, chunk, n_steps, n_items),
+       g, k, V, K, v_scale, k_scale, P),
    count_launch());
   BEM_CUDA_TRY(cudaGetLastError());
   return BEM_OK;
@@ -1102,9 +1094,8 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
   hh->nproblems = np;
   long long items = 0, pairs[3] = {0, 0, 0}, steps = 0;
   for (int p = 0; p < np; p++) steps += strip_steps(views[p].nblocks);
-  // about 8 items per warp, at most 16 trial blocks each
-  int chunk = (int)std::min<long long>(512, std::max<long long>(4, steps / (8 * grid * kStripWarps)));
-  if (g_tune_chunk > 0) chunk = (int)std::min<long long>(32LL * g_tune_chunk, 1 << 30);
+  // about 8 items per warp over the whole batch, at most 16 trial blocks each
+  const long long share = std::min<long long>(512, std::max<long long>(4, steps / (8 * grid * kStripWarps)));
   const size_t elem = sizeof(float2);
   for (int p = 0; p < np; p++) {
     const GeomView& g = views[p];
@@ -1115,12 +1106,11 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
     BatchProblem& P = hp[p];
     P.g = g;
     P.k = ks[p];
-    P.n_steps = strip_steps(g.nblocks);
-    P.chunk = chunk;
+    P.items = strip_items(g.nv, g.nblocks, std::max(1LL, strip_steps(g.nblocks) / share), 4, g_tune_chunk, kVkPanel, kVkPanelItems);
     P.V = Vs[p];
     P.K = Ks[p];
     P.item_begin = items;
-    items += (P.n_steps + chunk - 1) / chunk;
+    items += P.items.items;
     P.pair_begin[0] = pairs[0];
     P.pair_begin[1] = pairs[1];
     P.pair_begin[2] = pairs[2];

@@ -25,18 +25,13 @@
 //   lhs_ij = -ik nn S + T + (i/k) s cc      lhs_ji^T = -ik nn S + U + (i/k) s cc
 //   rhs_ij = -S + (i/k) U                   rhs_ji^T = -S + (i/k) T
 // with s = sum_ab S_ab (the P1 functions sum to one) and cc_ab the curl
-// products.  Work decomposition: a CTA of 8 warps owns one 16-triangle test
-// tile (test triangle = lane & 15) and sweeps 16-triangle trial tiles,
-// double-buffered in shared memory by bulk copies, each warp taking two trial
-// triangles (one per half-warp); the 3x3 blocks go to corner slabs that are
-// reduced on chip onto the tiles' distinct vertices, four vector atomics per
-// entry.  The slabs are small enough for three CTAs per SM, so one CTA's
-// reduction and barriers overlap the others' evaluation.
+// products, summed in registers along a warp's strip walk (strip.cuh).
 // Touching pairs: one warp per pair evaluates both kernels at each
 // Sauter-Schwab point (shared r and sincos); the coincident pass (FP64) adds
 // the mass terms.  A batch (meshes, wavenumbers) uses the same kernels with a
 // work queue over all problems.
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstring>
@@ -44,15 +39,11 @@
 #include "async_copy.cuh"
 #include "bem_common.cuh"
 #include "sauter_schwab.cuh"
+#include "strip.cuh"
 
 namespace bemb {
 
 namespace {
-
-constexpr int kBmThreads = 16 * kTile;       // 256: warp w takes trial triangles 2w, 2w + 1
-constexpr int kBmTest = kTile;               // test triangles per CTA (one tile), lane & 15
-constexpr int kBmCorners = 3 * kBmTest;      // 48
-constexpr int kBmStride = kTileCorners + 1;  // 49 float2: conflict-free column writes
 
 // C(q, b) = w_q phi_b(q): centroid rule 1/3; 3-point rule 1/3 * (q == b ?
 // 2/3 : 1/6); 6-point rule as the V/K assembly.
@@ -62,309 +53,208 @@ __host__ __device__ constexpr float bm_c(int q, int b) {
                  : (TN == 3 ? (q == b ? 2.0f / 9.0f : 1.0f / 18.0f) : (float)(tri6_w(q) * tri6_phi(q, b)));
 }
 
-// Coordinate c of the rule's points of a triangle (records in sorted order).
-template <int TN>
-__device__ __forceinline__ float bm_point(const TriRec& r, const BmRec& b, int c) {
-  return TN == 3 ? b.qp[c] : (TN == 6 ? r.qp[c] : r.c[c]);
-}
-
-struct BmSmem {
-  // rhs_ji[b][a] is not stored: rhs_ji^T - rhs_ij = (i/k)(T - U) =
-  // (i/k)(lhs_ij - lhs_ji^T) entry by entry, so it follows from the three
-  // reduced slots of each vertex pair.
-  float2 slotL[kBmCorners][kBmStride];   // lhs_ij[a][b] at [3 tl + a][3 tt + b]
-  float2 slotLT[kBmCorners][kBmStride];  // lhs_ji[b][a], same indexing
-  float2 slotR[kBmCorners][kBmStride];
-  float xs[18][kBmTest];                 // test quadrature points [coordinate][tl]
-  float xc[9][kBmTest];                  // test curls [3 a + d][tl]
-  TriRec trial[2][kTile];                // trial tile, double-buffered
-  BmRec trialB[2][kTile];
-  TileRec tileJ[2];
-  TileRec tileI;
-  uint64_t tile_full[2];
-};
-
 // A bounded wait of the Burton-Miller kernels expired (read by bm_status).
 __device__ int g_bm_err;
 
-__device__ __forceinline__ void bm_copy_words(void* dst, const void* src, int bytes, int tid) {
-  const int4* s = (const int4*)src;
-  int4* d = (int4*)dst;
-  for (int i = tid; i < bytes / 16; i += kBmThreads) d[i] = s[i];
+// G and H = (1 - ikr) G / r^2 (times 4 pi) at two trial points, FP32 pairs.
+__device__ __forceinline__ void bm_point2(float2 dx, float2 dy, float2 dz, float k, float2& gr, float2& gi,
+                                          float2& hr, float2& hi) {
+  float2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
+  r2.x = fmaxf(r2.x, kEps * kEps);  // r >= 1e-3, to a rounding
+  r2.y = fmaxf(r2.y, kEps * kEps);
+  const float2 ri = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 kr = f2_mul(f2(k), f2_mul(r2, ri)), ri2 = f2_mul(ri, ri);
+  float2 s, c;
+  __sincosf(kr.x, &s.x, &c.x);
+  __sincosf(kr.y, &s.y, &c.y);
+  gr = f2_mul(c, ri);
+  gi = f2_mul(s, ri);
+  hr = f2_mul(f2_fma(f2(k), s, gr), ri2);
+  hi = f2_mul(f2_fma(f2(-k), c, gi), ri2);
 }
 
-// Thread 0: bulk-copy trial tile jt (records, Burton-Miller records, vertex
-// table) into buffer b.
-__device__ __forceinline__ void bm_fetch_tile(BmSmem& sm, const GeomView& g, int jt, int b) {
-  const int ntri = min(kTile, g.nt - jt * kTile);
-  const uint32_t rb = (uint32_t)(ntri * sizeof(TriRec)), mb = (uint32_t)(ntri * sizeof(BmRec));
-  mbar_expect_tx(&sm.tile_full[b], rb + mb + (uint32_t)sizeof(TileRec));
-  bulk_load(sm.trial[b], &g.rec[jt * kTile], rb, &sm.tile_full[b]);
-  bulk_load(sm.trialB[b], &g.bm[jt * kTile], mb, &sm.tile_full[b]);
-  bulk_load(&sm.tileJ[b], &g.tiles[jt], (uint32_t)sizeof(TileRec), &sm.tile_full[b]);
+// The same at one point: (G, H).
+__device__ __forceinline__ void bm_point(float dx, float dy, float dz, float k, float2& g, float2& h) {
+  const float r2 = fmaxf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)), kEps * kEps);
+  const float ri = rsqrtf(r2), ri2 = ri * ri;
+  float s, c;
+  __sincosf(k * (r2 * ri), &s, &c);
+  g = make_float2(c * ri, s * ri);
+  h = make_float2(fmaf(k, s, g.x) * ri2, fmaf(-k, c, g.y) * ri2);
 }
 
-// S, T, U blocks of one unordered pair under the TN x TN point rule (test
-// triangle tl, points in xs; trial points yq, dq[q] = n_i . (c_i - y_q)).
-// Packed FP32 pairs (f32x2): complex sums as (re, im) pairs, distances for two
-// trial points at once; same operations and rounding as the scalar form.
 template <int TN>
-__device__ __forceinline__ void bm_pair_block(const float (*xs)[kBmTest], int tl, const float (&yq)[3 * TN],
-                                              const float (&dq)[TN], float njx, float njy, float njz, float cjx,
-                                              float cjy, float cjz, float k, float2 (&aS)[9], float2 (&aT)[9],
-                                              float2 (&aU)[9]) {
+using BmWarp = StripWarp<3 * TN + 9, true>;
+constexpr int kBmPanel = 2, kBmPanelItems = 8;  // strip_items
+
+// Strip walk of the Burton-Miller pair (strip.cuh): the open columns hold
+// lhs_ij, lhs_ji^T and rhs_ij; rhs_ji^T - rhs_ij = (i/k)(T - U) = (i/k)(lhs_ij
+// - lhs_ji^T) entry by entry, so it follows from the reduced sums.  Rows of xs:
+// the test points, then the test curls.
+//
+// Measured on B200 at the 3-point rule, the whole assembly: 8286 triangles 1.53
+// ms, 20 480 triangles 8.5 ms, against 2.20 and 12.7 ms for 16 x 16-triangle
+// tiles reduced in shared memory (at 9 point pairs per triangle pair the
+// reduction took over half of the time).  Issue slots and FP32 pipe 58 and 50 %
+// busy; the atomics' DRAM traffic (23 GB at 20 480 triangles with contiguous
+// items) is why the items go in panels (strip_items).
+template <int TN>
+struct BmStrip {
+  float k, kinv;
+  float2* L;
+  float2* R;
+  // the curl terms, which cancel over a vertex star, apart from the others
+  float2 aL[9], aT[9], aR[9], aC[9];
+
+  __device__ __forceinline__ void clear() {
 #pragma unroll
-  for (int e = 0; e < 9; e++) {
-    aS[e] = make_float2(0.f, 0.f);
-    aT[e] = make_float2(0.f, 0.f);
-    aU[e] = make_float2(0.f, 0.f);
+    for (int e = 0; e < 9; e++) aL[e] = aT[e] = aR[e] = aC[e] = make_float2(0.f, 0.f);
   }
-  const float2 kk = make_float2(k, -k);
+
+  __device__ __forceinline__ void load(BmWarp<TN>& sw, const StripTest& t, const GeomView& g, int lane) {
+    const int at = min(t.grp * kBlock + lane, g.nt - 1);
+    const TriRec& r = g.rec[at];
+    const BmRec& b = g.bm[at];
 #pragma unroll
-  for (int p = 0; p < TN; p++) {
-    const float px = xs[3 * p][tl], py = xs[3 * p + 1][tl], pz = xs[3 * p + 2][tl];
-    const float dn = njx * (cjx - px) + njy * (cjy - py) + njz * (cjz - pz);  // (y - x).n_j on plane j
-    float2 tS[3], tT[3], tU[3];
+    for (int e = 0; e < 3 * TN; e++) sw.xs[e][lane] = TN == 3 ? b.qp[e] : (TN == 6 ? r.qp[e] : r.c[e]);
 #pragma unroll
-    for (int b = 0; b < 3; b++) {
-      tS[b] = make_float2(0.f, 0.f);
-      tT[b] = make_float2(0.f, 0.f);
-      tU[b] = make_float2(0.f, 0.f);
-    }
+    for (int e = 0; e < 9; e++) sw.xs[3 * TN + e][lane] = b.curl[e];
+  }
+
+  __device__ __forceinline__ void pair(const BmWarp<TN>& sw, const StripTest& t, const TriRec& rj, const BmRec& bj,
+                                       float w, int lane) {
+    const float* yq = TN == 3 ? bj.qp : (TN == 6 ? rj.qp : rj.c);
+    const float njx = rj.n[0], njy = rj.n[1], njz = rj.n[2], cjx = rj.c[0], cjy = rj.c[1], cjz = rj.c[2];
+    const float sc = w * kInv4Pi;
+    const float knn = k * (t.nx * njx + t.ny * njy + t.nz * njz);
+    float dq[TN];  // n_i . (c_i - y_q)
 #pragma unroll
-    for (int q0 = 0; q0 < TN; q0 += 2) {
-      constexpr int kLast = TN - 1;
-      const int q1 = q0 + 1 < TN ? q0 + 1 : kLast;  // an odd rule repeats its last point in the idle lane
-      const float2 dx = f2_sub(make_float2(yq[3 * q0], yq[3 * q1]), f2(px));
-      const float2 dy = f2_sub(make_float2(yq[3 * q0 + 1], yq[3 * q1 + 1]), f2(py));
-      const float2 dz = f2_sub(make_float2(yq[3 * q0 + 2], yq[3 * q1 + 2]), f2(pz));
-      const float2 r2 = f2_fma(dx, dx, f2_fma(dy, dy, f2_mul(dz, dz)));
-      const float2 rinv = make_float2(fminf(rsqrtf(r2.x), 1.0f / kEps), fminf(rsqrtf(r2.y), 1.0f / kEps));
-      float2 r = f2_mul(r2, rinv);
-      r.x = fmaxf(r.x, kEps);
-      r.y = fmaxf(r.y, kEps);
-      const float2 kr = f2_mul(f2(k), r);
-      const float2 rinv2 = f2_mul(rinv, rinv);
-      float sc[2][2];  // [point][sin, cos]
-      __sincosf(kr.x, &sc[0][0], &sc[0][1]);
-      if (q0 + 1 < TN) __sincosf(kr.y, &sc[1][0], &sc[1][1]);
+    for (int q = 0; q < TN; q++)
+      dq[q] = t.nx * (t.cx - yq[3 * q]) + t.ny * (t.cy - yq[3 * q + 1]) + t.nz * (t.cz - yq[3 * q + 2]);
+    float2 total = make_float2(0.f, 0.f);  // weight sum of G over the pair
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        if (q0 + j < TN) {
-          const int q = q0 + j;
-          const float ri = j == 0 ? rinv.x : rinv.y, ri2 = j == 0 ? rinv2.x : rinv2.y;
-          const float2 g = f2_mul(make_float2(sc[j][1], sc[j][0]), f2(ri));                  // (c, s) / r
-          const float2 h = f2_mul(f2_fma(kk, make_float2(sc[j][0], sc[j][1]), g), f2(ri2));  // (c + kr s, s - kr c) / r^3
-          const float2 u = f2_mul(f2(dq[q]), h);
+    for (int p = 0; p < TN; p++) {
+      const float px = sw.xs[3 * p][lane], py = sw.xs[3 * p + 1][lane], pz = sw.xs[3 * p + 2][lane];
+      const float dn = njx * (cjx - px) + njy * (cjy - py) + njz * (cjz - pz);  // (y - x).n_j on plane j
+      // trial sums of G, H and dq H, by vertex
+      float2 tS[3], tH[3], tU[3];
+      if constexpr (TN == 1) {
+        float2 g, h;
+        bm_point(yq[0] - px, yq[1] - py, yq[2] - pz, k, g, h);
 #pragma unroll
-          for (int b = 0; b < 3; b++) {
-            const float2 w = f2(bm_c<TN>(q, b));
-            tS[b] = f2_fma(w, g, tS[b]);
-            tT[b] = f2_fma(w, h, tT[b]);
-            tU[b] = f2_fma(w, u, tU[b]);
-          }
+        for (int b = 0; b < 3; b++) {
+          tS[b] = f2_mul(f2(1.f / 3.f), g);
+          tH[b] = f2_mul(f2(1.f / 3.f), h);
+          tU[b] = f2_mul(f2(dq[0] / 3.f), h);
+        }
+      } else if constexpr (TN == 3) {
+        float2 gr, gi, hr, hi;
+        bm_point2(f2_sub(make_float2(yq[0], yq[3]), f2(px)), f2_sub(make_float2(yq[1], yq[4]), f2(py)),
+                f2_sub(make_float2(yq[2], yq[5]), f2(pz)), k, gr, gi, hr, hi);
+        tS[0] = make_float2(gr.x, gi.x);
+        tS[1] = make_float2(gr.y, gi.y);
+        tH[0] = make_float2(hr.x, hi.x);
+        tH[1] = make_float2(hr.y, hi.y);
+        bm_point(yq[6] - px, yq[7] - py, yq[8] - pz, k, tS[2], tH[2]);
+        float2 sS = f2_add(f2_add(tS[0], tS[1]), tS[2]), sH = f2_add(f2_add(tH[0], tH[1]), tH[2]), sU;
+#pragma unroll
+        for (int b = 0; b < 3; b++) tU[b] = f2_mul(f2(dq[b]), tH[b]);
+        sU = f2_add(f2_add(tU[0], tU[1]), tU[2]);
+        // w phi_b = 1/18 + 1/6 [b == q]
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          tS[b] = f2_fma(f2(1.f / 6.f), tS[b], f2_mul(f2(1.f / 18.f), sS));
+          tH[b] = f2_fma(f2(1.f / 6.f), tH[b], f2_mul(f2(1.f / 18.f), sH));
+          tU[b] = f2_fma(f2(1.f / 6.f), tU[b], f2_mul(f2(1.f / 18.f), sU));
+        }
+      } else {
+        constexpr float o0 = (float)tri6_w_own(0), o3 = (float)tri6_w_own(3), c0 = (float)tri6_w_common(0),
+                        c3 = (float)tri6_w_common(3);
+        float2 cS = make_float2(0.f, 0.f), cH = cS, cU = cS;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          float2 gr, gi, hr, hi;
+          const int i0 = 3 * b, i3 = 9 + 3 * b;
+          bm_point2(f2_sub(make_float2(yq[i0], yq[i3]), f2(px)), f2_sub(make_float2(yq[i0 + 1], yq[i3 + 1]), f2(py)),
+                  f2_sub(make_float2(yq[i0 + 2], yq[i3 + 2]), f2(pz)), k, gr, gi, hr, hi);
+          const float2 d = make_float2(dq[b], dq[b + 3]);
+          const float2 ur = f2_mul(d, hr), ui = f2_mul(d, hi);
+          tS[b] = make_float2(fmaf(o3, gr.y, o0 * gr.x), fmaf(o3, gi.y, o0 * gi.x));
+          tH[b] = make_float2(fmaf(o3, hr.y, o0 * hr.x), fmaf(o3, hi.y, o0 * hi.x));
+          tU[b] = make_float2(fmaf(o3, ur.y, o0 * ur.x), fmaf(o3, ui.y, o0 * ui.x));
+          cS.x += fmaf(c3, gr.y, c0 * gr.x);
+          cS.y += fmaf(c3, gi.y, c0 * gi.x);
+          cH.x += fmaf(c3, hr.y, c0 * hr.x);
+          cH.y += fmaf(c3, hi.y, c0 * hi.x);
+          cU.x += fmaf(c3, ur.y, c0 * ur.x);
+          cU.y += fmaf(c3, ui.y, c0 * ui.x);
+        }
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+          tS[b] = f2_add(tS[b], cS);
+          tH[b] = f2_add(tH[b], cH);
+          tU[b] = f2_add(tU[b], cU);
         }
       }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      const float wa = bm_c<TN>(p, a);
-      const float2 wa2 = f2(wa), wt2 = f2(wa * dn);
+      const float wp = (float)(TN == 1 ? 1.0 : (TN == 3 ? 1.0 / 3.0 : tri6_w(p)));
+      total = f2_fma(f2(wp), f2_add(f2_add(tS[0], tS[1]), tS[2]), total);
 #pragma unroll
       for (int b = 0; b < 3; b++) {
-        aS[3 * a + b] = f2_fma(wa2, tS[b], aS[3 * a + b]);
-        aT[3 * a + b] = f2_fma(wt2, tT[b], aT[3 * a + b]);
-        aU[3 * a + b] = f2_fma(wa2, tU[b], aU[3 * a + b]);
+        const float2 z = make_float2(knn * tS[b].y, -knn * tS[b].x);  // -ik (n_i.n_j) S
+        tH[b] = f2_fma(f2(dn), tH[b], z);
+        tS[b] = make_float2(fmaf(-kinv, tU[b].y, -tS[b].x), fmaf(kinv, tU[b].x, -tS[b].y));  // -S + (i/k) U
+        tU[b] = f2_add(tU[b], z);
       }
-    }
-  }
-}
-
-// One work item: test tile grp against trial tiles [jt_begin, jt_end), all
-// at or after grp.  `uses` counts the trial tiles this CTA has processed
-// (buffer = uses & 1, mbarrier parity = (uses >> 1) & 1).
-template <int TN>
-__device__ __forceinline__ void bm_item(BmSmem& sm, const GeomView& g, float k, float2* __restrict__ L,
-                                        float2* __restrict__ Rm, int grp, int jt_begin, int jt_end,
-                                        unsigned& uses) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tl = lane & 15;               // test triangle of this lane
-  const int tt = 2 * warp + (lane >> 4);  // trial triangle of this half-warp
-  const int nt = g.nt, nv = g.nv;
-  const int ti = grp * kBmTest + tl;
-  const bool valid_i = ti < nt;
-  const TriRec& ri = g.rec[valid_i ? ti : nt - 1];
-  const float area_i = ri.area;
-  const float nix = ri.n[0], niy = ri.n[1], niz = ri.n[2], cix = ri.c[0], ciy = ri.c[1], ciz = ri.c[2];
-  const int iv0 = ri.v[0], iv1 = ri.v[1], iv2 = ri.v[2];
-  const float kinv = 1.0f / k;
-
-  __syncthreads();  // the previous item is done with tileI, xs, xc and both trial buffers
-  if (tid == 0) bm_fetch_tile(sm, g, jt_begin, uses & 1);
-  bm_copy_words(&sm.tileI, &g.tiles[grp], sizeof(TileRec), tid);
-  for (int e = tid; e < (3 * TN + 9) * kBmTest; e += kBmThreads) {
-    const int c = e / kBmTest, l = e - c * kBmTest;
-    const int t = min(grp * kBmTest + l, nt - 1);
-    if (c < 3 * TN)
-      sm.xs[c][l] = bm_point<TN>(g.rec[t], g.bm[t], c);
-    else
-      sm.xc[c - 3 * TN][l] = g.bm[t].curl[c - 3 * TN];
-  }
-
-  for (int jt = jt_begin; jt < jt_end; jt++, uses++) {
-    const int bf = uses & 1;
-    __syncthreads();  // the previous tile's gather is done with the slots and with buffer bf ^ 1
-    if (tid == 0 && jt + 1 < jt_end) bm_fetch_tile(sm, g, jt + 1, bf ^ 1);
-    if (!mbar_wait(&sm.tile_full[bf], (uses >> 1) & 1u, g.err)) {
-      // expired (this geometry's status word raised): record it process-wide
-      // too, and let the copy land before the buffer is reused
-      if (threadIdx.x == 0) atomicExch(&g_bm_err, 1);
-      mbar_wait_drain(&sm.tile_full[bf], (uses >> 1) & 1u);
-    }
-    const TileRec& tileJ = sm.tileJ[bf];
-    const int ntriJ = min(kTile, nt - jt * kTile);
-
-    // ---- compute: half-warp h of warp w takes trial triangle 2w + h ----
-    const int tj = jt * kTile + tt;
-    float aa = 0.f;
-    if (tt < ntriJ) {
-      const TriRec& rj = sm.trial[bf][tt];
-      const int j0 = rj.v[0], j1 = rj.v[1], j2 = rj.v[2];
-      const bool touching = (iv0 == j0) | (iv0 == j1) | (iv0 == j2) | (iv1 == j0) | (iv1 == j1) | (iv1 == j2) |
-                            (iv2 == j0) | (iv2 == j1) | (iv2 == j2);
-      const bool once = jt > grp || tj > ti;  // on the test tile itself each unordered pair once
-      aa = (valid_i && !touching && once) ? area_i * rj.area : 0.f;
-    }
-    const bool any = __any_sync(0xffffffffu, aa != 0.f);  // every lane, before the half-warp branch
-    if (tt < ntriJ && any) {
-      const TriRec& rj = sm.trial[bf][tt];
-      const BmRec& bj = sm.trialB[bf][tt];
-      float yq[3 * TN];
 #pragma unroll
-      for (int e = 0; e < 3 * TN; e++) yq[e] = bm_point<TN>(rj, bj, e);
-      float dq[TN];
-#pragma unroll
-      for (int q = 0; q < TN; q++)
-        dq[q] = nix * (cix - yq[3 * q]) + niy * (ciy - yq[3 * q + 1]) + niz * (ciz - yq[3 * q + 2]);
-      float2 aS[9], aT[9], aU[9];
-      bm_pair_block<TN>(sm.xs, tl, yq, dq, rj.n[0], rj.n[1], rj.n[2], rj.c[0], rj.c[1], rj.c[2], k, aS, aT, aU);
-      const float sc = aa * kInv4Pi;
-      float2 s9 = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int e = 0; e < 9; e++) {
-        s9.x += aS[e].x;
-        s9.y += aS[e].y;
-      }
-      s9.x *= sc * kinv;  // (i/k) s = (-s.y / k, s.x / k), scaled
-      s9.y *= sc * kinv;
-      const float knn = k * (nix * rj.n[0] + niy * rj.n[1] + niz * rj.n[2]);
-#pragma unroll
-      for (int a = 0; a < 3; a++)
+      for (int a = 0; a < 3; a++) {
+        const float2 wa = f2(sc * bm_c<TN>(p, a));
 #pragma unroll
         for (int b = 0; b < 3; b++) {
-          const float cc = sm.xc[3 * a][tl] * bj.curl[3 * b] + sm.xc[3 * a + 1][tl] * bj.curl[3 * b + 1] +
-                           sm.xc[3 * a + 2][tl] * bj.curl[3 * b + 2];
-          const float Sx = aS[3 * a + b].x * sc, Sy = aS[3 * a + b].y * sc;
-          const float Tx = aT[3 * a + b].x * sc, Ty = aT[3 * a + b].y * sc;
-          const float Ux = aU[3 * a + b].x * sc, Uy = aU[3 * a + b].y * sc;
-          const float lx = fmaf(knn, Sy, -s9.y * cc), ly = fmaf(-knn, Sx, s9.x * cc);
-          sm.slotL[3 * tl + a][3 * tt + b] = make_float2(lx + Tx, ly + Ty);
-          sm.slotLT[3 * tl + a][3 * tt + b] = make_float2(lx + Ux, ly + Uy);
-          sm.slotR[3 * tl + a][3 * tt + b] = make_float2(fmaf(-Uy, kinv, -Sx), fmaf(Ux, kinv, -Sy));
+          aL[3 * a + b] = f2_fma(wa, tH[b], aL[3 * a + b]);
+          aT[3 * a + b] = f2_fma(wa, tU[b], aT[3 * a + b]);
+          aR[3 * a + b] = f2_fma(wa, tS[b], aR[3 * a + b]);
         }
-    } else if (tt < ntriJ) {
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-          sm.slotL[3 * tl + a][3 * tt + b] = make_float2(0.f, 0.f);
-          sm.slotLT[3 * tl + a][3 * tt + b] = make_float2(0.f, 0.f);
-          sm.slotR[3 * tl + a][3 * tt + b] = make_float2(0.f, 0.f);
-        }
-    }
-    __syncthreads();
-
-    // ---- reduce corner slots onto distinct vertices: (A, B) and (B, A) ----
-    // Pass 1, in place: for every trial corner column, the row of test
-    // vertex A's first corner gets the sum over A's test corners (corner rows
-    // of different vertices are disjoint); pass 2: entry (A, B) sums B's
-    // trial corners along that row.
-    const TileRec& TI = sm.tileI;
-    const int nI = TI.nlv, nJ = tileJ.nlv;
-    const int ncol = 3 * ntriJ;
-    const float rcol = 1.f / (float)ncol, rJ = 1.f / (float)(nJ > 0 ? nJ : 1);
-    for (int e = tid; e < nI * ncol; e += kBmThreads) {
-      const int a = div_by(e, ncol, rcol);
-      const int col = e - a * ncol;
-      const int ca0 = TI.lv_ptr[a], ca1 = TI.lv_ptr[a + 1];
-      const int rep = TI.lv_corner[ca0];
-      float2 l = sm.slotL[rep][col], lt = sm.slotLT[rep][col], rr = sm.slotR[rep][col];
-#pragma unroll 4
-      for (int ca = ca0 + 1; ca < ca1; ca++) {
-        const int row = TI.lv_corner[ca];
-        const float2 l1 = sm.slotL[row][col], lt1 = sm.slotLT[row][col], r1 = sm.slotR[row][col];
-        l.x += l1.x;
-        l.y += l1.y;
-        lt.x += lt1.x;
-        lt.y += lt1.y;
-        rr.x += r1.x;
-        rr.y += r1.y;
       }
-      sm.slotL[rep][col] = l;
-      sm.slotLT[rep][col] = lt;
-      sm.slotR[rep][col] = rr;
     }
-    __syncthreads();
-    for (int e = tid; e < nI * nJ; e += kBmThreads) {
-      const int a = div_by(e, nJ, rJ);
-      const int b = e - a * nJ;
-      const int rep = TI.lv_corner[TI.lv_ptr[a]];
-      const int cb0 = tileJ.lv_ptr[b], cb1 = tileJ.lv_ptr[b + 1];
-      float2 l = make_float2(0.f, 0.f), lt = l, rr = l;
-#pragma unroll 4
-      for (int cb = cb0; cb < cb1; cb++) {
-        const int col = tileJ.lv_corner[cb];
-        const float2 l1 = sm.slotL[rep][col], lt1 = sm.slotLT[rep][col], r1 = sm.slotR[rep][col];
-        l.x += l1.x;
-        l.y += l1.y;
-        lt.x += lt1.x;
-        lt.y += lt1.y;
-        rr.x += r1.x;
-        rr.y += r1.y;
-      }
-      const float2 rt = make_float2(fmaf(lt.y - l.y, kinv, rr.x), fmaf(l.x - lt.x, kinv, rr.y));
-      const int A = TI.vid[a], B = tileJ.vid[b];
-      if (l.x != 0.f || l.y != 0.f || lt.x != 0.f || lt.y != 0.f || rr.x != 0.f || rr.y != 0.f) {
-        atomicAdd(&L[(size_t)A * nv + B], l);
-        atomicAdd(&L[(size_t)B * nv + A], lt);
-        atomicAdd(&Rm[(size_t)A * nv + B], rr);
-        atomicAdd(&Rm[(size_t)B * nv + A], rt);
+    const float2 v = make_float2(-total.y * (sc * kinv), total.x * (sc * kinv));  // (i/k) times the sum
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const float cx = sw.xs[3 * TN + 3 * a][lane], cy = sw.xs[3 * TN + 3 * a + 1][lane],
+                  cz = sw.xs[3 * TN + 3 * a + 2][lane];
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const float2 cc = f2(cx * bj.curl[3 * b] + cy * bj.curl[3 * b + 1] + cz * bj.curl[3 * b + 2]);
+        aC[3 * a + b] = f2_fma(cc, v, aC[3 * a + b]);
       }
     }
   }
-}
 
-// Splits units [pos, end) of one problem at test-tile boundaries.
-template <int TN>
-__device__ __forceinline__ void bm_units(BmSmem& sm, const GeomView& g, float k, float2* L, float2* Rm,
-                                         long long pos, long long end, unsigned& uses) {
-  while (pos < end) {  // uniform over the block
-    const int grp = tile_group_of(pos, g.ntiles);
-    const long long base = tile_units_before(grp, g.ntiles);
-    const long long gend = base + (g.ntiles - grp);
-    const long long stop = end < gend ? end : gend;
-    const int jt0 = grp + (int)(pos - base);
-    bm_item<TN>(sm, g, k, L, Rm, grp, jt0, jt0 + (int)(stop - pos), uses);
-    pos = stop;
+  template <int B>
+  __device__ __forceinline__ void take(BmWarp<TN>& sw, int i, int lane) {
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const float2 l = f2_add(aL[3 * a + B], aC[3 * a + B]), lt = f2_add(aT[3 * a + B], aC[3 * a + B]);
+      sw.col4[i][32 * a + lane] = make_float4(l.x, l.y, lt.x, lt.y);
+      sw.col2[i][32 * a + lane] = aR[3 * a + B];
+      aL[3 * a + B] = aT[3 * a + B] = aR[3 * a + B] = aC[3 * a + B] = make_float2(0.f, 0.f);
+    }
   }
-}
+
+  __device__ __forceinline__ void store(const GeomView& g, int A, int B, const float4& s, const float2& r) const {
+    if (s.x == 0.f && s.y == 0.f && s.z == 0.f && s.w == 0.f && r.x == 0.f && r.y == 0.f) return;
+    const size_t ab = (size_t)A * g.nv + B, ba = (size_t)B * g.nv + A;
+    atomicAdd(&L[ab], make_float2(s.x, s.y));
+    atomicAdd(&L[ba], make_float2(s.z, s.w));
+    atomicAdd(&R[ab], r);
+    atomicAdd(&R[ba], make_float2(fmaf(s.w - s.y, kinv, r.x), fmaf(s.x - s.z, kinv, r.y)));
+  }
+};
 
 // ---- problem descriptors (one problem, or a batch) ----
 struct BmProblem {
   GeomView g;
   float k;
-  int chunk;                // units per work item
-  long long n_units;        // used (test group, trial tile) units
+  StripItems items;
   long long item_begin;     // prefix sum of work items
   long long pair_begin[3];  // prefix sums of coincident / edge / vertex pairs
   float2* L;
@@ -389,57 +279,51 @@ __device__ __forceinline__ int bm_find(const BmProblem* probs, int np, long long
   return lo;
 }
 
-__device__ __forceinline__ void bm_init_barriers(BmSmem& sm) {
-  if (threadIdx.x == 0) {
-    mbar_init(&sm.tile_full[0], 1);
-    mbar_init(&sm.tile_full[1], 1);
-    mbar_init_fence();
-  }
-}
-
-// CTAs per SM of the regular kernels: three at the 1- and 3-point rules
-// (80 registers, the slabs of three CTAs fit in shared memory: the barriers
-// and the on-chip reduction of one CTA overlap two others' evaluation), two at
-// the 6-point rule (whose accumulators would spill at 80 registers).
-__host__ __device__ constexpr int bm_min_ctas(int tn) { return tn == 6 ? 2 : 3; }
-
-// Regular pairs of one problem: equal work items dealt round-robin to a
-// persistent grid.
+// Regular pairs of one problem: equal work items dealt round-robin to the
+// warps of a persistent grid.
 template <int TN>
-__global__ void __launch_bounds__(kBmThreads, bm_min_ctas(TN))
-    regular_bm_kernel(const __grid_constant__ BmProblem P, int n_items) {
+__global__ void __launch_bounds__(kStripThreads, 2)
+    regular_bm_kernel(const __grid_constant__ BmProblem P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BmSmem& sm = *reinterpret_cast<BmSmem*>(smem_raw);
-  bm_init_barriers(sm);
+  BmWarp<TN>& sw = reinterpret_cast<BmWarp<TN>*>(smem_raw)[threadIdx.x >> 5];
+  strip_init(sw);
+  BmStrip<TN> pol;
+  pol.k = P.k;
+  pol.kinv = 1.0f / P.k;
+  pol.L = P.L;
+  pol.R = P.R;
+  pol.clear();
+  StripTest test;
   unsigned uses = 0;
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const long long pos = (long long)item * P.chunk;
-    const long long end = pos + P.chunk < P.n_units ? pos + P.chunk : P.n_units;
-    bm_units<TN>(sm, P.g, P.k, P.L, P.R, pos, end, uses);
-  }
+  const long long warps = (long long)gridDim.x * kStripWarps;
+  for (long long item = (long long)blockIdx.x * kStripWarps + (threadIdx.x >> 5); item < P.items.items; item += warps)
+    strip_item(sw, test, P.g, pol, P.items, item, uses, &g_bm_err);
 }
 
-// Regular pairs of a batch: CTAs drain one queue of work items.
 template <int TN>
-__global__ void __launch_bounds__(kBmThreads, bm_min_ctas(TN))
+__global__ void __launch_bounds__(kStripThreads, 2)
     regular_bm_batch_kernel(BmHeader* __restrict__ hdr, const BmProblem* __restrict__ probs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  BmSmem& sm = *reinterpret_cast<BmSmem*>(smem_raw);
-  __shared__ long long s_item;
-  bm_init_barriers(sm);
+  BmWarp<TN>& sw = reinterpret_cast<BmWarp<TN>*>(smem_raw)[threadIdx.x >> 5];
+  strip_init(sw);
   const int np = hdr->nproblems;
   const long long total = hdr->total_items;
+  BmStrip<TN> pol;
+  pol.clear();
+  StripTest test;
   unsigned uses = 0;
   for (;;) {
-    __syncthreads();  // everyone has read s_item of the previous round
-    if (threadIdx.x == 0) s_item = (long long)atomicAdd(&hdr->next_item, 1ull);
-    __syncthreads();
-    const long long item = s_item;
+    long long item = 0;
+    if ((threadIdx.x & 31) == 0) item = (long long)atomicAdd(&hdr->next_item, 1ull);
+    item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= total) break;
     const BmProblem& P = probs[bm_find(probs, np, item, -1)];
-    const long long pos = (item - P.item_begin) * P.chunk;
-    const long long end = pos + P.chunk < P.n_units ? pos + P.chunk : P.n_units;
-    bm_units<TN>(sm, P.g, P.k, P.L, P.R, pos, end, uses);
+    pol.k = P.k;
+    pol.kinv = 1.0f / P.k;
+    pol.L = P.L;
+    pol.R = P.R;
+    test.grp = -1;  // another problem's block may have the same number
+    strip_item(sw, test, P.g, pol, P.items, item - P.item_begin, uses, &g_bm_err);
   }
 }
 
@@ -680,20 +564,18 @@ int bm_check(float k, const float2* L, const float2* R) {
 }
 
 // Persistent grid of a regular kernel (shared-memory attribute set once).
-template <typename KernelT>
+template <int TN, typename KernelT>
 int bm_grid(KernelT kernel, std::atomic<bool>& attr, long long* grid) {
-  const int smem = (int)sizeof(BmSmem);
+  const int smem = (int)(kStripWarps * sizeof(BmWarp<TN>));
   if (!attr.load(std::memory_order_acquire)) {
     BEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr.store(true, std::memory_order_release);
   }
   int occ = 0;
-  BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kBmThreads, smem));
+  BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kStripThreads, smem));
   *grid = (long long)bm_sm_count() * (occ > 0 ? occ : 1);
   return BEM_OK;
 }
-
-long long bm_units_of(const GeomView& g) { return (long long)g.ntiles * (g.ntiles + 1) / 2; }
 
 }  // namespace
 
@@ -706,13 +588,13 @@ namespace {
 template <int TN>
 int bm_single_grid(long long* grid) {
   static std::atomic<bool> attr{false};
-  return bm_grid(regular_bm_kernel<TN>, attr, grid);
+  return bm_grid<TN>(regular_bm_kernel<TN>, attr, grid);
 }
 
 template <int TN>
 int bm_batch_grid(long long* grid) {
   static std::atomic<bool> attr{false};
-  return bm_grid(regular_bm_batch_kernel<TN>, attr, grid);
+  return bm_grid<TN>(regular_bm_batch_kernel<TN>, attr, grid);
 }
 
 int bm_rule(int order, int* tn) {
@@ -727,7 +609,8 @@ template <int TN, int LN>
 void bm_single_launch(const BmProblem& P, long long grid, long long items, cudaStream_t s) {
   const GeomView& g = P.g;
   if (items > 0)
-    (regular_bm_kernel<TN><<<(unsigned)(grid < items ? grid : items), kBmThreads, sizeof(BmSmem), s>>>(P, (int)items),
+    (regular_bm_kernel<TN><<<(unsigned)std::min(grid, (items + kStripWarps - 1) / kStripWarps), kStripThreads,
+                             kStripWarps * sizeof(BmWarp<TN>), s>>>(P),
      count_launch());
   const int wpb = 4, ppb = wpb * BmSingLanes<LN>::kPairsPerWarp;  // warps, pairs per block
   (singular_bm_kernel<double, 3, LN><<<(g.nt + ppb - 1) / ppb, 32 * wpb, 0, s>>>(P, g.nt), count_launch());
@@ -743,7 +626,8 @@ template <int TN, int LN>
 void bm_batch_launch(BmHeader* dh, BmProblem* dp, long long grid, long long items, const long long* pairs,
                      cudaStream_t s) {
   if (items > 0)
-    (regular_bm_batch_kernel<TN><<<(unsigned)(grid < items ? grid : items), kBmThreads, sizeof(BmSmem), s>>>(dh, dp),
+    (regular_bm_batch_kernel<TN><<<(unsigned)std::min(grid, (items + kStripWarps - 1) / kStripWarps), kStripThreads,
+                                   kStripWarps * sizeof(BmWarp<TN>), s>>>(dh, dp),
      count_launch());
   const int wpb = 4, ppb = wpb * BmSingLanes<LN>::kPairsPerWarp;  // warps, pairs per block
   if (pairs[0])
@@ -775,12 +659,10 @@ int assemble_bm(const GeomView& g, int order, float k, float2* L, float2* R, cud
   std::memset(&P, 0, sizeof(P));
   P.g = g;
   P.k = k;
-  P.n_units = bm_units_of(g);
-  const long long chunk = (P.n_units + 8 * grid - 1) / (8 * grid);  // 8 equal items per CTA
-  P.chunk = (int)(chunk < 1 ? 1 : chunk);
+  P.items = strip_items(g.nv, g.nblocks, grid * kStripWarps, 4, 0, kBmPanel, kBmPanelItems);
   P.L = L;
   P.R = R;
-  const long long items = (P.n_units + P.chunk - 1) / P.chunk;
+  const long long items = P.items.items;
   if (tn == 6)
     bm_single_launch<6, 4>(P, grid, items, s);
   else if (tn == 3)
@@ -821,11 +703,10 @@ int assemble_bm_batch(const GeomView* views, const float* ks, float2* const* Ls,
   std::memset(hh, 0, sizeof(BmHeader));
   std::memset(hp, 0, pbytes);
   hh->nproblems = np;
-  long long units_all = 0;
-  for (int p = 0; p < np; p++) units_all += bm_units_of(views[p]);
-  // about 8 items per CTA over the whole batch, at most 64 units per item
-  long long chunk = (units_all + 8 * grid - 1) / (8 * grid);
-  chunk = chunk < 1 ? 1 : (chunk > 64 ? 64 : chunk);
+  long long steps = 0;
+  for (int p = 0; p < np; p++) steps += strip_steps(views[p].nblocks);
+  // about 8 items per warp over the whole batch, at most 16 trial blocks each
+  const long long share = std::min<long long>(512, std::max<long long>(4, steps / (8 * grid * kStripWarps)));
   long long items = 0, pairs[3] = {0, 0, 0};
   for (int p = 0; p < np; p++) {
     const GeomView& g = views[p];
@@ -834,10 +715,9 @@ int assemble_bm_batch(const GeomView* views, const float* ks, float2* const* Ls,
     BmProblem& P = hp[p];
     P.g = g;
     P.k = ks[p];
-    P.n_units = bm_units_of(g);
-    P.chunk = (int)chunk;
+    P.items = strip_items(g.nv, g.nblocks, std::max(1LL, strip_steps(g.nblocks) / share), 4, 0, kBmPanel, kBmPanelItems);
     P.item_begin = items;
-    items += (P.n_units + P.chunk - 1) / P.chunk;
+    items += P.items.items;
     P.pair_begin[0] = pairs[0];
     P.pair_begin[1] = pairs[1];
     P.pair_begin[2] = pairs[2];

@@ -170,10 +170,11 @@ __device__ __forceinline__ void strip_reduce(StripWarp<ROWS, BM>& sw, const Stri
   __syncwarp();  // the columns may be overwritten
 }
 
-// Walks steps [pos, end) of one problem: step 32 u + t is trial triangle t of
-// unit u, the units being (test block, trial block at or after it) in order
-// (tile_units_before).  `uses` counts the trial blocks this warp has fetched
-// (buffer uses & 1, mbarrier parity (uses >> 1) & 1).  Pol provides
+// Walks `steps` steps of one problem from trial triangle t0 of trial block jb on,
+// for test block grp: a step is one trial triangle (blocks count 32, the last
+// one too), after the last trial block comes the next test block's own.
+// `uses` counts the trial blocks this warp has fetched (buffer uses & 1,
+// mbarrier parity (uses >> 1) & 1).  Pol provides
 //   load(sw, t, g, lane)                  the test block's rows of sw.xs,
 //   pair(sw, t, rec, bm record, weight)   adds the pair's blocks,
 //   take<B>(sw, i, lane)                  moves trial slot B's column into
@@ -181,21 +182,20 @@ __device__ __forceinline__ void strip_reduce(StripWarp<ROWS, BM>& sw, const Stri
 //   store(g, A, B, sum4, sum2)            adds the sums of vertices (A, B).
 template <int ROWS, bool BM, typename Pol>
 __device__ __forceinline__ void strip_walk(StripWarp<ROWS, BM>& sw, StripTest& test, const GeomView& g, Pol& pol,
-                                           long long pos, long long end, unsigned& uses, int* process_err) {
+                                           int grp, int jb, int t0, int steps, unsigned& uses,
+                                           int* process_err) {
   const int lane = threadIdx.x & 31;
-  if (pos >= end) return;
+  if (steps <= 0) return;
   const int nb = g.nblocks;
-  int grp = tile_group_of(pos >> 5, nb);
-  int jb = grp + (int)((pos >> 5) - tile_units_before(grp, nb));
   if (lane == 0) strip_fetch(sw, g, jb, uses & 1);
-  for (; pos < end; uses++) {
-    const int t0 = (int)(pos & 31), t1 = (int)(end - pos < 32 - t0 ? t0 + (end - pos) : 32);
+  for (; steps > 0; uses++) {
+    const int t1 = min(32, t0 + steps);
     const int bf = uses & 1;
-    pos += t1 - t0;
+    steps -= t1 - t0;
     int next_grp = grp, next_jb = jb + 1;
     if (next_jb == nb) next_jb = ++next_grp;
     __syncwarp();  // every lane is done with buffer bf ^ 1 and with xs
-    if (lane == 0 && pos < end) strip_fetch(sw, g, next_jb, bf ^ 1);
+    if (lane == 0 && steps > 0) strip_fetch(sw, g, next_jb, bf ^ 1);
     if (grp != test.grp) {
       strip_load_test(test, g, grp);
       pol.load(sw, test, g, lane);
@@ -243,10 +243,77 @@ __device__ __forceinline__ void strip_walk(StripWarp<ROWS, BM>& sw, StripTest& t
     }
     grp = next_grp;
     jb = next_jb;
+    t0 = 0;
   }
+}
+
+// Work items of one problem, in one of two orders.
+//   panel == 0: runs of `chunk` steps, the block pairs taken test block by test
+//     block.  Items as long as an equal share for every warp of the grid have
+//     the fewest column flushes, but the warps then work all over the matrices.
+//   panel > 0: an item is one test block against `panel` trial blocks, panel by
+//     panel: at any time the warps work on a few columns of block pairs (and,
+//     mirrored, rows), whose entries stay in L2 until their neighbours'
+//     contributions have arrived.
+struct StripItems {
+  long long items, steps;
+  int chunk, panel;
+};
+
+// Item `item` of P (all lanes).
+template <int ROWS, bool BM, typename Pol>
+__device__ __forceinline__ void strip_item(StripWarp<ROWS, BM>& sw, StripTest& test, const GeomView& g, Pol& pol,
+                                           const StripItems& P, long long item, unsigned& uses, int* process_err) {
+  const int nb = g.nblocks;
+  int grp, jb, t0 = 0, steps;
+  if (P.panel == 0) {
+    const long long pos = item * P.chunk, unit = pos >> 5;
+    grp = tile_group_of(unit, nb);
+    jb = grp + (int)(unit - tile_units_before(grp, nb));
+    t0 = (int)(pos & 31);
+    steps = (int)(P.steps - pos < P.chunk ? P.steps - pos : P.chunk);
+  } else {
+    // panel c holds test blocks 0 .. panel (c + 1) - 1 (or nb - 1)
+    const long long q = item / P.panel;
+    long long c = (long long)((sqrt(8.0 * (double)q + 1.0) - 1.0) * 0.5);
+    while (c > 0 && c * (c + 1) / 2 > q) c--;
+    while ((c + 1) * (c + 2) / 2 <= q) c++;
+    grp = (int)(item - P.panel * (c * (c + 1) / 2));
+    const int first = (int)c * P.panel;
+    jb = first > grp ? first : grp;
+    steps = 32 * ((first + P.panel < nb ? first + P.panel : nb) - jb);
+  }
+  strip_walk(sw, test, g, pol, grp, jb, t0, steps, uses, process_err);  // one copy (instruction cache)
 }
 
 // Steps of a problem's walk.
 inline long long strip_steps(int nblocks) { return 32LL * nblocks * (nblocks + 1) / 2; }
+
+// The items for a grid of `warps` warps, at least `least` steps each; `blocks`
+// trial blocks per item if that is not 0 (tuning).  Panels of `panel` blocks
+// are taken where the two matrices exceed the L2 cache by far (64 MB) and every
+// warp gets `panel_items` of them, so that the uneven last round is small.
+// Measured on B200, contiguous items against panels: Burton-Miller at the
+// 3-point rule (a pair takes a third of the V/K pair's time, so that its
+// atomics weigh more), panels of 2, 20 480 triangles 11.8 and 8.5 ms, 8286
+// triangles 1.75 and 1.53 ms, 5120 triangles 0.66 and 0.68 ms; V and K, panels
+// of 8, 81 920 triangles 225 and 220 ms, 20 480 triangles 14.57 and 14.87 ms
+// (loading a test block per item, uneven last round).
+inline StripItems strip_items(int nv, int nblocks, long long warps, long long least, int blocks, int panel,
+                              int panel_items) {
+  StripItems P;
+  P.steps = strip_steps(nblocks);
+  const long long share = (P.steps + warps - 1) / warps;
+  P.panel = blocks == 0 && 16.0 * nv * nv > 64e6 && share >= 32LL * panel * panel_items ? panel : 0;
+  const long long chunk = blocks > 0 ? 32LL * blocks : (share > least ? share : least);
+  P.chunk = (int)(chunk < (1 << 30) ? chunk : (1 << 30));
+  if (P.panel) {
+    const long long panels = (nblocks + P.panel - 1) / P.panel;
+    P.items = P.panel * (panels * (panels - 1) / 2) + nblocks;
+  } else {
+    P.items = (P.steps + P.chunk - 1) / P.chunk;
+  }
+  return P;
+}
 
 }  // namespace bemb
