@@ -36,6 +36,7 @@
 
 #include "async_copy.cuh"
 #include "bem_common.cuh"
+#include "sauter_schwab.cuh"
 #include "strip.cuh"
 
 namespace bemb {
@@ -460,6 +461,7 @@ __global__ void __launch_bounds__(kStripThreads, 2)
                             float k_scale, StripItems P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   VkWarp& sw = reinterpret_cast<VkWarp*>(smem_raw)[threadIdx.x >> 5];
+  launch_next();
   strip_init(sw);
   VkStrip pol;
   pol.k = k;
@@ -476,297 +478,249 @@ __global__ void __launch_bounds__(kStripThreads, 2)
 }
 
 // ---------------------------------------------------------------------------
-// Singular (touching) pairs: Sauter-Schwab quadrature on the reference
-// triangle (0,0),(1,0),(1,1) (integrand.h:54-185), after re-ordering so the
-// shared vertices come first (integrand.h:351-387).  One warp per pair; the
-// lanes split the 4^4 Gauss-Legendre points; blocks are reduced with
-// shuffles and added with one atomic per entry.
+// Touching pairs: Sauter-Schwab quadrature (sauter_schwab.cuh) on the reference
+// triangle (0,0),(1,0),(1,1) (integrand.h:54-185), shared vertices first
+// (integrand.h:351-387).  A warp per pair, the lanes split the 4^4
+// Gauss-Legendre points; the sums are transposed over the lanes and added with
+// one atomic per entry.  Both triangles start at a shared vertex, so the
+// difference is d = y1 F1 + y2 F2 - x1 E1 - x2 E2 in their edges E1 = a1 - a0,
+// E2 = a2 - a1 (F of the trial triangle), without the vertices' own size.
+//
+// What the symmetries save:
+//   * coincident pairs (FP64): the six regions are three and their mirrors, so
+//     V = T + T^T from three, with |d|^2 from the triangle's metric; (y - x).n
+//     vanishes, so K gets the mass term only;
+//   * pairs with one common vertex (FP32): the two regions are mirrors, so one
+//     sweep of the unordered pair gives V_ij, V_ji = V_ij^T, K_ij and K_ji;
+//   * pairs with a common edge (FP32) have no such symmetry: ordered pairs.
+// All pairs go into one launch, so that the types fill the chip together.  It
+// may start while the regular pairs' kernel still runs (programmatic launch;
+// both only add to the matrices): beside it on small meshes, in the gaps of its
+// last round on large ones.  Measured on B200, the three types together: 20 480
+// triangles 705 us (coincident 389, edge 329 and vertex pairs 515 us before),
+// 320 triangles 18 us (19 + 12 + 12, one after the other, before).  More than
+// one warp per coincident pair of a small mesh gains nothing.
 // ---------------------------------------------------------------------------
+constexpr int kTouchThreads = 128;
+constexpr int kTouchWarps = kTouchThreads / 32;
 
+struct TouchShared {
+  double c[kTouchWarps][32];
+  float f[kTouchWarps][64];
+};
+
+// Gauss-Legendre point pt of the 4^4 rule on [0,1]^4 and its weight.
 template <typename R>
-struct R3 {
-  R x, y, z;
-};
-
-// Re-ordering of the reference (integrand.h:351-387): for a common edge the
-// shared vertices take local slots 0,1 in trial order; for a common vertex it
-// is swapped into slot 0 on both triangles.  Kept in scalar registers (no
-// runtime-indexed local arrays): p.i[c] / p.j[c] is the original local index
-// of re-ordered slot c.
-struct Perm {
-  int i0, i1, i2, j0, j1, j2;
-};
-
-__device__ __forceinline__ int pick3(int a0, int a1, int a2, int idx) { return idx == 0 ? a0 : (idx == 1 ? a1 : a2); }
-
-template <int NCOMMON>
-__device__ __forceinline__ Perm reorder_pair(int s0, int s1, int s2, int t0, int t1, int t2) {
-  Perm p{0, 1, 2, 0, 1, 2};
-  const int si[3] = {s0, s1, s2}, sj[3] = {t0, t1, t2};
-  if (NCOMMON == 2) {
-    int mi0 = 0, mj0 = 0, mi1 = 1, mj1 = 1, cnt = 0;
-#pragma unroll
-    for (int jj = 0; jj < 3; jj++)
-#pragma unroll
-      for (int ii = 0; ii < 3; ii++) {
-        const bool eq = si[ii] == sj[jj];
-        if (eq && cnt == 0) { mi0 = ii; mj0 = jj; }
-        if (eq && cnt == 1) { mi1 = ii; mj1 = jj; }
-        cnt += eq ? 1 : 0;
-      }
-    p = Perm{mi0, mi1, 3 - mi0 - mi1, mj0, mj1, 3 - mj0 - mj1};
-  } else if (NCOMMON == 1) {
-    int ci = 0, cj = 0;
-#pragma unroll
-    for (int ii = 0; ii < 3; ii++)
-#pragma unroll
-      for (int jj = 0; jj < 3; jj++)
-        if (si[ii] == sj[jj]) { ci = ii; cj = jj; }
-    p = Perm{ci, ci == 1 ? 0 : 1, ci == 2 ? 0 : 2, cj, cj == 1 ? 0 : 1, cj == 2 ? 0 : 2};
-  }
-  return p;
+__device__ __forceinline__ void touch_point(int pt, R& xi, R& e1, R& e2, R& e3, R& w) {
+  const int i0 = pt >> 6, i1 = (pt >> 4) & 3, i2 = (pt >> 2) & 3, i3 = pt & 3;
+  xi = R(0.5) * (R(gl4_x(i0)) + R(1));
+  e1 = R(0.5) * (R(gl4_x(i1)) + R(1));
+  e2 = R(0.5) * (R(gl4_x(i2)) + R(1));
+  e3 = R(0.5) * (R(gl4_x(i3)) + R(1));
+  w = R(gl4_w(i0)) * R(gl4_w(i1)) * R(gl4_w(i2)) * R(gl4_w(i3));
 }
 
-template <typename R, int NCOMMON, bool DO_V, bool DO_K>
-struct SingularAcc {
-  R v[18];  // 9 complex, (re, im) pairs, index 3 * test + trial (re-ordered)
-  R kk[18];
-  R3<R> a[3];  // re-ordered test vertices
-  R3<R> b[3];  // re-ordered trial vertices
-  R3<R> nj;    // unit normal of the trial triangle
-  R k;
-
-  // One Sauter-Schwab region: point (x1, x2) on the test triangle and (y1, y2)
-  // on the trial triangle, shape functions (1 - s, s - t, t), weight ww.
-  __device__ __forceinline__ void region(R x1, R x2, R y1, R y2, R ww) {
-    const R lx0 = R(1) - x1, lx1 = x1 - x2, lx2 = x2;
-    const R ly0 = R(1) - y1, ly1 = y1 - y2, ly2 = y2;
-    const R xx = lx0 * a[0].x + lx1 * a[1].x + lx2 * a[2].x;
-    const R xy = lx0 * a[0].y + lx1 * a[1].y + lx2 * a[2].y;
-    const R xz = lx0 * a[0].z + lx1 * a[1].z + lx2 * a[2].z;
-    const R yx = ly0 * b[0].x + ly1 * b[1].x + ly2 * b[2].x;
-    const R yy = ly0 * b[0].y + ly1 * b[1].y + ly2 * b[2].y;
-    const R yz = ly0 * b[0].z + ly1 * b[1].z + ly2 * b[2].z;
-    const R dx = yx - xx, dy = yy - xy, dz = yz - xz;
-    R r, inv_r;
-    inv_dist<R>(dx * dx + dy * dy + dz * dz, &r, &inv_r);
-    R s, c;
-    const R kr = k * r;
-    sincos_t<R>(kr, &s, &c);
-    const R gvr = c * inv_r * ww, gvi = s * inv_r * ww;
-    R gkr = 0, gki = 0;
-    if (DO_K) {
-      const R dn = dx * nj.x + dy * nj.y + dz * nj.z;  // (y - x) . n_trial
-      const R f = dn * inv_r * inv_r * inv_r * ww;
-      gkr = (c + kr * s) * f;
-      gki = (s - kr * c) * f;
+// Coincident pair (ti, ti).
+template <bool DO_V, bool DO_K>
+__device__ __forceinline__ void touch_coincident(const GeomView& g, int ti, float k, float2* __restrict__ V,
+                                                 float2* __restrict__ K, float v_scale,
+                                                 float mass_coeff, double* total) {
+  const int lane = threadIdx.x & 31;
+  const int v[3] = {g.triangles[3 * ti], g.triangles[3 * ti + 1], g.triangles[3 * ti + 2]};
+  double E1[3], E2[3], cr[3];
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    const double a1 = (double)g.vertices[3 * v[1] + e];
+    E1[e] = a1 - (double)g.vertices[3 * v[0] + e];
+    E2[e] = (double)g.vertices[3 * v[2] + e] - a1;
+  }
+  cr[0] = E1[1] * E2[2] - E1[2] * E2[1];
+  cr[1] = E1[2] * E2[0] - E1[0] * E2[2];
+  cr[2] = E1[0] * E2[1] - E1[1] * E2[0];
+  const double J2 = cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2];  // (2 area)^2
+  const size_t nv = (size_t)g.nv;
+  if (DO_V) {
+    const double g11 = E1[0] * E1[0] + E1[1] * E1[1] + E1[2] * E1[2], g22 = E2[0] * E2[0] + E2[1] * E2[1] + E2[2] * E2[2],
+                 g12 = 2.0 * (E1[0] * E2[0] + E1[1] * E2[1] + E1[2] * E2[2]);
+    const double jw = J2 / 16.0, kk = (double)k;
+    double t[12];  // entries (0,0) (0,1) (0,2) (1,1) (1,2) (2,2), (re, im)
+#pragma unroll
+    for (int e = 0; e < 12; e++) t[e] = 0.0;
+    auto region = [&](double x1, double x2, double y1, double y2, double w) {
+      const double u = y1 - x1, s = y2 - x2;
+      const double r2 = fmax(u * (u * g11 + s * g12) + s * s * g22, (double)kEps * (double)kEps);
+      const double ri = rsqrt(r2);
+      double sn, cs;
+      sincos_touch(kk * (r2 * ri), &sn, &cs);
+      const double gr = cs * ri * w, gi = sn * ri * w;
+      const double lx[3] = {1.0 - x1, x1 - x2, x2}, ly[3] = {1.0 - y1, y1 - y2, y2};
+      int e = 0;
+#pragma unroll
+      for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = a; b < 3; b++, e++) {
+          const double f = lx[a] * ly[b] + ly[a] * lx[b];
+          t[2 * e] += f * gr;
+          t[2 * e + 1] += f * gi;
+        }
+    };
+#pragma unroll 1
+    for (int pt = lane; pt < 256; pt += 32) {
+      double xi, e1, e2, e3, w;
+      touch_point<double>(pt, xi, e1, e2, e3, w);
+      const double e12 = e1 * e2, e123 = e12 * e3, sc = xi * xi * xi * e1 * e1 * e2 * w * jw;
+      region(xi, xi * (1.0 - e1 + e12), xi * (1.0 - e123), xi * (1.0 - e1), sc);
+      region(xi, xi * (e1 - e12 + e123), xi * (1.0 - e12), xi * (e1 - e12), sc);
+      region(xi * (1.0 - e123), xi * (e1 - e123), xi, xi * (e1 - e12), sc);
     }
-    const R lx[3] = {lx0, lx1, lx2}, ly[3] = {ly0, ly1, ly2};
-    if constexpr (std::is_same<R, float>::value) {
-      // packed FP32: (re, im) pairs, the trial weight applied first (3 + 3
-      // multiplies, then one packed FMA per entry and kernel)
-      float2 gy[3], ky[3];
-#pragma unroll
-      for (int jj = 0; jj < 3; jj++) {
-        gy[jj] = f2_mul(f2(ly[jj]), make_float2(gvr, gvi));
-        ky[jj] = f2_mul(f2(ly[jj]), make_float2(gkr, gki));
-      }
-#pragma unroll
-      for (int ii = 0; ii < 3; ii++)
-#pragma unroll
-        for (int jj = 0; jj < 3; jj++) {
-          const int e = 3 * ii + jj;
-          if (DO_V) {
-            const float2 t = f2_fma(f2(lx[ii]), gy[jj], make_float2(v[2 * e], v[2 * e + 1]));
-            v[2 * e] = t.x;
-            v[2 * e + 1] = t.y;
-          }
-          if (DO_K) {
-            const float2 t = f2_fma(f2(lx[ii]), ky[jj], make_float2(kk[2 * e], kk[2 * e + 1]));
-            kk[2 * e] = t.x;
-            kk[2 * e + 1] = t.y;
-          }
-        }
-    } else {
-#pragma unroll
-      for (int ii = 0; ii < 3; ii++)
-#pragma unroll
-        for (int jj = 0; jj < 3; jj++) {
-          const R f = lx[ii] * ly[jj];
-          if (DO_V) {
-            v[2 * (3 * ii + jj)] += gvr * f;
-            v[2 * (3 * ii + jj) + 1] += gvi * f;
-          }
-          if (DO_K) {
-            kk[2 * (3 * ii + jj)] += gkr * f;
-            kk[2 * (3 * ii + jj) + 1] += gki * f;
-          }
-        }
+    warp_totals<12>(t, total);
+    if (lane < 9) {
+      const int a = lane / 3, b = lane % 3, lo = min(a, b), hi = max(a, b);
+      const int e = lo == 0 ? hi : (lo == 1 ? 2 + hi : 5);
+      atomicAdd(&V[v[a] * nv + v[b]], make_float2((float)(total[2 * e] * (double)v_scale),
+                                                  (float)(total[2 * e + 1] * (double)v_scale)));
     }
   }
-
-  // One 4D Gauss point (xi, e1, e2, e3 on [0,1]) of weight w0; the region
-  // Jacobian w (integrand.h:121,134,146) is applied to every region.
-  __device__ __forceinline__ void point(R xi, R e1, R e2, R e3, R w0) {
-    const R e12 = e1 * e2, e123 = e1 * e2 * e3;
-    if (NCOMMON == 3) {
-      const R sc = xi * xi * xi * e1 * e1 * e2 * w0;
-      region(xi, xi * (R(1) - e1 + e12), xi * (R(1) - e123), xi * (R(1) - e1), sc);
-      region(xi * (R(1) - e123), xi * (R(1) - e1), xi, xi * (R(1) - e1 + e12), sc);
-      region(xi, xi * (e1 - e12 + e123), xi * (R(1) - e12), xi * (e1 - e12), sc);
-      region(xi * (R(1) - e12), xi * (e1 - e12), xi, xi * (e1 - e12 + e123), sc);
-      region(xi * (R(1) - e123), xi * (e1 - e123), xi, xi * (e1 - e12), sc);
-      region(xi, xi * (e1 - e12), xi * (R(1) - e123), xi * (e1 - e123), sc);
-    } else if (NCOMMON == 2) {
-      const R sc = xi * xi * xi * e1 * e1 * w0;
-      region(xi, xi * e1 * e3, xi * (R(1) - e12), xi * e1 * (R(1) - e2), sc);
-      region(xi, xi * e1, xi * (R(1) - e123), xi * e1 * e2 * (R(1) - e3), e2 * sc);
-      region(xi * (R(1) - e12), xi * e1 * (R(1) - e2), xi, xi * e123, e2 * sc);
-      region(xi * (R(1) - e123), xi * e12 * (R(1) - e3), xi, xi * e1, e2 * sc);
-      region(xi * (R(1) - e123), xi * e1 * (R(1) - e2 * e3), xi, xi * e12, e2 * sc);
-    } else {
-      const R sc = xi * xi * xi * e2 * w0;
-      region(xi, xi * e1, xi * e2, xi * e2 * e3, sc);
-      region(xi * e2, xi * e2 * e3, xi, xi * e1, sc);
-    }
-  }
-};
-
-template <typename R>
-__device__ __forceinline__ R warp_sum(R x) {
+  if (DO_K && mass_coeff != 0.f && lane < 9) {
+    // P1 mass block (integrand.h:257-278): area * sum_q w_q phi_a phi_b
+    const int a = lane / 3, b = lane % 3;
+    double m = 0.0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+    for (int q = 0; q < 6; q++) m += tri6_w(q) * tri6_phi(q, a) * tri6_phi(q, b);
+    atomicAdd(&K[v[a] * nv + v[b]], make_float2((float)(mass_coeff * 0.5 * sqrt(J2) * m), 0.f));
+  }
 }
 
-// NCOMMON = 3: pairs (i, i), i = pair index; otherwise pairs from the list.
-template <typename R, int NCOMMON, bool DO_V, bool DO_K>
-__device__ __forceinline__ void singular_pair(const GeomView& g, int ti, int tj, float k, float2* __restrict__ V,
-                                              float2* __restrict__ K, float v_scale, float k_scale,
-                                              float mass_coeff) {
+// Pair (ti, tj) with a common edge (NCOMMON = 2), or the unordered pair with one
+// common vertex (NCOMMON = 1), which also gives V_ji and K_ji.
+template <int NCOMMON, bool DO_V, bool DO_K>
+__device__ __forceinline__ void touch_pair(const GeomView& g, int ti, int tj, float k, float2* __restrict__ V,
+                                           float2* __restrict__ K, float v_scale, float k_scale, float* total) {
   const int lane = threadIdx.x & 31;
   const int s0 = g.triangles[3 * ti], s1 = g.triangles[3 * ti + 1], s2 = g.triangles[3 * ti + 2];
   const int t0 = g.triangles[3 * tj], t1 = g.triangles[3 * tj + 1], t2 = g.triangles[3 * tj + 2];
-  const Perm pm = reorder_pair<NCOMMON>(s0, s1, s2, t0, t1, t2);
-  const int pi_[3] = {pm.i0, pm.i1, pm.i2}, pj_[3] = {pm.j0, pm.j1, pm.j2};
-  R3<R> pa[3], pb[3];
+  const Perm6 pm = reorder6<NCOMMON>(s0, s1, s2, t0, t1, t2);
+  const int vi[3] = {sel3(s0, s1, s2, pm.i0), sel3(s0, s1, s2, pm.i1), sel3(s0, s1, s2, pm.i2)};
+  const int vj[3] = {sel3(t0, t1, t2, pm.j0), sel3(t0, t1, t2, pm.j1), sel3(t0, t1, t2, pm.j2)};
+  float E1[3], E2[3], F1[3], F2[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    const int va = pick3(s0, s1, s2, pi_[c]), vb = pick3(t0, t1, t2, pj_[c]);
-    pa[c] = {(R)g.vertices[3 * va], (R)g.vertices[3 * va + 1], (R)g.vertices[3 * va + 2]};
-    pb[c] = {(R)g.vertices[3 * vb], (R)g.vertices[3 * vb + 1], (R)g.vertices[3 * vb + 2]};
+  for (int e = 0; e < 3; e++) {
+    const float a1 = g.vertices[3 * vi[1] + e], b1 = g.vertices[3 * vj[1] + e];
+    E1[e] = a1 - g.vertices[3 * vi[0] + e];
+    E2[e] = g.vertices[3 * vi[2] + e] - a1;
+    F1[e] = b1 - g.vertices[3 * vj[0] + e];
+    F2[e] = g.vertices[3 * vj[2] + e] - b1;
   }
-  const int si[3] = {s0, s1, s2}, sj[3] = {t0, t1, t2};
-  // Jacobians and the trial normal of the un-permuted triangles
-  auto jac_normal = [](const R3<R>* p, R3<R>* n) {
-    const R e1x = p[1].x - p[0].x, e1y = p[1].y - p[0].y, e1z = p[1].z - p[0].z;
-    const R e2x = p[2].x - p[0].x, e2y = p[2].y - p[0].y, e2z = p[2].z - p[0].z;
-    const R cx = e1y * e2z - e1z * e2y, cy = e1z * e2x - e1x * e2z, cz = e1x * e2y - e1y * e2x;
-    const R J = sqrt(cx * cx + cy * cy + cz * cz);
-    if (n) *n = {cx / J, cy / J, cz / J};
-    return J;
+  float ni[3], nj[3];  // unit normals
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    ni[e] = g.normals[3 * ti + e];
+    nj[e] = g.normals[3 * tj + e];
+  }
+  auto twice_area = [](const float (&a)[3], const float (&b)[3]) {
+    const float x = a[1] * b[2] - a[2] * b[1], y = a[2] * b[0] - a[0] * b[2], z = a[0] * b[1] - a[1] * b[0];
+    return sqrtf(x * x + y * y + z * z);
   };
-  R3<R> oa[3], ob[3];
+  const float jw = twice_area(E1, E2) * twice_area(F1, F2) / 16.f;
+  // V_ij (9), K_ij (9) and, for a common vertex, K_ji^T (9), (re, im), by re-ordered slot 3 a + b
+  constexpr bool kMirror = NCOMMON == 1;
+  constexpr int oK = DO_V ? 9 : 0, oM = oK + (DO_K ? 9 : 0), kEntries = oM + (DO_K && kMirror ? 9 : 0);
+  float2 acc[kEntries];
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    oa[c] = {(R)g.vertices[3 * si[c]], (R)g.vertices[3 * si[c] + 1], (R)g.vertices[3 * si[c] + 2]};
-    ob[c] = {(R)g.vertices[3 * sj[c]], (R)g.vertices[3 * sj[c] + 1], (R)g.vertices[3 * sj[c] + 2]};
-  }
-  R3<R> nj;
-  const R Ji = jac_normal(oa, nullptr);
-  const R Jj = jac_normal(ob, &nj);
-
-  SingularAcc<R, NCOMMON, DO_V, DO_K> acc;
+  for (int e = 0; e < kEntries; e++) acc[e] = make_float2(0.f, 0.f);
+  auto region = [&](float x1, float x2, float y1, float y2, float w) {
+    float d[3];
 #pragma unroll
-  for (int e = 0; e < 18; e++) {
-    acc.v[e] = 0;
-    acc.kk[e] = 0;
-  }
+    for (int e = 0; e < 3; e++)
+      d[e] = NCOMMON == 2 ? (y1 - x1) * E1[e] + y2 * F2[e] - x2 * E2[e]  // F1 = E1, the shared edge
+                          : y1 * F1[e] + y2 * F2[e] - x1 * E1[e] - x2 * E2[e];
+    const float r2 = fmaxf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2], kEps * kEps);
+    const float ri = rsqrtf(r2), kr = k * (r2 * ri);
+    float s, c;
+    __sincosf(kr, &s, &c);
+    const float riw = ri * w;
+    const float lx[3] = {1.f - x1, x1 - x2, x2}, ly[3] = {1.f - y1, y1 - y2, y2};
+    if (DO_V) {
+      const float2 gv = make_float2(c * riw, s * riw);
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    acc.a[c] = pa[c];
-    acc.b[c] = pb[c];
-  }
-  acc.nj = nj;
-  acc.k = (R)k;
-  const R jw = Ji * Jj / R(16);
+      for (int b = 0; b < 3; b++) {
+        const float2 gy = f2_mul(f2(ly[b]), gv);
+#pragma unroll
+        for (int a = 0; a < 3; a++) acc[3 * a + b] = f2_fma(f2(lx[a]), gy, acc[3 * a + b]);
+      }
+    }
+    if (DO_K) {
+      const float dj = d[0] * nj[0] + d[1] * nj[1] + d[2] * nj[2];     // (y - x) . n_j
+      const float di = -(d[0] * ni[0] + d[1] * ni[1] + d[2] * ni[2]);  // (x - y) . n_i
+      const float f = ri * ri * riw;
+      const float2 h = make_float2(fmaf(kr, s, c) * f, fmaf(-kr, c, s) * f);
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const float2 hy = f2_mul(f2(ly[b]), h);
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+          acc[oK + 3 * a + b] = f2_fma(f2(lx[a] * dj), hy, acc[oK + 3 * a + b]);
+          if (kMirror) acc[oM + 3 * a + b] = f2_fma(f2(lx[a] * di), hy, acc[oM + 3 * a + b]);
+        }
+      }
+    }
+  };
 #pragma unroll 1
   for (int pt = lane; pt < 256; pt += 32) {
-    const int i0 = pt >> 6, i1 = (pt >> 4) & 3, i2 = (pt >> 2) & 3, i3 = pt & 3;
-    const R xi = R(0.5) * (R(gl4_x(i0)) + R(1));
-    const R e1 = R(0.5) * (R(gl4_x(i1)) + R(1));
-    const R e2 = R(0.5) * (R(gl4_x(i2)) + R(1));
-    const R e3 = R(0.5) * (R(gl4_x(i3)) + R(1));
-    const R w0 = R(gl4_w(i0)) * R(gl4_w(i1)) * R(gl4_w(i2)) * R(gl4_w(i3)) * jw;
-    acc.point(xi, e1, e2, e3, w0);
+    float xi, e1, e2, e3, w;
+    touch_point<float>(pt, xi, e1, e2, e3, w);
+    ss_regions<NCOMMON, float>(xi, e1, e2, e3, w * jw, region);
   }
-  // reduce: values 0..31 by a transpose-reduce (lane L ends with the warp
-  // total of value L), values 32..35 by plain sums; then lane e (< 9) takes
-  // V entry e, lane 9 + e K entry e
-  constexpr int NV = (DO_V ? 18 : 0) + (DO_K ? 18 : 0);
-  R t[32];
+  float t[2 * kEntries];
 #pragma unroll
-  for (int i = 0; i < 32; i++) {
-    const int vi = i, ki = DO_V ? i - 18 : i;
-    t[i] = (DO_V && vi < 18) ? acc.v[vi] : ((DO_K && ki >= 0 && ki < 18) ? acc.kk[ki] : R(0));
+  for (int e = 0; e < kEntries; e++) {
+    t[2 * e] = acc[e].x;
+    t[2 * e + 1] = acc[e].y;
   }
-  R extra[4] = {R(0), R(0), R(0), R(0)};
-  if (NV > 32) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) extra[i] = warp_sum(acc.kk[14 + i]);
-  }
-#pragma unroll
-  for (int o = 16, half = 16; o >= 1; o >>= 1, half >>= 1) {
-    const bool hi = (lane & o) != 0;
-#pragma unroll
-    for (int i = 0; i < half; i++) {
-      const R send = hi ? t[i] : t[i + half];
-      const R keep = hi ? t[i + half] : t[i];
-      t[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+  warp_totals<2 * kEntries>(t, total);
+  if (lane < kEntries) {
+    const int e = lane % 9, A = vi[e / 3], B = vj[e % 3];
+    const bool isV = DO_V && lane < 9;
+    const float sc = isV ? v_scale : k_scale;
+    const float2 x = make_float2(total[2 * lane] * sc, total[2 * lane + 1] * sc);
+    const size_t ab = (size_t)A * g.nv + B, ba = (size_t)B * g.nv + A;
+    if (isV) {
+      atomicAdd(&V[ab], x);
+      if (kMirror) atomicAdd(&V[ba], x);
+    } else {
+      atomicAdd(&K[lane >= oM ? ba : ab], x);
     }
-  }
-  const R mine = t[0];  // warp total of value `lane`
-  // value indices of this lane's entry (re, im)
-  const int e = lane < 9 ? lane : lane - 9;
-  const int base = lane < 9 ? 0 : (DO_V ? 18 : 0);
-  const int ire = base + 2 * e, iim = ire + 1;
-  const R vre = __shfl_sync(0xffffffffu, mine, ire & 31), vim = __shfl_sync(0xffffffffu, mine, iim & 31);
-  R re = ire < 32 ? vre : extra[ire - 32 < 4 ? ire - 32 : 0];
-  R im = iim < 32 ? vim : extra[iim - 32 < 4 ? iim - 32 : 0];
-  float out_re = 0.f, out_im = 0.f;
-  int out_row = -1, out_col = -1;
-  if (lane < 18) {
-    const R sc = lane < 9 ? R(v_scale) : R(k_scale);
-    out_re = (float)(re * sc);
-    out_im = (float)(im * sc);
-    out_row = pick3(s0, s1, s2, pi_[e / 3]);
-    out_col = pick3(t0, t1, t2, pj_[e % 3]);
-  }
-  const size_t nv = (size_t)g.nv;
-  if (lane < 9 && DO_V) atomicAdd(&V[out_row * nv + out_col], make_float2(out_re, out_im));
-  if (lane >= 9 && lane < 18 && DO_K) {
-    float add_re = out_re;
-    if (NCOMMON == 3 && mass_coeff != 0.f) {
-      // P1 mass block of a coincident pair (integrand.h:257-278): area * sum_q w_q phi_a phi_b
-      const int e = lane - 9, a = pick3(pm.i0, pm.i1, pm.i2, e / 3), b = pick3(pm.j0, pm.j1, pm.j2, e % 3);
-      double m = 0.0;
-#pragma unroll
-      for (int q = 0; q < 6; q++) m += tri6_w(q) * tri6_phi(q, a) * tri6_phi(q, b);
-      add_re += (float)(mass_coeff * 0.5 * (double)Ji * m);
-    }
-    atomicAdd(&K[out_row * nv + out_col], make_float2(add_re, out_im));
   }
 }
 
-template <typename R, int NCOMMON, bool DO_V, bool DO_K>
-__global__ void __launch_bounds__(128)
-    singular_vk_kernel(GeomView g, const int2* __restrict__ pairs, int npairs, float k, float2* __restrict__ V,
-                       float2* __restrict__ K, float v_scale, float k_scale, float mass_coeff) {
-  const int pair = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (pair >= npairs) return;
-  const int ti = NCOMMON == 3 ? pair : pairs[pair].x;
-  const int tj = NCOMMON == 3 ? pair : pairs[pair].y;
-  singular_pair<R, NCOMMON, DO_V, DO_K>(g, ti, tj, k, V, K, v_scale, k_scale, mass_coeff);
+// Warp `w` of one problem's touching pairs: the triangles, the edge pairs, the
+// unordered vertex pairs.
+__host__ __device__ inline long long touch_warps(const GeomView& g) { return (long long)g.nt + g.n_edge + g.n_vert / 2; }
+template <bool DO_V, bool DO_K>
+__device__ __forceinline__ void touch_warp(const GeomView& g, long long w, float k, float2* __restrict__ V,
+                                           float2* __restrict__ K, float v_scale, float k_scale, float mass_coeff,
+                                           TouchShared& sm) {
+  const int warp = threadIdx.x >> 5;
+  const long long n0 = g.nt;
+  if (w < n0) {
+    touch_coincident<DO_V, DO_K>(g, (int)w, k, V, K, v_scale, mass_coeff, sm.c[warp]);
+  } else if (w < n0 + g.n_edge) {
+    const int2 p = g.edge_pairs[w - n0];
+    touch_pair<2, DO_V, DO_K>(g, p.x, p.y, k, V, K, v_scale, k_scale, sm.f[warp]);
+  } else {
+    const int2 p = g.vert_pairs[w - n0 - g.n_edge];
+    touch_pair<1, DO_V, DO_K>(g, p.x, p.y, k, V, K, v_scale, k_scale, sm.f[warp]);
+  }
+}
+
+template <bool DO_V, bool DO_K>
+__global__ void __launch_bounds__(kTouchThreads)
+    touch_vk_kernel(const __grid_constant__ GeomView g, float k, float2* __restrict__ V,
+                    float2* __restrict__ K, float v_scale, float k_scale, float mass_coeff) {
+  __shared__ TouchShared sm;
+  const long long w = (long long)blockIdx.x * kTouchWarps + (threadIdx.x >> 5);
+  if (w < touch_warps(g)) touch_warp<DO_V, DO_K>(g, w, k, V, K, v_scale, k_scale, mass_coeff, sm);
+  wait_previous();
 }
 
 // ---------------------------------------------------------------------------
@@ -783,22 +737,21 @@ struct BatchProblem {
   float2* V;
   float2* K;
   long long item_begin;   // prefix sum of regular items
-  long long pair_begin[3];  // prefix sums of coincident / edge / vertex pairs
+  long long touch_begin;  // prefix sum of touching-pair warps
 };
 
 struct BatchHeader {
   unsigned long long next_item;  // queue head (zeroed before each launch)
   int nproblems;
   int pad;
-  long long total_items;
-  long long total_pairs[3];
+  long long total_items, total_touch;
 };
 
-__device__ __forceinline__ int find_problem(const BatchProblem* probs, int np, long long x, int which) {
+__device__ __forceinline__ int find_problem(const BatchProblem* probs, int np, long long x, bool touch) {
   int lo = 0, hi = np - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    const long long b = which < 0 ? probs[mid].item_begin : probs[mid].pair_begin[which];
+    const long long b = touch ? probs[mid].touch_begin : probs[mid].item_begin;
     if (b <= x) lo = mid; else hi = mid - 1;
   }
   return lo;
@@ -810,6 +763,7 @@ __global__ void __launch_bounds__(kStripThreads, 2)
                                   float k_scale) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   VkWarp& sw = reinterpret_cast<VkWarp*>(smem_raw)[threadIdx.x >> 5];
+  launch_next();
   strip_init(sw);
   const int np = hdr->nproblems;
   const long long total = hdr->total_items;
@@ -824,7 +778,7 @@ __global__ void __launch_bounds__(kStripThreads, 2)
     if ((threadIdx.x & 31) == 0) item = (long long)atomicAdd(&hdr->next_item, 1ull);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= total) break;
-    const BatchProblem& P = probs[find_problem(probs, np, item, -1)];
+    const BatchProblem& P = probs[find_problem(probs, np, item, false)];
     pol.k = P.k;
     pol.V = P.V;
     pol.K = P.K;
@@ -833,25 +787,16 @@ __global__ void __launch_bounds__(kStripThreads, 2)
   }
 }
 
-template <typename R, int NCOMMON>
-__global__ void __launch_bounds__(128)
-    singular_vk_batch_kernel(const BatchHeader* __restrict__ hdr, const BatchProblem* __restrict__ probs,
-                             float v_scale, float k_scale, float mass_coeff) {
-  const int which = NCOMMON == 3 ? 0 : (NCOMMON == 2 ? 1 : 2);
-  const long long pair = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (pair >= hdr->total_pairs[which]) return;
-  const int pi = find_problem(probs, hdr->nproblems, pair, which);
-  const BatchProblem& P = probs[pi];
-  const int local = (int)(pair - P.pair_begin[which]);
-  int ti = local, tj = local;
-  if (NCOMMON == 2) {
-    ti = P.g.edge_pairs[local].x;
-    tj = P.g.edge_pairs[local].y;
-  } else if (NCOMMON == 1) {
-    ti = P.g.vert_pairs[local].x;
-    tj = P.g.vert_pairs[local].y;
+__global__ void __launch_bounds__(kTouchThreads)
+    touch_vk_batch_kernel(const BatchHeader* __restrict__ hdr, const BatchProblem* __restrict__ probs, float v_scale,
+                          float k_scale, float mass_coeff) {
+  __shared__ TouchShared sm;
+  const long long w = (long long)blockIdx.x * kTouchWarps + (threadIdx.x >> 5);
+  if (w < hdr->total_touch) {
+    const BatchProblem& P = probs[find_problem(probs, hdr->nproblems, w, true)];
+    touch_warp<true, true>(P.g, w - P.touch_begin, P.k, P.V, P.K, v_scale, k_scale, mass_coeff, sm);
   }
-  singular_pair<R, NCOMMON, true, true>(P.g, ti, tj, P.k, P.V, P.K, v_scale, k_scale, mass_coeff);
+  wait_previous();
 }
 
 // Dense P1 mass matrix, one thread per triangle (bind.cu:10-21).
@@ -907,18 +852,12 @@ int launch_regular(const GeomView& g, float k, float2* V, float2* K, float v_sca
 }
 
 template <bool DO_V, bool DO_K>
-int launch_singular(const GeomView& g, float k, float2* V, float2* K, float v_scale, float k_scale, float mass_coeff,
-                    cudaStream_t s) {
-  const int wpb = 4;  // warps per block
-  (singular_vk_kernel<double, 3, DO_V, DO_K><<<(g.nt + wpb - 1) / wpb, 32 * wpb, 0, s>>>(
-      g, nullptr, g.nt, k, V, K, v_scale, k_scale, mass_coeff), count_launch());
-  if (g.n_edge)
-    (singular_vk_kernel<float, 2, DO_V, DO_K><<<(g.n_edge + wpb - 1) / wpb, 32 * wpb, 0, s>>>(
-        g, g.edge_pairs, g.n_edge, k, V, K, v_scale, k_scale, 0.f), count_launch());
-  if (g.n_vert)
-    (singular_vk_kernel<float, 1, DO_V, DO_K><<<(g.n_vert + wpb - 1) / wpb, 32 * wpb, 0, s>>>(
-        g, g.vert_pairs, g.n_vert, k, V, K, v_scale, k_scale, 0.f), count_launch());
-  BEM_CUDA_TRY(cudaGetLastError());
+int launch_touch(const GeomView& g, float k, float2* V, float2* K, float v_scale, float k_scale, float mass_coeff,
+                 cudaStream_t s) {
+  EarlyLaunch l((unsigned)((touch_warps(g) + kTouchWarps - 1) / kTouchWarps), kTouchThreads, 0, s);
+  if (!(DO_V && DO_K)) l.cfg.numAttrs = 0;  // regular_vk_kernel does not start it early
+  BEM_CUDA_TRY(cudaLaunchKernelEx(&l.cfg, touch_vk_kernel<DO_V, DO_K>, g, k, V, K, v_scale, k_scale, mass_coeff));
+  count_launch();
   return BEM_OK;
 }
 
@@ -965,13 +904,13 @@ int assemble_vk(const GeomView& g, float k, float2* V, float2* Kout, float mass_
   int rc;
   if (V && Kout) {
     if ((rc = launch_strip_vk(g, k, V, Kout, v_scale, k_scale, s))) return rc;
-    return launch_singular<true, true>(g, k, V, Kout, v_scale, k_scale, mass_coeff, s);
+    return launch_touch<true, true>(g, k, V, Kout, v_scale, k_scale, mass_coeff, s);
   } else if (V) {
     if ((rc = launch_regular<true, false>(g, k, V, nullptr, v_scale, 0.f, s))) return rc;
-    return launch_singular<true, false>(g, k, V, nullptr, v_scale, 0.f, 0.f, s);
+    return launch_touch<true, false>(g, k, V, nullptr, v_scale, 0.f, 0.f, s);
   } else if (Kout) {
     if ((rc = launch_regular<false, true>(g, k, nullptr, Kout, 0.f, k_scale, s))) return rc;
-    return launch_singular<false, true>(g, k, nullptr, Kout, 0.f, k_scale, mass_coeff, s);
+    return launch_touch<false, true>(g, k, nullptr, Kout, 0.f, k_scale, mass_coeff, s);
   }
   return BEM_OK;
 }
@@ -1092,7 +1031,7 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
   BatchProblem* hp = (BatchProblem*)((char*)t_stage.buf + hbytes);
   std::memset(hh, 0, sizeof(BatchHeader));
   hh->nproblems = np;
-  long long items = 0, pairs[3] = {0, 0, 0}, steps = 0;
+  long long items = 0, touch = 0, steps = 0;
   for (int p = 0; p < np; p++) steps += strip_steps(views[p].nblocks);
   // about 8 items per warp over the whole batch, at most 16 trial blocks each
   const long long share = std::min<long long>(512, std::max<long long>(4, steps / (8 * grid * kStripWarps)));
@@ -1111,38 +1050,25 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
     P.K = Ks[p];
     P.item_begin = items;
     items += P.items.items;
-    P.pair_begin[0] = pairs[0];
-    P.pair_begin[1] = pairs[1];
-    P.pair_begin[2] = pairs[2];
-    pairs[0] += g.nt;
-    pairs[1] += g.n_edge;
-    pairs[2] += g.n_vert;
+    P.touch_begin = touch;
+    touch += touch_warps(g);
   }
   hh->total_items = items;
-  for (int t = 0; t < 3; t++) hh->total_pairs[t] = pairs[t];
+  hh->total_touch = touch;
   BatchHeader* dh = (BatchHeader*)ws;
   BatchProblem* dp = (BatchProblem*)((char*)ws + hbytes);
   BEM_CUDA_TRY(cudaMemcpyAsync(ws, t_stage.buf, hbytes + pbytes, cudaMemcpyHostToDevice, s));
   BEM_CUDA_TRY(cudaEventRecord(t_stage.ev, s));
   const float v_scale = kInv4Pi, k_scale = -kInv4Pi * k_coeff;
   const long long blocks = (items + kStripWarps - 1) / kStripWarps;
-  if (items > 0)
-    (regular_strip_vk_batch_kernel<<<(unsigned)(grid < blocks ? grid : blocks), kStripThreads,
-                                     kStripWarps * sizeof(VkWarp), s>>>(dh, dp, v_scale, k_scale),
-     count_launch());
-  const int wpb = 4;
-  if (pairs[0])
-    (singular_vk_batch_kernel<double, 3><<<(unsigned)((pairs[0] + wpb - 1) / wpb), 32 * wpb, 0, s>>>(
-         dh, dp, v_scale, k_scale, mass_coeff),
-     count_launch());
-  if (pairs[1])
-    (singular_vk_batch_kernel<float, 2><<<(unsigned)((pairs[1] + wpb - 1) / wpb), 32 * wpb, 0, s>>>(
-         dh, dp, v_scale, k_scale, mass_coeff),
-     count_launch());
-  if (pairs[2])
-    (singular_vk_batch_kernel<float, 1><<<(unsigned)((pairs[2] + wpb - 1) / wpb), 32 * wpb, 0, s>>>(
-         dh, dp, v_scale, k_scale, mass_coeff),
-     count_launch());
+  (regular_strip_vk_batch_kernel<<<(unsigned)(grid < blocks ? grid : blocks), kStripThreads,
+                                   kStripWarps * sizeof(VkWarp), s>>>(dh, dp, v_scale, k_scale),
+   count_launch());
+  BEM_CUDA_TRY(cudaGetLastError());
+  EarlyLaunch l((unsigned)((touch + kTouchWarps - 1) / kTouchWarps), kTouchThreads, 0, s);
+  BEM_CUDA_TRY(cudaLaunchKernelEx(&l.cfg, touch_vk_batch_kernel, (const BatchHeader*)dh, (const BatchProblem*)dp,
+                                  v_scale, k_scale, mass_coeff));
+  count_launch();
   BEM_CUDA_TRY(cudaGetLastError());
   return BEM_OK;
 }

@@ -166,7 +166,7 @@ struct GeomHeader {
   uint64_t off_trirec_orig;  // TriRec[nt] in input order
   uint64_t off_tiles;      // TileRec[ntiles]
   uint64_t off_edge_pairs;  // int2[n_edge]  (test tri, trial tri), input ids
-  uint64_t off_vert_pairs;  // int2[n_vert]
+  uint64_t off_vert_pairs;  // int2[n_vert], first those with test < trial (half of them)
   uint64_t off_normals;    // float[nt*3]
   uint64_t off_curls;      // float[nt*9]   rows: n x grad(phi_b)
   uint64_t off_bmrec;      // BmRec[nt] in sorted order
@@ -212,12 +212,39 @@ __device__ __forceinline__ int tile_group_of(long long pos, int n) {
 }
 
 // ---- small math -------------------------------------------------------------
-// sine and cosine of one argument: the library sincos in FP64
+// FP64 phases of touching triangles are small (k times their size): Taylor sums
+// up to x^15 and x^16, below 1e-16 off for |x| <= pi / 4; the library beyond.
+__device__ __forceinline__ void sincos_touch(double x, double* s, double* c) {
+  if (fabs(x) > 0.78539816339744831) {
+    sincos(x, s, c);
+    return;
+  }
+  const double t = x * x;
+  double p = -1.0 / 1307674368000.0;
+  p = fma(p, t, 1.0 / 6227020800.0);
+  p = fma(p, t, -1.0 / 39916800.0);
+  p = fma(p, t, 1.0 / 362880.0);
+  p = fma(p, t, -1.0 / 5040.0);
+  p = fma(p, t, 1.0 / 120.0);
+  p = fma(p, t, -1.0 / 6.0);
+  *s = fma(p * t, x, x);
+  double q = 1.0 / 20922789888000.0;
+  q = fma(q, t, -1.0 / 87178291200.0);
+  q = fma(q, t, 1.0 / 479001600.0);
+  q = fma(q, t, -1.0 / 3628800.0);
+  q = fma(q, t, 1.0 / 40320.0);
+  q = fma(q, t, -1.0 / 720.0);
+  q = fma(q, t, 1.0 / 24.0);
+  q = fma(q, t, -0.5);
+  *c = fma(q, t, 1.0);
+}
+
+// sine and cosine of a touching pair's phase
 template <typename R>
 __device__ __forceinline__ void sincos_t(R x, R* s, R* c);
 template <>
 __device__ __forceinline__ void sincos_t<double>(double x, double* s, double* c) {
-  sincos(x, s, c);
+  sincos_touch(x, s, c);
 }
 // FP32 (edge and vertex pairs of the touching-pair kernels): the hardware
 // approximation, accurate to a few 1e-7 absolute for the |k r| <= ~1 of
@@ -227,16 +254,42 @@ __device__ __forceinline__ void sincos_t<float>(float x, float* s, float* c) {
   __sincosf(x, s, c);
 }
 
-// 1 / r and r from r^2 (r clamped to kEps as in potential.h): rsqrt in FP32, a
-// correctly rounded sqrt and division in FP64.
+// Totals over the warp of N values per lane: value v in total[v] (one warp's
+// shared memory, ROUNDUP(N, 32) entries), visible to all lanes on return.
+// Groups of 32 values by a transpose: every round halves the values a lane
+// keeps, so a group costs 31 shuffles instead of 5 per value.
+template <int N, typename R>
+__device__ __forceinline__ void warp_totals(const R (&v)[N], R* total) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int g = 0; g < N; g += 32) {
+    R t[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) t[i] = g + i < N ? v[g + i < N ? g + i : 0] : R(0);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      const bool hi = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < o; i++) {
+        const R send = hi ? t[i] : t[i + o];
+        const R keep = hi ? t[i + o] : t[i];
+        t[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    total[g + lane] = t[0];
+  }
+  __syncwarp();
+}
+
+// 1 / r and r from r^2 (r clamped to kEps as in potential.h).
 template <typename R>
 __device__ __forceinline__ void inv_dist(R r2, R* r, R* inv_r);
 template <>
 __device__ __forceinline__ void inv_dist<double>(double r2, double* r, double* inv_r) {
-  double rr = sqrt(r2);
-  if (rr < kEps) rr = kEps;
-  *r = rr;
-  *inv_r = 1.0 / rr;
+  r2 = fmax(r2, (double)kEps * (double)kEps);
+  const double ri = rsqrt(r2);
+  *inv_r = ri;
+  *r = r2 * ri;
 }
 template <>
 __device__ __forceinline__ void inv_dist<float>(float r2, float* r, float* inv_r) {

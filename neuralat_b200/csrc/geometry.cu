@@ -41,7 +41,7 @@ struct HostGeom {
   std::vector<int> slots;
   std::vector<TileRec> tiles;
   std::vector<BlockRec> blocks;
-  std::vector<int2> edge_pairs, vert_pairs;
+  std::vector<int2> edge_pairs, vert_pairs, vert_mirror;  // vert_pairs: test < trial, vert_mirror: test > trial
   int max_valence = 0;
   GeomHeader hdr{};
 };
@@ -94,6 +94,7 @@ int analyse(const float* d_vertices, int nv, const int* d_triangles, int nt, cud
   t_stage_ok = false;
   t_last.edge_pairs.clear();  // the vectors keep their capacity from mesh to mesh
   t_last.vert_pairs.clear();
+  t_last.vert_mirror.clear();
   t_last.max_valence = 0;
   t_last.nv = nv;
   t_last.nt = nt;
@@ -332,7 +333,8 @@ int analyse_host(HostGeom& g) {
   std::vector<int> nbr(3 * (size_t)nt, -1);  // triangles across an edge (three at most are used)
   std::vector<int> touch, shared(nt, 0);  // triangles meeting i in the order of its stars, vertices shared with each
   g.edge_pairs.reserve(3 * (size_t)nt);
-  g.vert_pairs.reserve(10 * (size_t)nt);
+  g.vert_pairs.reserve(5 * (size_t)nt);
+  g.vert_mirror.reserve(5 * (size_t)nt);
   for (int i = 0; i < nt; i++) {
     const int* ti = &g.triangles[3 * (size_t)i];
     touch.clear();
@@ -355,7 +357,7 @@ int analyse_host(HostGeom& g) {
         g.edge_pairs.push_back(make_int2(i, j));
         if (edges < 3) nbr[3 * (size_t)i + edges++] = j;
       } else {
-        g.vert_pairs.push_back(make_int2(i, j));
+        (i < j ? g.vert_pairs : g.vert_mirror).push_back(make_int2(i, j));
       }
     }
   }
@@ -393,7 +395,7 @@ int analyse_host(HostGeom& g) {
   h.nt = nt;
   h.ntiles = g.ntiles;
   h.n_edge = (int)g.edge_pairs.size();
-  h.n_vert = (int)g.vert_pairs.size();
+  h.n_vert = (int)(g.vert_pairs.size() + g.vert_mirror.size());
   h.max_valence = g.max_valence;
   uint64_t off = align_up(sizeof(GeomHeader), 256);
   auto take = [&](uint64_t bytes) {
@@ -607,7 +609,11 @@ extern "C" int bem_geometry_build(const float* vertices, int nv, const int* tria
     std::memcpy(st + h.off_blocks, g.blocks.data(), sizeof(BlockRec) * (size_t)g.nblocks);
     std::memcpy(st + h.off_tiles, g.tiles.data(), sizeof(TileRec) * (size_t)g.ntiles);
     if (h.n_edge) std::memcpy(st + h.off_edge_pairs, g.edge_pairs.data(), sizeof(int2) * h.n_edge);
-    if (h.n_vert) std::memcpy(st + h.off_vert_pairs, g.vert_pairs.data(), sizeof(int2) * h.n_vert);
+    if (h.n_vert) {
+      const size_t half = sizeof(int2) * g.vert_pairs.size();
+      std::memcpy(st + h.off_vert_pairs, g.vert_pairs.data(), half);
+      std::memcpy(st + h.off_vert_pairs + half, g.vert_mirror.data(), sizeof(int2) * g.vert_mirror.size());
+    }
     t_stage_ok = true;
   }
   BEM_CUDA_TRY(cudaMemcpyAsync(geom, t_stage.p, nstage, cudaMemcpyHostToDevice, s));

@@ -19,6 +19,28 @@
 
 namespace bemb {
 
+// Programmatic launch: lets the next kernel start as soon as every block of
+// this one runs / waits for the kernels before this one to finish.
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launch attributes of a kernel that may start while the one before it in the
+// stream still runs (it calls wait_previous() before it ends).
+struct EarlyLaunch {
+  cudaLaunchAttribute attr{};
+  cudaLaunchConfig_t cfg{};
+  EarlyLaunch(unsigned blocks, int threads, size_t smem, cudaStream_t s) {
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+  }
+};
+
 constexpr int kStripThreads = 128;
 constexpr int kStripWarps = kStripThreads / 32;
 constexpr int kStripZero = kBlockCorners;  // index of a column entry that stays zero

@@ -68,18 +68,14 @@ def test_block_edges(name):
     v, t, k = v.astype(np.float32), t.astype(np.int32), 21.7
     s = BEM_Solver(torch.from_numpy(v).cuda(), torch.from_numpy(t).cuda())
     v64, M = v.astype(np.float64), O.identity_matrix(v.astype(np.float64), t)
-    V, A = (x.cpu().numpy() for x in s.assemble_vk(k))
-    K = O.boundary_matrix("double", v64, t, k)
-    assert rel(V, O.boundary_matrix("single", v64, t, k)) < TOL
-    assert rel(A, 0.5 * M - K) < TOL
-    (Vb, Ab), = assemble_batch([s], [k])
-    assert rel(Vb.cpu().numpy(), V) < 1e-6 and rel(Ab.cpu().numpy(), A) < 1e-6
+    refs = (O.boundary_matrix("single", v64, t, k), 0.5 * M - O.boundary_matrix("double", v64, t, k))
+    for pair in (s.assemble_vk(k), assemble_batch([s], [k])[0]):  # one problem, and the same through the queue
+        assert all(rel(x.cpu().numpy(), y) < TOL for x, y in zip(pair, refs))
     for approx, order in ((True, "_approx"), (False, "")):
-        L, R = (x.cpu().numpy() for x in s.assemble_bm(k, approx=approx))
-        assert rel(L, O.boundary_matrix("bm_lhs", v64, t, k, order) + 0.5 * M) < TOL
-        assert rel(R, O.boundary_matrix("bm_rhs", v64, t, k, order) - 0.5j / k * M) < TOL
-        (Lb, Rb), = assemble_batch_bm([s], [k], approx=approx)
-        assert rel(Lb.cpu().numpy(), L) < 1e-6 and rel(Rb.cpu().numpy(), R) < 1e-6
+        refs = (O.boundary_matrix("bm_lhs", v64, t, k, order) + 0.5 * M,
+                O.boundary_matrix("bm_rhs", v64, t, k, order) - 0.5j / k * M)
+        for pair in (s.assemble_bm(k, approx=approx), assemble_batch_bm([s], [k], approx=approx)[0]):
+            assert all(rel(x.cpu().numpy(), y) < TOL for x, y in zip(pair, refs))
     for layer in ("hypersingular", "bm_lhs"):  # the sorted records' curls in the general kernel
         got = s.assemble_boundary_matrix(k, layer, approx=True).cpu().numpy()
         assert rel(got, O.boundary_matrix(layer, v64, t, k, "_approx")) < TOL
