@@ -119,45 +119,53 @@ __device__ __forceinline__ void listen_triangle(const TriRec& r, float px, float
   }
 }
 
-constexpr int kLsThreads = 128;  // listeners per CTA
+constexpr int kLsThreads = 128;
+constexpr int kLsWarps = kLsThreads / 32;
+constexpr int kLsChunk = 16;  // triangles staged per warp
 
 // out[p, s] += -S neumann + D dirichlet over the triangles of one run
-// (blockIdx.y), for up to M <= 4 right-hand sides: the products with the
-// vertex densities stay in the listener's own registers.
+// (blockIdx.y) for 32 listeners, up to M <= 4 right-hand sides: the products
+// with the vertex densities stay in the listener's own registers.  Each warp
+// walks a quarter of the run; their sums meet in shared memory, so that few
+// FP32 terms are added to an output one after the other.
 //
 // Bound by the FP32 and sincos units (about 125 instructions for the 6 points
 // of a triangle).  Measured on B200: 1000 listeners x 5110 triangles x 1
-// right-hand side 43 us, against 165 us with the densities
-// interpolated onto the quadrature points by a pass of their own and 8 products
-// per point and right-hand side.
+// right-hand side 46 us, against 165 us with the densities interpolated onto
+// the quadrature points by a pass of their own and 8 products per point and
+// right-hand side.
 template <int M>
 __global__ void __launch_bounds__(kLsThreads)
     listen_few_kernel(GeomView g, const float* __restrict__ pts, int np, float k, const float2* __restrict__ neu,
                       const float2* __restrict__ dir, int nrhs, int run, float2* __restrict__ out) {
-  __shared__ TriRec rec[kBlock];
-  __shared__ float4 dens[kBlock][3][M];  // (neumann, dirichlet) at the triangle's vertices
-  const int tid = threadIdx.x, p = blockIdx.x * kLsThreads + tid;
+  __shared__ TriRec rec_s[kLsWarps][kLsChunk];
+  __shared__ float4 dens_s[kLsWarps][kLsChunk][3][M];  // (neumann, dirichlet) at the triangle's vertices
+  __shared__ float2 sum_s[kLsWarps][M][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
+  TriRec* rec = rec_s[warp];
+  float4(*dens)[3][M] = dens_s[warp];
   const float* x = pts + 3 * (size_t)min(p, np - 1);
   const float px = x[0], py = x[1], pz = x[2];
-  const int t0 = blockIdx.y * run, t1 = min(t0 + run, g.nt);
+  const int part = (run + kLsWarps - 1) / kLsWarps, r0 = blockIdx.y * run;
+  const int t0 = min(r0 + warp * part, g.nt), t1 = min(min(t0 + part, r0 + run), g.nt);
   ListenSums acc;
 #pragma unroll
   for (int b = 0; b < 3; b++) acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
   float2 sum[M];
 #pragma unroll
   for (int s = 0; s < M; s++) sum[s] = make_float2(0.f, 0.f);
-  for (int c0 = t0; c0 < t1; c0 += kBlock) {
-    const int n = min(kBlock, t1 - c0);
-    __syncthreads();
-    for (int e = tid; e < 8 * n; e += kLsThreads) ((float4*)rec)[e] = ((const float4*)&g.rec[c0])[e];
-    for (int e = tid; e < 3 * M * n; e += kLsThreads) {
+  for (int c0 = t0; c0 < t1; c0 += kLsChunk) {
+    const int n = min(kLsChunk, t1 - c0);
+    __syncwarp();
+    for (int e = lane; e < 8 * n; e += 32) ((float4*)rec)[e] = ((const float4*)&g.rec[c0])[e];
+    for (int e = lane; e < 3 * M * n; e += 32) {
       const int t = e / (3 * M), b = (e / M) % 3, s = e % M;
       const size_t at = (size_t)g.rec[c0 + t].v[b] * nrhs + s;
       const float2 zero = make_float2(0.f, 0.f);
       const float2 a = neu && s < nrhs ? neu[at] : zero, u = dir && s < nrhs ? dir[at] : zero;
       dens[t][b][s] = make_float4(a.x, a.y, u.x, u.y);
     }
-    __syncthreads();
+    __syncwarp();
 #pragma unroll 1
     for (int t = 0; t < n; t++) {
       listen_triangle(rec[t], px, py, pz, k, acc);
@@ -176,10 +184,17 @@ __global__ void __launch_bounds__(kLsThreads)
       }
     }
   }
-  if (p < np) {
 #pragma unroll
-    for (int s = 0; s < M; s++)
-      if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], sum[s]);
+  for (int s = 0; s < M; s++) sum_s[warp][s][lane] = sum[s];
+  __syncthreads();
+  if (warp == 0 && p < np) {
+#pragma unroll
+    for (int s = 0; s < M; s++) {
+      float2 t = sum_s[0][s][lane];
+#pragma unroll
+      for (int w = 1; w < kLsWarps; w++) t = f2_add(t, sum_s[w][s][lane]);
+      if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], t);
+    }
   }
 }
 
@@ -386,8 +401,8 @@ int listen_run(int groups, int nt, long long slots, int least) {
 template <int M>
 void listen_few(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
                 float2* out, int sms, cudaStream_t s) {
-  const int groups = (np + kLsThreads - 1) / kLsThreads;
-  const int run = listen_run(groups, g.nt, 8LL * sms, 4);
+  const int groups = (np + 31) / 32;
+  const int run = listen_run(groups, g.nt, 8LL * sms, 16);
   (listen_few_kernel<M><<<dim3(groups, (g.nt + run - 1) / run), kLsThreads, 0, s>>>(g, pts, np, k, neu, dir, nrhs, run,
                                                                                  out),
    count_launch());
