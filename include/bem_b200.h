@@ -188,7 +188,9 @@ enum {
   BEM_TUNE_GMRES_REORTH = 4,         /* Arnoldi Gram-Schmidt passes: 0 automatic (one), 1 one, 2 two */
   BEM_TUNE_ARNOLDI_CLUSTER = 5,      /* largest thread-block cluster (<= 16 CTAs) per Krylov column in
                                         the Arnoldi kernel (0: automatic) */
-  BEM_TUNE_ARNOLDI_MODE = 6,         /* Arnoldi step: 0 automatic (1), 1 one cluster kernel per step,
+  BEM_TUNE_ARNOLDI_MODE = 6,         /* Arnoldi step: 0 automatic (one right-hand side at FP32 level: a whole
+                                        cycle per launch where the basis fits in shared memory; else 1), 1 one
+                                        cluster kernel per step,
                                         2 streamed kernels over all SMs, 3 one cooperative kernel over
                                         all SMs (two grid barriers; falls back to 1 when its grid does
                                         not fit) */

@@ -2626,6 +2626,8 @@ int launch_block_xupdate(const GmPtrs& P, const BkPtrs& K, int na, cudaStream_t 
   return BEM_OK;
 }
 
+#include "krylov_cycle.cuh"
+
 // Back substitution H y = g on the Givens-reduced Hessenberg matrix, one
 // warp per column, column-oriented: y_j = g_j / H_jj, then the lanes update
 // g_0..g_{j-1} -= y_j H_{0..j-1, j} (column j of H is contiguous).
@@ -2803,7 +2805,7 @@ inline size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
 struct Layout {
   size_t Vb, H, cs, sn, g, w, d, x, r, X, Y, norm2, rnorm2, beta, tol, resid, active, kend, kcol, colstep, y, st,
-      bnorm2, hacc, nacc, bk_hacc, bk_gacc, bk_y, bk_step, tc, total;
+      bnorm2, hacc, nacc, cy, bk_hacc, bk_gacc, bk_y, bk_step, tc, total;
 };
 
 Layout layout(int n, int m, int R, int precision) {
@@ -2839,6 +2841,7 @@ Layout layout(int n, int m, int R, int precision) {
   L.bnorm2 = take(sizeof(double) * m);
   L.hacc = take(sizeof(double) * 2 * (size_t)m * 4 * (R + 1));
   L.nacc = take(sizeof(double) * 2 * (size_t)m * 3);
+  L.cy = take(m == 1 ? cy_global_bytes(R) : 0);
   // block solver state (used when 2 <= m <= kBkMaxP)
   const bool bk = m >= 2 && m <= kBkMaxRhs;
   size_t sh = 0, sg = 0, sy = 0;
@@ -3226,6 +3229,69 @@ struct CoShape {
   size_t smem = 0;
 };
 
+// Launch shape of gm_single_kernel: one CTA per SM at most, at least 16 unknowns
+// each (small systems leave SMs to the solves beside them and have a cheaper
+// barrier), the CTA's slice of the whole basis and one vector in shared memory.
+struct CyShape {
+  int rows = 0, grid = 0;
+  size_t smem = 0;
+};
+
+int cycle_shape(int n, int R, CyShape* out) {
+  int dev = 0, coop_ok = 0, smem_optin = 0, sms = 0;
+  BEM_CUDA_TRY(cudaGetDevice(&dev));
+  BEM_CUDA_TRY(cudaDeviceGetAttribute(&coop_ok, cudaDevAttrCooperativeLaunch, dev));
+  BEM_CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  BEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (!coop_ok) return BEM_ERR_UNSUPPORTED;
+  const int rows = std::max(16, (n + sms - 1) / sms);
+  const size_t smem = cy_layout(n, rows, R).total;
+  if (smem + 1024 > (size_t)smem_optin) return BEM_ERR_UNSUPPORTED;  // 1 KB for the static shared memory
+  BEM_CUDA_TRY(cudaFuncSetAttribute(gm_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int occ = 0;
+  BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gm_single_kernel, kCyThreads, smem));
+  out->rows = rows;
+  out->grid = (n + rows - 1) / rows;
+  out->smem = smem;
+  return occ >= 1 && out->grid <= occ * sms ? BEM_OK : BEM_ERR_UNSUPPORTED;
+}
+
+int solve_single(const GmPtrs& P, const CyShape& shape, const float2* A, const float2* B, float2* X, int use_x0,
+                 const bem_solver_params* params, CyGlobal* G, bem_solver_info* info, cudaStream_t s) {
+  BEM_CUDA_TRY(cudaMemsetAsync(G, 0, cy_global_bytes(P.R), s));
+  CyParams prm;
+  prm.rtol = params->rtol;
+  prm.atol = params->atol;
+  prm.inner_rtol = 3e-7;  // one cycle to the target unless it is below FP32 accuracy; then refinement takes over
+  prm.max_iters = params->max_iters;
+  prm.max_refine = params->max_refine;
+  prm.use_x0 = use_x0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)shape.grid, 1, 1);
+  cfg.blockDim = dim3(kCyThreads, 1, 1);
+  cfg.dynamicSmemBytes = shape.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  BEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, gm_single_kernel, P, A, B, X, G, shape.rows, prm));
+  count_launch();
+  CyGlobal out;
+  BEM_CUDA_TRY(cudaMemcpyAsync(&out, G, sizeof(out), cudaMemcpyDeviceToHost, s));
+  BEM_CUDA_TRY(cudaStreamSynchronize(s));
+  const int status = out.state.err ? (int)BEM_ERR_CUDA : out.status;  // a bounded barrier wait expired
+  if (info) {
+    info->status = status;
+    info->iterations = out.iterations;
+    info->refinements = out.refinements;
+    info->matvecs = out.matvecs;
+    info->rel_residual = out.rel;
+  }
+  return status;
+}
+
 int coop_shape(int n, int m, int R, CoShape* out) {
   static std::atomic<bool> attr{false};
   int dev = 0, coop_ok = 0, smem_optin = 0;
@@ -3443,6 +3509,12 @@ extern "C" int bem_gmres_solve(const void* A, int n, const void* B, int m, void*
   P.nacc = (double*)(w + L.nacc);
   double* rnorm2 = (double*)(w + L.rnorm2);
   void* tcws = w + L.tc;
+  // one right-hand side at FP32 level: whole cycles in one launch where the
+  // basis fits (its FP32 products are at least as accurate as fp16x3's)
+  CyShape cyc;
+  const bool cycle = m == 1 && (params->precision == BEM_PREC_FP32 || params->precision == BEM_PREC_FP16X3) &&
+                     g_arn_mode == 0 && g_gmres_reorth != 2 && cycle_shape(n, R, &cyc) == BEM_OK;
+  if (cycle) return solve_single(P, cyc, (const float2*)A, (const float2*)B, (float2*)X, use_x0, params, (CyGlobal*)(w + L.cy), info, s);
   const int prec = params->precision;
   // block Krylov spaces (see gm_block_kernel): one for 2..16 right-hand
   // sides, groups of <= 16 columns for up to 64, one shared matvec per step
