@@ -7,8 +7,8 @@
 // copies start and end a solve.  Here a CTA owns rows of A and the same unknowns
 // of every vector for the whole solve, and its slice of the basis never leaves
 // shared memory.  Per step:
-//   x = v_k (all of it, from L2);  w = A x on the CTA's rows: the 15 warps split
-//     the columns and sweep 8 rows at a time, FP32 products, row sums in FP64;
+//   x = v_k (all of it, from L2);  w = A x on the CTA's rows: a warp sweeps 1, 2
+//     or 4 rows at once, FP32 products, the lanes' sums added in FP64;
 //   <v_j, w> and |w|^2 over the slice in FP64, added over the CTAs by FP64
 //     atomics (8 copies, so that no address takes more than 19 additions);
 //   == grid barrier ==
@@ -25,17 +25,20 @@
 // host loop of the other paths; every CTA takes the same decisions from the
 // same sums.
 //
-// Bound by the matrix (8 n^2 bytes per step, from L2) and the latency of the two
-// barriers (about 8 us per step).  Measured on B200, a whole solve, against a
-// launch pair per step: 597 unknowns, 39 steps, 0.50 and 1.31 ms; 2487 unknowns,
-// 46 steps, 0.84 and 1.97 ms; 5762 unknowns, 32 steps, 1.83 and 2.47 ms.
+// Bound by the matrix (8 n^2 bytes per step, from L2 up to about 3500 unknowns)
+// and the latency of the two barriers (about 7 us per step).  Measured on B200, a
+// whole solve, against a launch pair per step: 597 unknowns, 39 steps, 0.40 and
+// 1.31 ms; 2487 unknowns, 46 steps, 0.81 and 1.97 ms; 5762 unknowns, 32 steps,
+// 1.80 and 2.45 ms; 8412 unknowns, 32 steps, 3.81 and 3.79 ms; 10 242 unknowns,
+// 32 steps, 7.4 and 5.1 ms (hence kCyMaxRows).
 // Barrier waits are bounded (state.err on expiry, after which every CTA leaves).
 
 constexpr int kCyWarps = 15;
 constexpr int kCyCompute = 32 * kCyWarps;
 constexpr int kCyThreads = kCyCompute + 32;  // + the Givens warp (512: 128 registers each)
 constexpr int kCyCopies = 8;
-constexpr int kCyRows = 8;  // rows of A a warp sweeps together
+constexpr int kCyMinRows = kCyWarps;  // unknowns per CTA: a row per warp at the least
+constexpr int kCyMaxRows = 50;        // above, the matvec kernels stream the matrix faster
 
 struct CyParams {
   double rtol, atol, inner_rtol;
@@ -82,10 +85,7 @@ __host__ __device__ inline CyLayout cy_layout(int n, int rows, int R) {
   L.gs = take(sizeof(double2) * (R + 2));
   L.hc = take(sizeof(double2) * (R + 2));
   L.cs = take(sizeof(double) * R);
-  // matvec: [kCyWarps][2 rows] doubles (rows rounded up to kCyRows); dots: a double2 per thread
-  const size_t mv = sizeof(double) * 2 * kCyWarps * (size_t)((rows + kCyRows - 1) / kCyRows * kCyRows);
-  const size_t dt = sizeof(double2) * kCyCompute;
-  L.part = take(mv > dt ? mv : dt);
+  L.part = take(sizeof(double2) * kCyCompute);  // a double2 per thread
   L.total = o;
   return L;
 }
@@ -159,25 +159,56 @@ __device__ __forceinline__ double cy_givens(double2* hc, int k, double hn, doubl
   return sqrt(g1.x * g1.x + g1.y * g1.y);
 }
 
-// acc[r] += A[row r][j] x[j] over columns j0.. (step 32 from `lane`), kCyRows rows.
-template <typename T2, typename T, typename X>
-__device__ __forceinline__ void cy_rows(const float2* __restrict__ A, int n, int row0, int last, int j, int j1, X&& x,
-                                        T2 (&acc)[kCyRows]) {
-  const float2* row[kCyRows];
+// w = A x on the CTA's rows (compute warps): a warp sweeps RG rows at once, its
+// lanes the columns, U columns in flight; passes of 15 RG rows.
+template <int RG, int U, typename T2, typename T, typename X>
+__device__ __forceinline__ void cy_sweep(const float2* __restrict__ A, int n, int i0, int rows, X&& x, double2* w) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r0 = warp; r0 < rows; r0 += RG * kCyWarps) {
+    const float2* row[RG];
+    T2 acc[RG];
 #pragma unroll
-  for (int r = 0; r < kCyRows; r++) {
-    row[r] = A + (size_t)min(row0 + r, last) * n;
-    acc[r].x = 0;
-    acc[r].y = 0;
-  }
+    for (int r = 0; r < RG; r++) {
+      row[r] = A + (size_t)(i0 + min(r0 + r * kCyWarps, rows - 1)) * n;
+      acc[r].x = 0;
+      acc[r].y = 0;
+    }
+    int j = lane;
+    for (; j + 32 * (U - 1) < n; j += 32 * U) {
+      float2 a[U][RG];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+#pragma unroll
+        for (int r = 0; r < RG; r++) a[u][r] = __ldcg(&row[r][j + 32 * u]);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const T2 v = x(j + 32 * u);
+#pragma unroll
+        for (int r = 0; r < RG; r++) {
+          acc[r].x = fma((T)a[u][r].x, v.x, fma((T)-a[u][r].y, v.y, acc[r].x));
+          acc[r].y = fma((T)a[u][r].x, v.y, fma((T)a[u][r].y, v.x, acc[r].y));
+        }
+      }
+    }
 #pragma unroll 2
-  for (; j < j1; j += 32) {
-    const T2 v = x(j);
+    for (; j < n; j += 32) {
+      const T2 v = x(j);
 #pragma unroll
-    for (int r = 0; r < kCyRows; r++) {
-      const float2 a = __ldcg(&row[r][j]);
-      acc[r].x = fma((T)a.x, v.x, fma((T)-a.y, v.y, acc[r].x));
-      acc[r].y = fma((T)a.x, v.y, fma((T)a.y, v.x, acc[r].y));
+      for (int r = 0; r < RG; r++) {
+        const float2 a = __ldcg(&row[r][j]);
+        acc[r].x = fma((T)a.x, v.x, fma((T)-a.y, v.y, acc[r].x));
+        acc[r].y = fma((T)a.x, v.y, fma((T)a.y, v.x, acc[r].y));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RG; r++) {
+      double re = (double)acc[r].x, im = (double)acc[r].y;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        re += __shfl_xor_sync(0xffffffffu, re, o);
+        im += __shfl_xor_sync(0xffffffffu, im, o);
+      }
+      if (lane == 0 && r0 + r * kCyWarps < rows) w[r0 + r * kCyWarps] = make_double2(re, im);
     }
   }
 }
@@ -211,7 +242,6 @@ __global__ void __launch_bounds__(kCyThreads, 1)
   const bool compute = warp < kCyWarps, givens = blockIdx.x == 0 && warp == kCyWarps;
   const int copy = blockIdx.x % kCyCopies;
   const int i0 = blockIdx.x * rows_per_cta, rows = min(rows_per_cta, n - i0);
-  const int seg = (n + kCyWarps - 1) / kCyWarps, j0 = warp * seg + lane, j1 = min(warp * seg + seg, n);
   unsigned bars = 0, sums = 0;
   __shared__ int s_done;
   __shared__ double s_sum;
@@ -255,52 +285,26 @@ __global__ void __launch_bounds__(kCyThreads, 1)
     ((j & 1) ? P.Y : P.X)[i0 + i] = f;
     return (double)f.x * f.x + (double)f.y * f.y;
   };
-  // compute threads: w = (sums of `acc`'s rows) for the CTA's rows, from per-warp partial sums
-  auto row_sums = [&]() {
-    cy_compute_sync();
-    for (int e = tid; e < 2 * rows; e += kCyCompute) {
-      double t = 0.0;
-      for (int q = 0; q < kCyWarps; q++) t += part[(size_t)q * 2 * ((rows + kCyRows - 1) / kCyRows * kCyRows) + e];
-      ((double*)w)[e] = t;
-    }
-    cy_compute_sync();
-  };
-  auto row_part = [&](int r0, double (&t)[2 * kCyRows]) {
-    const double mine = warp_reduce_scatter<2 * kCyRows, double>(t, lane);  // value lane >> 1
-    if ((lane & 1) == 0) part[(size_t)warp * 2 * ((rows + kCyRows - 1) / kCyRows * kCyRows) + 2 * r0 + (lane >> 1)] = mine;
-  };
   // compute threads: w = A v, FP32 products (v: all unknowns, complex64)
   auto product = [&](const float2* v) {
     for (int i = tid; i < n; i += kCyCompute) x[i] = __ldcg(&v[i]);
     cy_compute_sync();
-    for (int r0 = 0; r0 < rows; r0 += kCyRows) {
-      float2 acc[kCyRows];
-      cy_rows<float2, float>(A, n, i0 + r0, i0 + rows - 1, j0, j1, [&](int j) { return x[j]; }, acc);
-      double t[2 * kCyRows];
-#pragma unroll
-      for (int r = 0; r < kCyRows; r++) {
-        t[2 * r] = (double)acc[r].x;
-        t[2 * r + 1] = (double)acc[r].y;
-      }
-      row_part(r0, t);
-    }
-    row_sums();
+    auto xv = [&](int j) { return x[j]; };
+    if (rows_per_cta <= kCyWarps)
+      cy_sweep<1, 8, float2, float>(A, n, i0, rows, xv, w);
+    else if (rows_per_cta <= 2 * kCyWarps)
+      cy_sweep<2, 8, float2, float>(A, n, i0, rows, xv, w);
+    else if (rows_per_cta <= 3 * kCyWarps)
+      cy_sweep<3, 6, float2, float>(A, n, i0, rows, xv, w);
+    else
+      cy_sweep<4, 4, float2, float>(A, n, i0, rows, xv, w);
+    cy_compute_sync();
   };
   // compute threads: w = A x in FP64 (x: all unknowns, complex128)
   auto product64 = [&](const double2* v) {
-    for (int r0 = 0; r0 < rows; r0 += kCyRows) {
-      double2 acc[kCyRows];
-      cy_rows<double2, double>(A, n, i0 + r0, i0 + rows - 1, j0, j1,
-                               [&](int j) { return make_double2(__ldcg(&v[j].x), __ldcg(&v[j].y)); }, acc);
-      double t[2 * kCyRows];
-#pragma unroll
-      for (int r = 0; r < kCyRows; r++) {
-        t[2 * r] = acc[r].x;
-        t[2 * r + 1] = acc[r].y;
-      }
-      row_part(r0, t);
-    }
-    row_sums();
+    cy_sweep<2, 4, double2, double>(
+        A, n, i0, rows, [&](int j) { return make_double2(__ldcg(&v[j].x), __ldcg(&v[j].y)); }, w);
+    cy_compute_sync();
   };
   // column j's rotations (CTA 0's Givens warp)
   auto rotate = [&](int j, double hn, double tol, int max_steps) {

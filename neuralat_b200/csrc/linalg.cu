@@ -3229,9 +3229,9 @@ struct CoShape {
   size_t smem = 0;
 };
 
-// Launch shape of gm_single_kernel: one CTA per SM at most, at least 16 unknowns
-// each (small systems leave SMs to the solves beside them and have a cheaper
-// barrier), the CTA's slice of the whole basis and one vector in shared memory.
+// Launch shape of gm_single_kernel: one CTA per SM at most, a row per warp at the
+// least (fewer gain nothing and leave no SMs to the solves beside them), the
+// CTA's slice of the whole basis and one vector in shared memory.
 struct CyShape {
   int rows = 0, grid = 0;
   size_t smem = 0;
@@ -3244,7 +3244,8 @@ int cycle_shape(int n, int R, CyShape* out) {
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (!coop_ok) return BEM_ERR_UNSUPPORTED;
-  const int rows = std::max(16, (n + sms - 1) / sms);
+  const int rows = std::max(kCyMinRows, (n + sms - 1) / sms);
+  if (rows > kCyMaxRows) return BEM_ERR_UNSUPPORTED;
   const size_t smem = cy_layout(n, rows, R).total;
   if (smem + 1024 > (size_t)smem_optin) return BEM_ERR_UNSUPPORTED;  // 1 KB for the static shared memory
   BEM_CUDA_TRY(cudaFuncSetAttribute(gm_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

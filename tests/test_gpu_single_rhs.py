@@ -1,5 +1,5 @@
-"""One right-hand side in one launch (whole GMRES solve): sizes around the 16
-unknowns of a CTA and the 8 rows of a sweep, odd sizes, restarts, a start
+"""One right-hand side in one launch (whole GMRES solve): sizes around the 15
+unknowns of a CTA and the rows of a sweep, odd sizes, restarts, a start
 vector, the iteration cap, a breakdown (b an eigenvector), zero and non-finite
 right-hand sides; against the FP64 residual of the returned solution and the
 cluster kernel's iteration count.
@@ -36,7 +36,7 @@ def solve(A, b, **kw):
     return x, res, info
 
 
-@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 127, 480, 481, 1000, 2367, 2369, 3001])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 15, 16, 17, 31, 33, 127, 480, 481, 1000, 2220, 2221, 2367, 2369, 3001, 4441, 6661, 7400, 7401])
 def test_sizes(n):
     A, b = system(n)
     for precision in ("fp32", "fp16x3"):
