@@ -202,23 +202,31 @@ __global__ void __launch_bounds__(kLsThreads)
 // its listener's path vertices as rows of a shared-memory tile; every
 // kLsRows rows the CTA multiplies the tile (128 listeners x kLsRows vertices,
 // S and D) with the densities of those vertices, a thread holding 8 listeners
-// x J right-hand sides.  The tile stores Im also negated, and the densities
-// stand twice, as the packed arithmetic takes them.
+// x J right-hand sides.  The densities of a row's vertex are copied
+// asynchronously as soon as the vertex is known and arrive while the CTA walks
+// on.  The tile stores Im also negated, as the packed arithmetic takes it.
 //
 // Bound by the FP32 unit: per path vertex 16 operations per right-hand side
 // and listener, besides the 125 instructions per triangle.  Measured on B200:
-// 4096 listeners x 20 480 triangles x 64 right-hand sides 2.86 ms (one
-// pass), against 21.2 ms with 8 products per quadrature point and right-hand
+// 4096 listeners x 20 480 triangles x 64 right-hand sides 2.47 ms (one
+// pass; FP32 pipe 71 % busy; 2.86 ms with the densities gathered between two
+// barriers), against 21.2 ms with 8 products per quadrature point and right-hand
 // side in four passes.
 constexpr int kLsRows = 16;
 
 template <int J>
 struct ListenSmem {
   float w[kLsRows][6][kLsThreads];  // Re S, Im S, -Im S, Re D, Im D, -Im D
-  float4 dens[kLsRows][2][8 * J];   // (re, re, im, im) of neumann and dirichlet
+  float2 dens[kLsRows][2][8 * J];   // neumann and dirichlet
   TriRec rec[kBlock];
-  int vertex[kLsRows];
 };
+
+// 8-byte asynchronous copy to shared memory; zeros if !in.
+__device__ __forceinline__ void listen_copy(float2* dst, const float2* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 8 : 0)
+               : "memory");
+}
 
 template <int J>
 __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
@@ -262,25 +270,22 @@ __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
           sm.w[rows][3][tid] = dv.x;
           sm.w[rows][4][tid] = dv.y;
           sm.w[rows][5][tid] = -dv.y;
-          if (tid == 0) sm.vertex[rows] = r.v[b];
+          // 16 J densities: thread tid copies column tid of (neumann, dirichlet)
+          for (int e = tid; e < 16 * J; e += kLsThreads) {
+            const int layer = e / (8 * J), c = e - layer * 8 * J;
+            const float2* src = layer ? dir : neu;
+            const bool in = src && rhs0 + c < nrhs;
+            listen_copy(&sm.dens[rows][layer][c], in ? src + (size_t)r.v[b] * nrhs + rhs0 + c : (const float2*)g.rec, in);
+          }
           rows++;
           acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
         }
       }
       const bool last = t == n && c0 + n == t1;
       if (!last && rows + 3 <= kLsRows) continue;  // more records first
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
-      // ---- densities of the rows' vertices, then the product ----
-      for (int e = tid; e < rows * 8 * J; e += kLsThreads) {
-        const int row = e / (8 * J), c = e - row * 8 * J;
-        const size_t at = (size_t)sm.vertex[row] * nrhs + rhs0 + c;
-        const bool in = rhs0 + c < nrhs;
-        const float2 zero = make_float2(0.f, 0.f);
-        const float2 a = neu && in ? neu[at] : zero, u = dir && in ? dir[at] : zero;
-        sm.dens[row][0][c] = make_float4(a.x, a.x, a.y, a.y);
-        sm.dens[row][1][c] = make_float4(u.x, u.x, u.y, u.y);
-      }
-      __syncthreads();
+      // ---- the product ----
 #pragma unroll 1
       for (int row = 0; row < rows; row++) {
 #pragma unroll
@@ -300,8 +305,7 @@ __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
           }
 #pragma unroll
           for (int j = 0; j < J; j++) {
-            const float4 d = sm.dens[row][layer][cg + 8 * j];
-            const float2 dr = make_float2(d.x, d.y), di = make_float2(d.z, d.w);
+            const float2 d = sm.dens[row][layer][cg + 8 * j], dr = f2(d.x), di = f2(d.y);
 #pragma unroll
             for (int l = 0; l < 4; l++) {
               ar[l][j] = f2_fma(ni[l], di, f2_fma(re[l], dr, ar[l][j]));
