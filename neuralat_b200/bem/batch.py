@@ -61,7 +61,7 @@ def assemble_batch(solvers, ks, mass_coeff=0.5, k_coeff=-1.0, stream=None):
     nbytes = int(lib.bem_batch_workspace_bytes(n))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
-        st = ctypes.c_void_p(stream.cuda_stream) if stream is not None else _stream(dev)
+        st = stream.cuda_stream if stream is not None else _stream(dev)
         L.check(lib.bem_batch_matrices_vk(probs, n, float(mass_coeff), float(k_coeff), _vp(ws), nbytes, st),
                 "bem_batch_matrices_vk")
     return outs
@@ -86,7 +86,7 @@ def assemble_batch_bm(solvers, ks, stream=None, approx=True):
     nbytes = int(lib.bem_batch_workspace_bytes(n))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
-        st = ctypes.c_void_p(stream.cuda_stream) if stream is not None else _stream(dev)
+        st = stream.cuda_stream if stream is not None else _stream(dev)
         L.check(lib.bem_batch_matrices_bm(probs, n, _order(approx), _vp(ws), nbytes, st), "bem_batch_matrices_bm")
     return outs
 

@@ -25,6 +25,7 @@ built once per ``BEM_Solver`` and reused by every call.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import math
 
@@ -45,12 +46,22 @@ _LAYERS = {
 _PRECISIONS = {"fp32": L.PREC_FP32, "bf16x3": L.PREC_BF16X3, "bf16": L.PREC_BF16, "fp16x3": L.PREC_FP16X3}
 
 
-def _vp(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _vp(t) -> int:
+    """Device address for a ``void*`` argument (the bindings declare the type)."""
+    return 0 if t is None else t.data_ptr()
 
 
-def _stream(device=None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+def _stream(device=None) -> int:
+    return torch.cuda.current_stream(device).cuda_stream
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """``torch.cuda.device(device)`` where another device is current, else
+    nothing (entering and leaving it takes microseconds of a short call)."""
+    return _HERE if device.index == torch.cuda.current_device() else torch.cuda.device(device)
 
 
 def check_tensor(tensor, dtype):
@@ -68,7 +79,7 @@ class Geometry:
         self.device = vertices.device
         self.nv = int(vertices.shape[0])
         self.nt = int(triangles.shape[0])
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             st = _stream(self.device)
             nbytes = ctypes.c_size_t(0)
             L.check(lib.bem_geometry_bytes(_vp(vertices), self.nv, _vp(triangles), self.nt, ctypes.byref(nbytes), st),
@@ -79,14 +90,14 @@ class Geometry:
 
     @property
     def ptr(self) -> ctypes.c_void_p:
-        return _vp(self.buffer)
+        return ctypes.c_void_p(self.buffer.data_ptr())
 
     def check_status(self) -> None:
         """Raise ``BEMError`` (BEM_ERR_CUDA) if a bounded wait of an assembly
         kernel expired on this geometry since the last check (the matrices
         assembled meanwhile may be wrong); synchronises the current stream."""
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_geometry_status(self.ptr, _stream(self.device)), "assembly on this geometry")
+        with _on(self.device):
+            L.check(L.lib().bem_geometry_status(_vp(self.buffer), _stream(self.device)), "assembly on this geometry")
 
     def __del__(self):
         # the library caches the header per workspace address: forget it
@@ -101,8 +112,8 @@ class Geometry:
     def normals_and_curls(self):
         normals = torch.empty((self.nt, 3), dtype=torch.float32, device=self.device)
         curls = torch.empty((self.nt, 3, 3), dtype=torch.float32, device=self.device)
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_geometry_normals(self.ptr, _vp(normals), _vp(curls), _stream(self.device)),
+        with _on(self.device):
+            L.check(L.lib().bem_geometry_normals(_vp(self.buffer), _vp(normals), _vp(curls), _stream(self.device)),
                     "bem_geometry_normals")
         return normals, curls
 
@@ -120,7 +131,7 @@ def cmatmul(A: torch.Tensor, X: torch.Tensor) -> torch.Tensor:
     Xc = X.contiguous()
     m = 1 if Xc.dim() == 1 else Xc.shape[1]
     Y = torch.empty_like(Xc)
-    with torch.cuda.device(A.device):
+    with _on(A.device):
         L.check(L.lib().bem_cmatmul(_vp(A), n, _vp(Xc), m, _vp(Y), _stream(A.device)), "bem_cmatmul")
     return Y
 
@@ -153,7 +164,7 @@ def gmres(A: torch.Tensor, b: torch.Tensor, x=None, *, rtol=1e-5, atol=0.0, max_
         raise L.BEMError(L.BEM_ERR_INVALID_ARGUMENT, "bem_gmres_workspace_bytes")
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=A.device)
     out = L.SolverInfo()
-    with torch.cuda.device(A.device):
+    with _on(A.device):
         st = lib.bem_gmres_solve(_vp(A), n, _vp(B), m, _vp(X), 0 if x is None else 1, ctypes.byref(p), _vp(ws),
                                  ws_bytes, ctypes.byref(out), _stream(A.device))
     if info is not None:
@@ -217,10 +228,10 @@ class BEM_Solver:
         (False: <4,6>, True: <2,3>, "1" or 1 (beyond the reference's bool): <2,1>)."""
         order = _order(approx)
         out = self._new_matrix()
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_boundary_matrix(self.geometry.ptr, _LAYERS[layer_type], order, float(wavenumber),
-                                                _vp(self.normals), _vp(self.surface_curls_trans), _vp(out),
-                                                _stream(self.device)), f"assemble {layer_type}")
+        with _on(self.device):
+            L.check(L.lib().bem_boundary_matrix(_vp(self.geometry.buffer), _LAYERS[layer_type], order,
+                                                float(wavenumber), _vp(self.normals), _vp(self.surface_curls_trans),
+                                                _vp(out), _stream(self.device)), f"assemble {layer_type}")
         return out
 
     def assemble_vk(self, wavenumber, single=True, lhs=True, *, check=True):
@@ -232,9 +243,9 @@ class BEM_Solver:
         (the solve paths check once after their solver has synchronised)."""
         V = self._new_matrix() if single else None
         A = self._new_matrix() if lhs else None
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_boundary_matrices_vk(self.geometry.ptr, float(wavenumber), _vp(V), _vp(A), 0.5, -1.0,
-                                                     _stream(self.device)), "bem_boundary_matrices_vk")
+        with _on(self.device):
+            L.check(L.lib().bem_boundary_matrices_vk(_vp(self.geometry.buffer), float(wavenumber), _vp(V), _vp(A),
+                                                     0.5, -1.0, _stream(self.device)), "bem_boundary_matrices_vk")
         if check:
             self.geometry.check_status()
         return V, A
@@ -245,17 +256,18 @@ class BEM_Solver:
         <2,3> rules of ``neumann2dirichlet``; False: <4,6>, which is the
         ``HBIE`` system).  ``check`` as in ``assemble_vk``."""
         lhs, rhs = self._new_matrix(), self._new_matrix()
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_boundary_matrices_bm(self.geometry.ptr, _order(approx), float(wavenumber), _vp(lhs),
-                                                     _vp(rhs), _stream(self.device)), "bem_boundary_matrices_bm")
+        with _on(self.device):
+            L.check(L.lib().bem_boundary_matrices_bm(_vp(self.geometry.buffer), _order(approx), float(wavenumber),
+                                                     _vp(lhs), _vp(rhs), _stream(self.device)),
+                    "bem_boundary_matrices_bm")
         if check:
             self.geometry.check_status()
         return lhs, rhs
 
     def identity_matrix(self):
         out = self._new_matrix()
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_identity_matrix(self.geometry.ptr, _vp(out), _stream(self.device)),
+        with _on(self.device):
+            L.check(L.lib().bem_identity_matrix(_vp(self.geometry.buffer), _vp(out), _stream(self.device)),
                     "bem_identity_matrix")
         return out
 
@@ -300,32 +312,41 @@ class BEM_Solver:
         """Explicit (P, N) potential matrix (bind.cu:156-176)."""
         check_tensor(points, torch.float32)
         out = self._new_matrix(rows=points.shape[0])
-        with torch.cuda.device(self.device):
-            L.check(L.lib().bem_potential_matrix(self.geometry.ptr, _LAYERS[layer_type], _vp(points),
+        with _on(self.device):
+            L.check(L.lib().bem_potential_matrix(_vp(self.geometry.buffer), _LAYERS[layer_type], _vp(points),
                                                  int(points.shape[0]), float(k), _vp(out), _stream(self.device)),
                     "bem_potential_matrix")
         return out
 
     def _b2p(self, k, neumann, dirichlet, points):
-        points = points.to(torch.float32).contiguous()
+        if points.dtype is not torch.float32 or not points.is_contiguous():
+            points = points.to(torch.float32).contiguous()
         ref = neumann if neumann is not None else dirichlet
         vec = ref.dim() == 1
-        n = self.geometry.nv
+        n, nt = self.geometry.nv, self.geometry.nt
 
         def prep(u):
-            return None if u is None else u.reshape(n, -1).to(torch.complex64).contiguous()
+            if u is None or (u.dtype is torch.complex64 and u.dim() == 2 and u.shape[0] == n and u.is_contiguous()):
+                return u
+            return u.reshape(n, -1).to(torch.complex64).contiguous()
 
         nu, du = prep(neumann), prep(dirichlet)
         m = (nu if nu is not None else du).shape[1]
         P = int(points.shape[0])
         out = torch.empty((P, m), dtype=torch.complex64, device=self.device)
         lib = L.lib()
-        sb = int(lib.bem_boundary2potential_scratch_bytes(self.geometry.nt, m))
-        scratch = torch.empty(sb, dtype=torch.uint8, device=self.device)
-        with torch.cuda.device(self.device):
-            L.check(lib.bem_boundary2potential(self.geometry.ptr, _vp(points), P, float(k), _vp(nu), _vp(du), m,
-                                               _vp(out), _vp(scratch), sb, _stream(self.device)),
-                    "bem_boundary2potential")
+        with _on(self.device):
+            # without the scratch tensor where the library takes it so (same kernels; 2 us of a 25 us call)
+            if 6 * nt * m <= lib.bem_boundary2potential_noalloc_max():
+                L.check(lib.bem_boundary2potential_noalloc(_vp(self.geometry.buffer), _vp(points), P, float(k), _vp(nu),
+                                                           _vp(du), m, _vp(out), _stream(self.device)),
+                        "bem_boundary2potential")
+            else:
+                sb = int(lib.bem_boundary2potential_scratch_bytes(nt, m))
+                scratch = torch.empty(sb, dtype=torch.uint8, device=self.device)
+                L.check(lib.bem_boundary2potential(_vp(self.geometry.buffer), _vp(points), P, float(k), _vp(nu),
+                                                   _vp(du), m, _vp(out), _vp(scratch), sb, _stream(self.device)),
+                        "bem_boundary2potential")
         return out[:, 0] if vec else out
 
     def single_potential(self, k, neumann, points):
@@ -357,7 +378,7 @@ def map_triangle2vertex(vertices, triangles, features):
     g = Geometry(vertices, triangles)
     out = torch.empty(g.nv, dtype=torch.complex64, device=vertices.device)
     counts = torch.empty(g.nv, dtype=torch.int32, device=vertices.device)
-    with torch.cuda.device(vertices.device):
+    with _on(vertices.device):
         L.check(L.lib().bem_triangle2vertex(g.ptr, _vp(features), _vp(out), _vp(counts), _stream(vertices.device)),
                 "bem_triangle2vertex")
     return out

@@ -329,31 +329,32 @@ int analyse_host(HostGeom& g) {
     for (int i = 0; i < nt; i++)
       for (int a = 0; a < 3; a++) vtri[fill[g.triangles[3 * (size_t)i + a]]++] = i;
   }
-  std::vector<int> seen(nt, -1);
   std::vector<int> nbr(3 * (size_t)nt, -1);  // triangles across an edge (three at most are used)
-  std::vector<int> touch, shared(nt, 0);  // triangles meeting i in the order of its stars, vertices shared with each
+  // triangles meeting i in the order of its stars; 4 i + vertices shared with i
+  std::vector<int> touch;
+  std::vector<long long> shared(nt, -1);
   g.edge_pairs.reserve(3 * (size_t)nt);
   g.vert_pairs.reserve(5 * (size_t)nt);
   g.vert_mirror.reserve(5 * (size_t)nt);
   for (int i = 0; i < nt; i++) {
     const int* ti = &g.triangles[3 * (size_t)i];
     touch.clear();
-    seen[i] = i;
+    const long long tag = 4LL * i;
     for (int a = 0; a < 3; a++)
       for (int p = vptr[ti[a]]; p < vptr[ti[a] + 1]; p++) {
         const int j = vtri[p];
         if (j == i) continue;
-        if (seen[j] != i) {
-          seen[j] = i;
-          shared[j] = 0;
+        if (shared[j] < tag) {
+          shared[j] = tag;
           touch.push_back(j);
         }
         shared[j]++;
       }
     int edges = 0;
     for (int j : touch) {
-      if (shared[j] >= 3) return BEM_ERR_DEGENERATE;  // duplicated triangle
-      if (shared[j] == 2) {
+      const int common = (int)(shared[j] - tag);
+      if (common >= 3) return BEM_ERR_DEGENERATE;  // duplicated triangle
+      if (common == 2) {
         g.edge_pairs.push_back(make_int2(i, j));
         if (edges < 3) nbr[3 * (size_t)i + edges++] = j;
       } else {
@@ -636,9 +637,11 @@ extern "C" int bem_geometry_status(const void* geom, bem_stream_t stream) {
   int err = 0;
   const int zero = 0;
   BEM_CUDA_TRY(cudaMemcpyAsync(&err, v.err, sizeof(int), cudaMemcpyDeviceToHost, s));
+  BEM_CUDA_TRY(cudaStreamSynchronize(s));
+  if (!err) return BEM_OK;
   BEM_CUDA_TRY(cudaMemcpyAsync(v.err, &zero, sizeof(int), cudaMemcpyHostToDevice, s));
   BEM_CUDA_TRY(cudaStreamSynchronize(s));
-  return err ? BEM_ERR_CUDA : BEM_OK;
+  return BEM_ERR_CUDA;
 }
 
 extern "C" int bem_geometry_release(const void* geom) {

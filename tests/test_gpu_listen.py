@@ -56,3 +56,24 @@ def test_listen_edges(solver, points, rhs, which):
         ref = ref + O.potential_matrix("double", v, t, x.astype(np.float64), np.float32(k)) @ u.astype(complex)
     err = np.linalg.norm(got - ref, axis=0) / np.linalg.norm(ref, axis=0)
     assert err.max() < TOL, err.max()
+
+
+@pytest.mark.parametrize("rhs", [440, 441])  # 6 * 397 * 440 <= 2^20 < 6 * 397 * 441: without and with a scratch tensor
+@pytest.mark.parametrize("form", ["plain", "strided", "complex128"])
+def test_scratch_limit_and_forms(solver, rhs, form):
+    import torch
+
+    s, v, t = solver
+    rng = np.random.default_rng(rhs)
+    x = rng.standard_normal((9, 3))
+    x = (0.6 * x / np.linalg.norm(x, axis=1, keepdims=True)).astype(np.float32)
+    u = (rng.standard_normal((len(v), rhs)) + 1j * rng.standard_normal((len(v), rhs))).astype(np.complex64)
+    du, dx = torch.from_numpy(u).cuda(), torch.from_numpy(x).cuda()
+    if form == "strided":
+        du, dx = du.T.contiguous().T, dx.T.contiguous().T
+    if form == "complex128":
+        du, dx = du.to(torch.complex128), dx.double()
+    got = s._b2p(21.0, None, du, dx).cpu().numpy()
+    ref = O.potential_matrix("double", v, t, x.astype(np.float64), np.float32(21.0)) @ u.astype(complex)
+    err = np.linalg.norm(got - ref, axis=0) / np.linalg.norm(ref, axis=0)
+    assert err.max() < TOL, err.max()
