@@ -958,7 +958,7 @@ extern "C" int bem_vertex_gradient(const void* geom, float k, const void* lambda
   const float2* gv = (const float2*)neumann;
   const float2* uv = (const float2*)dirichlet;
   BEM_CUDA_TRY(cudaMemsetAsync(grad, 0, sizeof(double) * 3 * (size_t)g.nv, s));
-  // regular pairs: an equal run of steps for every warp of a persistent grid
+  // regular pairs: equal runs of steps, in rounds over the resident warps
   int dev = 0, sms = 148, occ = 0;
   BEM_CUDA_TRY(cudaGetDevice(&dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -966,7 +966,7 @@ extern "C" int bem_vertex_gradient(const void* geom, float k, const void* lambda
   BEM_CUDA_TRY(cudaFuncSetAttribute(grad_regular_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grad_regular_kernel, kAdjThreads, smem));
   const long long n_steps = strip_steps(g.nblocks), warps = (long long)sms * (occ > 0 ? occ : 1) * kAdjWarps;
-  const long long chunk = std::max(2LL, (n_steps + warps - 1) / warps);
+  const long long chunk = std::max(2LL, strip_part(n_steps, warps, kStripRounds));
   const long long blocks = ((n_steps + chunk - 1) / chunk + kAdjWarps - 1) / kAdjWarps;
   (grad_regular_kernel<<<(unsigned)blocks, kAdjThreads, smem, s>>>(g, k, lam, gv, uv, grad, chunk, n_steps),
    count_launch());

@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kRegThreads, 2)
 // runs on packed pairs (the two points of a trial vertex): the same rounding
 // as scalar operations in fewer issued instructions.
 //
-// Measured on B200 with 20 480 triangles: 13.3 ms (both operators; FP32 pipe
+// Measured on B200 with 20 480 triangles: 12.8 ms (both operators; FP32 pipe
 // 61 % of its cycles, issue 61 %), of which 1.6 ms are the column reductions,
 // against 19.0 ms for 16 x 16-triangle tiles whose 3 x 3 blocks all went
 // through shared memory between block barriers.  Two CTAs of four warps per SM
@@ -331,7 +331,6 @@ constexpr float kTau = (float)(tri6_w_common(0) / tri6_w_own(0));
 __device__ int g_asm_err;
 
 using VkWarp = StripWarp<18, false>;
-constexpr int kVkPanel = 8, kVkPanelItems = 64;  // strip_items
 
 struct VkStrip {
   float k, v_scale, k_scale;
@@ -455,7 +454,8 @@ struct VkStrip {
   }
 };
 
-// One problem, its items dealt round-robin to the warps of a persistent grid.
+// One problem: a warp takes one item (or, past the grid's size, every
+// grid-width-th).
 __global__ void __launch_bounds__(kStripThreads, 2)
     regular_strip_vk_kernel(const __grid_constant__ GeomView g, float k, float2* __restrict__ V, float2* __restrict__ K, float v_scale,
                             float k_scale, StripItems P) {
@@ -884,8 +884,9 @@ int launch_strip_vk(const GeomView& g, float k, float2* V, float2* K, float v_sc
   long long grid = 0;
   int rc = strip_grid(regular_strip_vk_kernel, attr, 0, &grid);
   if (rc) return rc;
-  const StripItems P = strip_items(g.nv, g.nblocks, grid * kStripWarps, 2, g_tune_chunk, kVkPanel, kVkPanelItems);
+  const StripItems P = strip_items(g.nv, g.nblocks, grid * kStripWarps, kStripRounds, 2, g_tune_chunk, 0, 0);
   const long long blocks = (P.items + kStripWarps - 1) / kStripWarps;
+  grid *= kStripRounds;
   (regular_strip_vk_kernel<<<(unsigned)(grid < blocks ? grid : blocks), kStripThreads, kStripWarps * sizeof(VkWarp), s>>>(
        g, k, V, K, v_scale, k_scale, P),
    count_launch());
@@ -1045,7 +1046,7 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
     BatchProblem& P = hp[p];
     P.g = g;
     P.k = ks[p];
-    P.items = strip_items(g.nv, g.nblocks, std::max(1LL, strip_steps(g.nblocks) / share), 4, g_tune_chunk, kVkPanel, kVkPanelItems);
+    P.items = strip_items(g.nv, g.nblocks, std::max(1LL, strip_steps(g.nblocks) / share), 1, 4, g_tune_chunk, 0, 0);
     P.V = Vs[p];
     P.K = Ks[p];
     P.item_begin = items;

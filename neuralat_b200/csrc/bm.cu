@@ -92,8 +92,8 @@ constexpr int kBmPanel = 2, kBmPanelItems = 8;  // strip_items
 // - lhs_ji^T) entry by entry, so it follows from the reduced sums.  Rows of xs:
 // the test points, then the test curls.
 //
-// Measured on B200 at the 3-point rule, the whole assembly: 8286 triangles 1.53
-// ms, 20 480 triangles 8.5 ms, against 2.20 and 12.7 ms for 16 x 16-triangle
+// Measured on B200 at the 3-point rule, the whole assembly: 8286 triangles 1.49
+// ms, 20 480 triangles 8.3 ms, against 2.20 and 12.7 ms for 16 x 16-triangle
 // tiles reduced in shared memory (at 9 point pairs per triangle pair the
 // reduction took over half of the time).  Issue slots and FP32 pipe 58 and 50 %
 // busy; the atomics' DRAM traffic (23 GB at 20 480 triangles with contiguous
@@ -279,8 +279,8 @@ __device__ __forceinline__ int bm_find(const BmProblem* probs, int np, long long
   return lo;
 }
 
-// Regular pairs of one problem: equal work items dealt round-robin to the
-// warps of a persistent grid.
+// Regular pairs of one problem: a warp takes one work item (or, past the grid's
+// size, every grid-width-th).
 template <int TN>
 __global__ void __launch_bounds__(kStripThreads, 2)
     regular_bm_kernel(const __grid_constant__ BmProblem P) {
@@ -645,7 +645,7 @@ template <int TN, int LN>
 int bm_single_launch(const BmProblem& P, long long grid, long long items, cudaStream_t s) {
   const GeomView& g = P.g;
   int rc;
-  if ((rc = bm_regular_launch<TN>(regular_bm_kernel<TN>, grid, items, s, P))) return rc;
+  if ((rc = bm_regular_launch<TN>(regular_bm_kernel<TN>, grid * kStripRounds, items, s, P))) return rc;
   if ((rc = bm_touch_launch<LN>(singular_bm_kernel<double, 3, LN>, g.nt, s, P, g.nt))) return rc;
   if ((rc = bm_touch_launch<LN>(singular_bm_kernel<float, 2, LN>, g.n_edge, s, P, g.n_edge))) return rc;
   return bm_touch_launch<LN>(singular_bm_kernel<float, 1, LN>, g.n_vert, s, P, g.n_vert);
@@ -681,7 +681,7 @@ int assemble_bm(const GeomView& g, int order, float k, float2* L, float2* R, cud
   std::memset(&P, 0, sizeof(P));
   P.g = g;
   P.k = k;
-  P.items = strip_items(g.nv, g.nblocks, grid * kStripWarps, 4, 0, kBmPanel, kBmPanelItems);
+  P.items = strip_items(g.nv, g.nblocks, grid * kStripWarps, 1, 4, 0, kBmPanel, kBmPanelItems);
   P.L = L;
   P.R = R;
   const long long items = P.items.items;
@@ -735,7 +735,8 @@ int assemble_bm_batch(const GeomView* views, const float* ks, float2* const* Ls,
     BmProblem& P = hp[p];
     P.g = g;
     P.k = ks[p];
-    P.items = strip_items(g.nv, g.nblocks, std::max(1LL, strip_steps(g.nblocks) / share), 4, 0, kBmPanel, kBmPanelItems);
+    P.items = strip_items(g.nv, g.nblocks, std::max(1LL, strip_steps(g.nblocks) / share), 1, 4, 0, kBmPanel,
+                          kBmPanelItems);
     P.item_begin = items;
     P.pair_begin[0] = pairs[0];
     P.pair_begin[1] = pairs[1];

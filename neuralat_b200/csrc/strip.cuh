@@ -271,9 +271,9 @@ __device__ __forceinline__ void strip_walk(StripWarp<ROWS, BM>& sw, StripTest& t
 
 // Work items of one problem, in one of two orders.
 //   panel == 0: runs of `chunk` steps, the block pairs taken test block by test
-//     block.  Items as long as an equal share for every warp of the grid have
-//     the fewest column flushes, but the warps then work all over the matrices.
-//   panel > 0: an item is one test block against `panel` trial blocks, panel by
+//     block.  Long items have fewer column flushes, but the warps then work all
+//     over the matrices.
+//   panel > 0 (Burton-Miller): an item is one test block against `panel` trial blocks, panel by
 //     panel: at any time the warps work on a few columns of block pairs (and,
 //     mirrored, rows), whose entries stay in L2 until their neighbours'
 //     contributions have arrived.
@@ -288,7 +288,7 @@ __device__ __forceinline__ void strip_item(StripWarp<ROWS, BM>& sw, StripTest& t
                                            const StripItems& P, long long item, unsigned& uses, int* process_err) {
   const int nb = g.nblocks;
   int grp, jb, t0 = 0, steps;
-  if (P.panel == 0) {
+  if (!BM || P.panel == 0) {
     const long long pos = item * P.chunk, unit = pos >> 5;
     grp = tile_group_of(unit, nb);
     jb = grp + (int)(unit - tile_units_before(grp, nb));
@@ -311,23 +311,41 @@ __device__ __forceinline__ void strip_item(StripWarp<ROWS, BM>& sw, StripTest& t
 // Steps of a problem's walk.
 inline long long strip_steps(int nblocks) { return 32LL * nblocks * (nblocks + 1) / 2; }
 
-// The items for a grid of `warps` warps, at least `least` steps each; `blocks`
-// trial blocks per item if that is not 0 (tuning).  Panels of `panel` blocks
-// are taken where the two matrices exceed the L2 cache by far (64 MB) and every
-// warp gets `panel_items` of them, so that the uneven last round is small.
-// Measured on B200, contiguous items against panels: Burton-Miller at the
-// 3-point rule (a pair takes a third of the V/K pair's time, so that its
-// atomics weigh more), panels of 2, 20 480 triangles 11.8 and 8.5 ms, 8286
-// triangles 1.75 and 1.53 ms, 5120 triangles 0.66 and 0.68 ms; V and K, panels
-// of 8, 81 920 triangles 225 and 220 ms, 20 480 triangles 14.57 and 14.87 ms
-// (loading a test block per item, uneven last round).
-inline StripItems strip_items(int nv, int nblocks, long long warps, long long least, int blocks, int panel,
-                              int panel_items) {
+// Equal items go in `rounds` rounds over the warps that are resident, a CTA per
+// four items, handed out in order: an SM that is ahead takes more of them, and
+// what runs at one time writes neighbouring rows.  One item per warp left 10 %
+// of the warp slots empty at the end.  Measured on B200, one round against many
+// of at least 64 steps: V and K 20 480 triangles 14.1 and 13.5 ms, 8286
+// triangles 2.63 and 2.48 ms, 5120 triangles 1.06 and 1.05 ms (16 steps 1.11);
+// the Burton-Miller pair's panels 8.48 and 8.28 ms, with 6-point rules 20.2 and
+// 18.6 ms.
+constexpr int kStripRounds = 32, kStripRoundSteps = 64;
+
+// Steps of an item, at most `most` rounds.
+inline long long strip_part(long long steps, long long warps, int most) {
+  long long rounds = steps / (warps * kStripRoundSteps);
+  rounds = rounds < 1 ? 1 : (rounds < most ? rounds : most);
+  return (steps + warps * rounds - 1) / (warps * rounds);
+}
+
+// The items for `warps` resident warps, at least `least` steps each; `blocks`
+// trial blocks per item if that is not 0 (tuning).  Panels of `panel` blocks (0:
+// never) are taken where the two matrices exceed the L2 cache by far (64 MB)
+// and every warp gets `panel_items` of them, so that the uneven last round is
+// small.  Measured on B200 for the Burton-Miller pair (at the 3-point rule a
+// pair takes a third of the V/K pair's time, so that its atomics weigh more),
+// contiguous items in one round against panels of 2: 20 480 triangles 11.8 and
+// 8.5 ms, 8286 triangles 1.75 and 1.53 ms, 5120 triangles 0.66 and 0.68 ms.
+// Against contiguous items in rounds, panels gain 2 % with the 6-point rules.  V
+// and K take none: 81 920 triangles 206.4 ms in rounds, 207.0 ms in panels of 8.
+inline StripItems strip_items(int nv, int nblocks, long long warps, int rounds, long long least, int blocks,
+                              int panel, int panel_items) {
   StripItems P;
   P.steps = strip_steps(nblocks);
   const long long share = (P.steps + warps - 1) / warps;
   P.panel = blocks == 0 && 16.0 * nv * nv > 64e6 && share >= 32LL * panel * panel_items ? panel : 0;
-  const long long chunk = blocks > 0 ? 32LL * blocks : (share > least ? share : least);
+  const long long part = strip_part(P.steps, warps, rounds);
+  const long long chunk = blocks > 0 ? 32LL * blocks : (part > least ? part : least);
   P.chunk = (int)(chunk < (1 << 30) ? chunk : (1 << 30));
   if (P.panel) {
     const long long panels = (nblocks + P.panel - 1) / P.panel;

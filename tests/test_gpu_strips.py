@@ -79,3 +79,31 @@ def test_block_edges(name):
     for layer in ("hypersingular", "bm_lhs"):  # the sorted records' curls in the general kernel
         got = s.assemble_boundary_matrix(k, layer, approx=True).cpu().numpy()
         assert rel(got, O.boundary_matrix(layer, v64, t, k, "_approx")) < TOL
+
+
+def sheet(count):
+    """The first `count` triangles of a long bumpy sheet."""
+    n, m = 60, 56
+    i, j = np.meshgrid(np.arange(n), np.arange(m), indexing="ij")
+    v = np.stack([0.01 * i, 0.01 * j, 0.01 * np.sin(0.3 * i + 0.2 * j)], -1).reshape(-1, 3)
+    a = (np.arange(n - 1)[:, None] * m + np.arange(m - 1)).reshape(-1)
+    t = np.stack([a, a + m, a + 1, a + 1, a + m, a + m + 1], 1).reshape(-1, 3)[:count]
+    used, t = np.unique(t, return_inverse=True)
+    return v[used], t.reshape(-1, 3)
+
+
+@pytest.mark.parametrize("count", [3072, 3073, 4321, 6300])
+def test_rounds(count):
+    """Items in one round, in two (97 blocks) and more, and the Burton-Miller
+    panels with an uneven last one: one problem against the queue's items.
+    Tolerance: both within 1e-5 of the exact matrices, so within 2e-5."""
+    from neuralat_b200.bem import BEM_Solver
+    from neuralat_b200.bem.batch import assemble_batch, assemble_batch_bm
+
+    v, t = sheet(count)
+    s, k = BEM_Solver(v.astype(np.float32), t.astype(np.int32)), 17.0
+    pairs = [(s.assemble_vk(k), assemble_batch([s], [k])[0])]
+    pairs += [(s.assemble_bm(k, approx=a), assemble_batch_bm([s], [k], approx=a)[0]) for a in (True, False)]
+    for one, many in pairs:
+        for x, y in zip(one, many):
+            assert float((x - y).norm() / y.norm()) < 2 * TOL
