@@ -31,6 +31,7 @@
 
 #include "async_copy.cuh"
 #include "bem_common.cuh"
+#include "cgemm.cuh"
 
 namespace bemb {
 
@@ -3452,6 +3453,7 @@ int launch_block(const GmPtrs& P, const BkPtrs& K, const BkShape& sh, int group,
 
 int cmatmul(const float2* A, int n, const float2* X, int m, float2* Y, cudaStream_t s) {
   BEM_CUDA_TRY(cudaMemsetAsync(Y, 0, sizeof(float2) * (size_t)n * m, s));
+  if (m > kCgSides && n > kCgLeast) return launch_cgemm(A, n, X, m, Y, device_sms(), s);
   return launch_cgemv(A, n, X, m, Y, nullptr, s);
 }
 
