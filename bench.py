@@ -564,16 +564,17 @@ def run_ours(args):
     clocks = clk.summary()
     peak = fp32_peak_tflops(clocks.get("sm_max_mhz"))
     achieved = F_VK * n_eval / (asm_ms / 1e3) / 1e12
-    # DRAM traffic of regular_sym_kernel: 167.4 MB per launch measured by ncu at
-    # icosphere s4 (N = 2562: the atomic read-modify-write of the two output
-    # matrices), scaled by the units processed, (10242 / 2562)^2, to this mesh
-    traffic = 167.4e6 * (v.shape[0] / 2562.0) ** 2
+    # DRAM traffic of regular_strip_vk_kernel: 9.43 GB per launch measured by ncu
+    # at icosphere s5 (N = 10 242: the atomic read-modify-write of the two output
+    # matrices), scaled by the units processed to this mesh
+    traffic = 9.43e9 * (v.shape[0] / 10242.0) ** 2
     roofline = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": traffic,
-                "kernel": "bem_boundary_matrices_vk (regular_sym_kernel + singular + memset, timed as one stage), "
+                "kernel": "bem_boundary_matrices_vk (regular_strip_vk_kernel + touching + memset, timed as one stage), "
                           f"63 flop x {n_eval:.4e} ordered regular quadrature-point pairs per launch (the kernel "
-                          "evaluates each unordered pair once); peak = nominal FP32 (SMs x 128 FMA x 2 x max SM "
-                          "clock; no measured FP32 peak available); traffic scaled from an s4 ncu capture"}
+                          "evaluates each unordered pair once, and the rule's symmetry takes it fewer operations "
+                          "than these); peak = nominal FP32 (SMs x 128 FMA x 2 x max SM "
+                          "clock; no measured FP32 peak available); traffic scaled from an s5 ncu capture"}
 
     # ---- roofline of the solve's dominant kernel (tensor-core matvec) ----------
     roofline_matvec = None

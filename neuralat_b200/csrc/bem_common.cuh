@@ -195,9 +195,9 @@ struct GeomView {
   int* err;                // the header's status word (GeomHeader::err)
 };
 
-// Symmetric regular-pair work units (test tile g, trial tile jt >= g) in
-// order: test tile g owns the ntiles - g trial tiles from itself on, so
-// U(g) = g ntiles - g (g - 1) / 2 units come before it.
+// Symmetric regular-pair work units (test block g, trial block j >= g) in
+// order: test block g owns the n - g trial blocks from itself on, so
+// U(g) = g n - g (g - 1) / 2 units come before it.
 __device__ __forceinline__ long long tile_units_before(long long g, long long n) { return g * n - g * (g - 1) / 2; }
 
 __device__ __forceinline__ int tile_group_of(long long pos, int n) {
