@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/bem_b200.h"
 
 namespace bemb {
@@ -333,3 +335,27 @@ unsigned long long launch_count();
     cudaError_t _e = (expr);                        \
     if (_e != cudaSuccess) return BEM_ERR_CUDA;     \
   } while (0)
+
+namespace bemb {
+// Set-up of a kernel once on each device (one static object per kernel).  The
+// limit of a kernel's dynamic shared memory belongs to the kernel on the current
+// device and to all host threads: it is set once, to the largest size that any
+// launch asks for, since a thread that set its own call's size could lower it
+// between another thread's call and that call's launch.
+class DeviceOnce {
+ public:
+  template <typename F>
+  int operator()(F&& set) {
+    int dev = 0;
+    BEM_CUDA_TRY(cudaGetDevice(&dev));
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;  // beyond: each time
+    if (done_.load(std::memory_order_acquire) & bit) return BEM_OK;
+    const int rc = set();
+    if (rc == BEM_OK) done_.fetch_or(bit, std::memory_order_release);
+    return rc;
+  }
+
+ private:
+  std::atomic<unsigned long long> done_{0};
+};
+}  // namespace bemb

@@ -3257,7 +3257,13 @@ int cycle_shape(int n, int R, CyShape* out) {
   if (rows > kCyMaxRows) return BEM_ERR_UNSUPPORTED;
   const size_t smem = cy_layout(n, rows, R).total;
   if (smem + 1024 > (size_t)smem_optin) return BEM_ERR_UNSUPPORTED;  // 1 KB for the static shared memory
-  BEM_CUDA_TRY(cudaFuncSetAttribute(gm_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static DeviceOnce once;
+  const int rc = once([&]() -> int {
+    BEM_CUDA_TRY(
+        cudaFuncSetAttribute(gm_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
+    return BEM_OK;
+  });
+  if (rc) return rc;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gm_single_kernel, kCyThreads, smem));
   out->rows = rows;
