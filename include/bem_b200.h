@@ -271,7 +271,9 @@ int bem_boundary2potential_adjoint(const void* geom, const float* points, int np
                                    void* out_s, void* out_d, bem_stream_t stream);
 /* grad (nv x 3 float64, overwritten) = d/dx Re[ -pbar^H S g + pbar^H D u
  *   - lambda^H V g - 1/2 lambda^H M u + lambda^H K u ] with the vectors held
- * fixed (lambda, g = neumann, u = dirichlet: nv complex64; pbar: np). */
+ * fixed (lambda, g = neumann, u = dirichlet: nv complex64; pbar: np).  Its
+ * kernel has bounded waits, as the assembly kernels have: read
+ * bem_geometry_status before the gradient is used. */
 int bem_vertex_gradient(const void* geom, float k, const void* lambda, const void* neumann, const void* dirichlet,
                         const float* points, int np, const void* pbar, double* grad, bem_stream_t stream);
 

@@ -83,6 +83,7 @@ class _ListenerPressure(torch.autograd.Function):
                 L.check(lib.bem_vertex_gradient(s.geometry.ptr, float(k), _vp(lam), _vp(ctx.g), _vp(ctx.u), _vp(pts),
                                                 int(pts.shape[0]), _vp(pbar), _vp(gx), _stream(pbar.device)),
                         "bem_vertex_gradient")
+            s.geometry.check_status()  # a wait of its kernels that expired: the gradient may be wrong
             grad_x = gx.to(torch.float32)
         return grad_x, grad_g, None, None, None, None, None, None
 
