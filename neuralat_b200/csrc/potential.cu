@@ -14,6 +14,8 @@
 // right-hand sides, once per path vertex (1.15 per triangle) instead of once
 // per quadrature point (6 per triangle).
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 
@@ -126,8 +128,9 @@ constexpr int kLsChunk = 16;  // triangles staged per warp
 // out[p, s] += -S neumann + D dirichlet over the triangles of one run
 // (blockIdx.y) for 32 listeners, up to M <= 4 right-hand sides: the products
 // with the vertex densities stay in the listener's own registers.  Each warp
-// walks a quarter of the run; their sums meet in shared memory, so that few
-// FP32 terms are added to an output one after the other.
+// walks a quarter of the run; their sums meet in shared memory and those of a
+// cluster's runs in its first CTA, so that few FP32 terms are added to an output
+// one after the other.
 //
 // Bound by the FP32 and sincos units (about 125 instructions for the 6 points
 // of a triangle).  Measured on B200: 1000 listeners x 5110 triangles x 1
@@ -137,7 +140,7 @@ constexpr int kLsChunk = 16;  // triangles staged per warp
 template <int M>
 __global__ void __launch_bounds__(kLsThreads)
     listen_few_kernel(GeomView g, const float* __restrict__ pts, int np, float k, const float2* __restrict__ neu,
-                      const float2* __restrict__ dir, int nrhs, int run, float2* __restrict__ out) {
+                      const float2* __restrict__ dir, int nrhs, float2* __restrict__ out, int run) {
   __shared__ TriRec rec_s[kLsWarps][kLsChunk];
   __shared__ float4 dens_s[kLsWarps][kLsChunk][3][M];  // (neumann, dirichlet) at the triangle's vertices
   __shared__ float2 sum_s[kLsWarps][M][32];
@@ -187,15 +190,33 @@ __global__ void __launch_bounds__(kLsThreads)
 #pragma unroll
   for (int s = 0; s < M; s++) sum_s[warp][s][lane] = sum[s];
   __syncthreads();
-  if (warp == 0 && p < np) {
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  if (cluster.num_blocks() == 1) {
+    if (warp == 0 && p < np) {
 #pragma unroll
-    for (int s = 0; s < M; s++) {
-      float2 t = sum_s[0][s][lane];
+      for (int s = 0; s < M; s++) {
+        float2 t = sum_s[0][s][lane];
 #pragma unroll
-      for (int w = 1; w < kLsWarps; w++) t = f2_add(t, sum_s[w][s][lane]);
-      if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], t);
+        for (int w = 1; w < kLsWarps; w++) t = f2_add(t, sum_s[w][s][lane]);
+        if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], t);
+      }
     }
+    return;
   }
+  for (int s = warp; s < M; s += kLsWarps) {  // right-hand side s of listener `lane`
+    float2 t = sum_s[0][s][lane];
+#pragma unroll
+    for (int w = 1; w < kLsWarps; w++) t = f2_add(t, sum_s[w][s][lane]);
+    sum_s[0][s][lane] = t;
+  }
+  cluster.sync();  // every CTA's sums are complete
+  if (cluster.block_rank() == 0 && p < np)
+    for (int s = warp; s < M && s < nrhs; s += kLsWarps) {
+      float2 t = sum_s[0][s][lane];
+      for (unsigned r = 1; r < cluster.num_blocks(); r++) t = f2_add(t, *cluster.map_shared_rank(&sum_s[0][s][lane], r));
+      atomicAdd(&out[(size_t)p * nrhs + s], t);
+    }
+  cluster.sync();  // the sums have been read
 }
 
 // The same for 8 J right-hand sides at a time (from rhs0 on): a thread writes
@@ -206,19 +227,29 @@ __global__ void __launch_bounds__(kLsThreads)
 // asynchronously as soon as the vertex is known and arrive while the CTA walks
 // on.  The tile stores Im also negated, as the packed arithmetic takes it.
 //
+// A product is four FMAs into one FP32 sum per row; after kLsChain rows or more
+// the sums move on to second ones in shared memory (16 bytes per two outputs
+// and thread, 4 J of them).  In one chain over the whole run, neighbouring
+// vertices' like terms cost up to 2.9 times the error (33 right-hand sides, 4000
+// listeners, 9800 triangles at 500 Hz: 8.0e-7 off 64 bits, 2.7e-7 so; one
+// quadrature point after the other, in eight warps: 2.8e-7).  10 rows instead
+// of 16 leave room for the second sums beside two CTAs per SM.
+//
 // Bound by the FP32 unit: per path vertex 16 operations per right-hand side
 // and listener, besides the 125 instructions per triangle.  Measured on B200:
-// 4096 listeners x 20 480 triangles x 64 right-hand sides 2.47 ms (one
-// pass; FP32 pipe 71 % busy; 2.86 ms with the densities gathered between two
-// barriers), against 21.2 ms with 8 products per quadrature point and right-hand
-// side in four passes.
-constexpr int kLsRows = 16;
+// 4096 listeners x 20 480 triangles x 64 right-hand sides 2.58 ms in one pass
+// (2.47 ms in one chain per run, 2.81 ms moving on after 8 rows, 3.22 ms with 16
+// rows and one CTA per SM), against 21.1 ms with 8 products per quadrature point
+// and right-hand side in four passes.
+constexpr int kLsRows = 10;
+constexpr int kLsChain = 16;
 
 template <int J>
 struct ListenSmem {
   float w[kLsRows][6][kLsThreads];  // Re S, Im S, -Im S, Re D, Im D, -Im D
   float2 dens[kLsRows][2][8 * J];   // neumann and dirichlet
   TriRec rec[kBlock];
+  float4 sum[4 * J][kLsThreads];    // (re, im) of a thread's listener pair l and right-hand side j at l J + j
 };
 
 // 8-byte asynchronous copy to shared memory; zeros if !in.
@@ -231,7 +262,7 @@ __device__ __forceinline__ void listen_copy(float2* dst, const float2* src, bool
 template <int J>
 __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
     listen_many_kernel(GeomView g, const float* __restrict__ pts, int np, float k, const float2* __restrict__ neu,
-                       const float2* __restrict__ dir, int nrhs, int rhs0, int run, float2* __restrict__ out) {
+                       const float2* __restrict__ dir, int nrhs, int rhs0, float2* __restrict__ out, int run) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ListenSmem<J>& sm = *reinterpret_cast<ListenSmem<J>*>(smem_raw);
   const int tid = threadIdx.x;
@@ -247,7 +278,28 @@ __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
   ListenSums acc;
 #pragma unroll
   for (int b = 0; b < 3; b++) acc.s[b] = acc.d[b] = make_float2(0.f, 0.f);
-  int rows = 0;
+  // the products so far move on to the thread's own sums
+  bool first = true;
+  auto fold = [&]() {
+#pragma unroll
+    for (int l = 0; l < 4; l++)
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        float4& t = sm.sum[l * J + j][tid];
+        float4 v = make_float4(ar[l][j].x, ai[l][j].x, ar[l][j].y, ai[l][j].y);
+        if (!first) {
+          const float4 old = t;
+          v.x += old.x;
+          v.y += old.y;
+          v.z += old.z;
+          v.w += old.w;
+        }
+        t = v;
+        ar[l][j] = ai[l][j] = make_float2(0.f, 0.f);
+      }
+    first = false;
+  };
+  int rows = 0, chain = 0;
   for (int c0 = t0; c0 < t1; c0 += kBlock) {
     const int n = min(kBlock, t1 - c0);
     __syncthreads();  // everyone is done with the previous records
@@ -314,23 +366,47 @@ __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
           }
         }
       }
+      chain += rows;
       rows = 0;
+      if (chain >= kLsChain) {
+        fold();
+        chain = 0;
+      }
       __syncthreads();  // the tile may be overwritten
     }
   }
+  const int p = blockIdx.x * kLsThreads + 4 * lg;
+  auto add_out = [&](int l, int j, const float4& t) {
+    const int at = p + 64 * (l >> 1) + 2 * (l & 1), s = rhs0 + cg + 8 * j;
+    if (s >= nrhs) return;
+    if (at < np) atomicAdd(&out[(size_t)at * nrhs + s], make_float2(-t.x, -t.y));
+    if (at + 1 < np) atomicAdd(&out[(size_t)(at + 1) * nrhs + s], make_float2(-t.z, -t.w));
+  };
+  fold();
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int ctas = (int)cluster.num_blocks();
+  if (ctas == 1) {
 #pragma unroll
-  for (int l = 0; l < 4; l++)
+    for (int l = 0; l < 4; l++)
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int p = blockIdx.x * kLsThreads + 4 * lg + 64 * (l >> 1) + 2 * (l & 1) + i;
-      if (p >= np) continue;
-#pragma unroll
-      for (int j = 0; j < J; j++) {
-        const int s = rhs0 + cg + 8 * j;
-        const float re = i ? ar[l][j].y : ar[l][j].x, im = i ? ai[l][j].y : ai[l][j].x;
-        if (s < nrhs) atomicAdd(&out[(size_t)p * nrhs + s], make_float2(-re, -im));
-      }
+      for (int j = 0; j < J; j++) add_out(l, j, sm.sum[l * J + j][tid]);
+    return;
+  }
+  // the cluster's sums, an equal part of them per CTA
+  cluster.sync();  // every CTA's sums are complete
+  const int mine = 4 * J / ctas, q0 = (int)cluster.block_rank() * mine;
+  for (int q = q0; q < q0 + mine; q++) {
+    float4 t = *cluster.map_shared_rank(&sm.sum[q][tid], 0);
+    for (int r = 1; r < ctas; r++) {
+      const float4 v = *cluster.map_shared_rank(&sm.sum[q][tid], r);
+      t.x += v.x;
+      t.y += v.y;
+      t.z += v.z;
+      t.w += v.w;
     }
+    add_out(q / J, q % J, t);
+  }
+  cluster.sync();  // the sums have been read
 }
 
 __global__ void t2v_scatter_kernel(GeomView g, const float2* __restrict__ tv, float2* __restrict__ out,
@@ -386,48 +462,97 @@ extern "C" size_t bem_boundary2potential_scratch_bytes(int nt, int nrhs) {
 
 namespace bemb {
 namespace {
-// Triangles per CTA so that the grid is a little below a whole number of
-// waves of `slots` CTAs: as few waves as leave at most a tenth of the last one
-// empty, and runs of at least `least` triangles (each run loads its densities
-// and adds its sums to the output) and of at most 800 or so: longer serial
-// FP32 sums cost accuracy (20 480 triangles: 2.7e-6 off the FP64 pressures
-// with 9 runs, 2.3e-6 with 27; 2.1e-6 before).
-int listen_run(int groups, int nt, long long slots, int least) {
+// Runs of triangles: so many that the grid is a little below a whole number of
+// waves of `slots` CTAs (as few waves as leave at most a tenth of the last one
+// empty), of at least `least` triangles (each run loads its densities and adds
+// its sums) and of at most 400, so that a listener's sums stay short (above,
+// nothing is gained: 4096 listeners x 64 on 20 480 triangles 2.6 ms, with runs
+// of 800 2.68 ms).
+//
+// An output takes one FP32 addition per run.  Where these are more than 64, the
+// runs of a cluster (`most` CTAs at the most) are added up first, and there are
+// no more than 512 runs while that leaves at most 400 triangles in each: 20
+// listeners, one right-hand side, 20 480 triangles at 200 Hz 6.4e-7 -> 2.2e-7 off
+// 64 bits, in the same time.  Where they are fewer, a cluster gains nothing and
+// costs 2 us of a 46 us call.
+struct ListenRuns {
+  int run, parts, cluster;
+};
+
+ListenRuns listen_runs(int groups, int nt, long long slots, int least, int most) {
   long long splits = 1;
   for (int waves = 1; waves <= 64; waves++) {
     splits = std::max<long long>(1, waves * slots / groups);
-    if (10 * splits * groups >= 9 * waves * slots && nt <= 800 * splits) break;
+    if (10 * splits * groups >= 9 * waves * slots && nt <= 400 * splits) break;
   }
-  splits = std::min<long long>(splits, 65535);
-  return (int)std::max<long long>(least, (nt + splits - 1) / splits);
+  splits = std::min<long long>(splits, std::min(std::max(512, nt / 400), 65528));
+  ListenRuns r;
+  r.run = (int)std::max<long long>(least, (nt + splits - 1) / splits);
+  r.parts = (nt + r.run - 1) / r.run;
+  r.cluster = 1;
+  while (r.cluster < most && r.parts > 64 * r.cluster) r.cluster *= 2;
+  return r;
+}
+
+// Launch of a listener kernel with its runs as clusters along y; per_sm: CTAs
+// that an SM holds; clusters: how many clusters of 2, 4 and 8 the GPU holds (0:
+// not known yet).
+template <typename Kernel, typename... Args>
+int listen_launch(Kernel kernel, int groups, int nt, int sms, int per_sm, int least, int most, size_t smem,
+                  cudaStream_t s, std::atomic<int>* clusters, Args... args) {
+  ListenRuns r = listen_runs(groups, nt, (long long)per_sm * sms, least, most);
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kLsThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 1;
+  at[0].val.clusterDim.y = (unsigned)r.cluster;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = r.cluster > 1 ? 1 : 0;
+  if (r.cluster > 1) {  // fewer CTAs fit as clusters
+    std::atomic<int>& known = clusters[r.cluster == 2 ? 0 : (r.cluster == 4 ? 1 : 2)];
+    int n = known.load(std::memory_order_relaxed);
+    if (n == 0) {
+      cfg.gridDim = dim3(1, (unsigned)r.cluster, 1);
+      BEM_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
+      if (n < 1) return BEM_ERR_CUDA;
+      known.store(n, std::memory_order_relaxed);
+    }
+    const int c = r.cluster;
+    r = listen_runs(groups, nt, (long long)n * c, least, most);
+    r.cluster = c;
+    r.parts = (r.parts + c - 1) / c * c;  // the last runs may be empty
+  }
+  cfg.gridDim = dim3((unsigned)groups, (unsigned)r.parts, 1);
+  BEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args..., r.run));
+  count_launch();
+  return BEM_OK;
 }
 
 template <int M>
-void listen_few(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
-                float2* out, int sms, cudaStream_t s) {
-  const int groups = (np + 31) / 32;
-  const int run = listen_run(groups, g.nt, 8LL * sms, 16);
-  (listen_few_kernel<M><<<dim3(groups, (g.nt + run - 1) / run), kLsThreads, 0, s>>>(g, pts, np, k, neu, dir, nrhs, run,
-                                                                                 out),
-   count_launch());
+int listen_few(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
+               float2* out, int sms, cudaStream_t s) {
+  static std::atomic<int> clusters[3];
+  return listen_launch(listen_few_kernel<M>, (np + 31) / 32, g.nt, sms, 8, 16, 8, 0, s, clusters, g, pts, np, k, neu, dir,
+                       nrhs, out);
 }
 
 template <int J>
 int listen_many(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
                 int rhs0, float2* out, int dev, int sms, cudaStream_t s) {
   const int smem = (int)sizeof(ListenSmem<J>);
+  static std::atomic<int> clusters[3];
   static std::atomic<unsigned long long> attr{0};  // devices whose attribute is set
   const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
   if (!(attr.load(std::memory_order_acquire) & bit)) {
     BEM_CUDA_TRY(cudaFuncSetAttribute(listen_many_kernel<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr.fetch_or(bit, std::memory_order_release);
   }
-  const int groups = (np + kLsThreads - 1) / kLsThreads;
-  const int run = listen_run(groups, g.nt, (J == 8 ? 2LL : 3LL) * sms, 12);
-  (listen_many_kernel<J><<<dim3(groups, (g.nt + run - 1) / run), kLsThreads, smem, s>>>(g, pts, np, k, neu, dir, nrhs,
-                                                                                     rhs0, run, out),
-   count_launch());
-  return BEM_OK;
+  return listen_launch(listen_many_kernel<J>, (np + kLsThreads - 1) / kLsThreads, g.nt, sms, J == 8 ? 2 : 3, 12, 4,
+                       (size_t)smem, s, clusters, g, pts, np, k, neu, dir, nrhs, rhs0, out);
 }
 }  // namespace
 
@@ -444,12 +569,10 @@ int b2p_enqueue(const GeomView& g, const float* points, int np, float k, const v
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (nrhs <= 4) {
-    if (nrhs == 1)
-      listen_few<1>(g, points, np, k, neu, dir, nrhs, o, sms, s);
-    else if (nrhs == 2)
-      listen_few<2>(g, points, np, k, neu, dir, nrhs, o, sms, s);
-    else
-      listen_few<4>(g, points, np, k, neu, dir, nrhs, o, sms, s);
+    const int rc = nrhs == 1   ? listen_few<1>(g, points, np, k, neu, dir, nrhs, o, sms, s)
+                   : nrhs == 2 ? listen_few<2>(g, points, np, k, neu, dir, nrhs, o, sms, s)
+                               : listen_few<4>(g, points, np, k, neu, dir, nrhs, o, sms, s);
+    if (rc) return rc;
   } else {
     for (int r0 = 0; r0 < nrhs; r0 += 64) {
       const int left = nrhs - r0;
