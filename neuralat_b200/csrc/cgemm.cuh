@@ -1,27 +1,31 @@
-// Complex product Y += A X with more than eight right-hand sides (FP32).
+// Complex product Y += A X with more than eight right-hand sides (FP32), above
+// 8192 unknowns.
 //
-// A tile of 64 rows x 64 (64 x 32, 128 x 16) right-hand sides per CTA and 16
-// columns of A and rows of X per stage of a shared-memory ring filled by
-// cp.async.  A thread owns 4 rows x 4 right-hand sides; a column costs its warp
-// four shared-memory wavefronts and 32 packed FMAs a lane, so the FP32 pipe is
-// the bound (against eight right-hand sides at a time, with X read from shared
-// memory for 4 rows only, and A once per eight).  Measured on B200, 64
-// right-hand sides: 40 962 unknowns 35.9 -> 17.4 ms (49 TFLOP/s of 74), 10 242
-// unknowns 1.80 -> 1.12 ms, 2562 unknowns 118 -> 87 us; 16 right-hand sides:
-// 40 962 unknowns 7.26 -> 4.57 ms (0.45 of the bandwidth, 0.63 of the FP32 rate).
+// A tile of 64 rows x 64 (128 x 16) right-hand sides per CTA and 16 columns of A
+// and rows of X per stage of a shared-memory ring filled by cp.async.  A thread
+// owns 4 rows x 4 right-hand sides; a column costs its warp four shared-memory
+// wavefronts and 32 packed FMAs a lane, so the FP32 pipe is the bound (against
+// eight right-hand sides at a time, with X read from shared memory for 4 rows
+// only, and A once per eight).  Measured on B200: 40 962 unknowns, 64 right-hand
+// sides 35.6 -> 18.2 ms (47 TFLOP/s of 74), 48: 21.6 -> 15.6 ms, 16: 7.2 -> 4.9
+// ms; 10 242 unknowns, 64: 1.82 -> 1.23 ms, 24: 0.71 -> 0.61 ms, 16: 0.43 -> 0.32
+// ms.
 //
-// Sums: re(a) x and im(a) x over 32 columns each, these over the CTA's columns
-// (up to 1024, spread over the matrix so that a smooth integrand's oscillations
-// cancel within the sums), these by one atomic per CTA.  Error against 64 bits
-// on random entries, 64 right-hand sides: 1.93e-7 (lane sums over 1024 columns
-// added by atomics: 1.96e-7) for 40 962 unknowns, 1.36e-7 (1.53e-7) for 2562.
-// Below kCgLeast unknowns those lane sums have under 16 columns and the smaller
-// error, and both kernels take less time than their launch.
+// Sums: re(a) x and im(a) x over 16 columns each, these over 128 columns in
+// registers, these over the CTA's columns (up to 1024, spread over the matrix so
+// that a smooth integrand's oscillations cancel within the sums) in shared
+// memory, these over the CTAs of a cluster in FP64 and rounded once, and one
+// atomic per cluster, no more of them than with lane sums over 1024 columns.
+// Against 64 bits, 10 242 unknowns and smooth fields, those lane sums and this:
+// double layer 1.1e-7 and 0.9e-7, single layer 8.3e-8 and 6.6 to 7.4e-8 (with 32
+// columns, the CTA's columns in one chain and one atomic per CTA 1.2e-7 and
+// 9.1e-8).
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <atomic>
-#include <cmath>
 
 #include "async_copy.cuh"
 #include "bem_common.cuh"
@@ -29,12 +33,10 @@
 namespace bemb {
 namespace {
 
-constexpr int kCgLeast = 512;  // unknowns, and
-constexpr int kCgSides = 8;    // right-hand sides above which it is used
 constexpr int kCgCols = 16;    // columns of A per stage
-constexpr int kCgRun = 32;     // columns per first-level sum
+constexpr int kCgFar = 128;    // columns per second-level sum
 constexpr int kCgPitch = kCgCols * 8 + 16;  // bytes between A rows: 8 rows start in distinct bank groups
-static_assert(kCgRun % kCgCols == 0 && kCgCols % 2 == 0, "");
+static_assert(kCgFar % kCgCols == 0 && kCgCols % 2 == 0, "");
 
 template <int TM>
 struct CgShape {
@@ -43,7 +45,8 @@ struct CgShape {
   static constexpr int kRows = 16 * kThreads / TM;
   static constexpr int kStages = TM == 16 ? 2 : 4;
   static constexpr int kStageBytes = kRows * kCgPitch + kCgCols * TM * 8;
-  static constexpr int kSmem = kStages * kStageBytes;
+  static constexpr int kRing = kStages * kStageBytes;
+  static constexpr int kSmem = kRing + 16 * kThreads * (int)sizeof(float2);  // and the threads' sums
 };
 
 __device__ __forceinline__ void cg_copy16(void* dst, const void* src, bool valid) {
@@ -116,6 +119,20 @@ __global__ void __launch_bounds__(CgShape<TM>::kThreads, CgShape<TM>::kPerSm)
       }
   };
 
+  // the thread's sums of the columns before
+  float2* sums = reinterpret_cast<float2*>(cg_smem + Sh::kRing);
+  bool fresh = true;
+  auto move = [&]() {
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      float2 v = acc[e / 4][e % 4];
+      float2& t = sums[e * Sh::kThreads + threadIdx.x];
+      if (!fresh) v = f2_add(v, t);
+      t = v;
+      acc[e / 4][e % 4] = make_float2(0.f, 0.f);
+    }
+    fresh = false;
+  };
 #pragma unroll
   for (int t = 0; t < Sh::kStages - 1; t++) {
     if (t < tiles) cg_load<TM, PAIRS>(cg_smem + t * Sh::kStageBytes, A, n, X, m, s0, r0, c0 + t * step);
@@ -153,15 +170,27 @@ __global__ void __launch_bounds__(CgShape<TM>::kThreads, CgShape<TM>::kPerSm)
         }
       }
     }
-    if ((t + 1) % (kCgRun / kCgCols) == 0) fold();
+    fold();
+    if ((t + 1) % (kCgFar / kCgCols) == 0) move();
   }
-  fold();
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (r0 + row + 8 * i < n && s0 + side + j < m)
-        atomicAdd(&Y[(size_t)(r0 + row + 8 * i) * m + s0 + side + j], acc[i][j]);
+  auto add_out = [&](int i, int j, float2 v) {
+    if (r0 + row + 8 * i < n && s0 + side + j < m) atomicAdd(&Y[(size_t)(r0 + row + 8 * i) * m + s0 + side + j], v);
+  };
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int ctas = (int)cluster.num_blocks();
+  move();
+  // every CTA adds up a part of the cluster's sums
+  cluster.sync();  // they are complete
+  for (int e = (int)cluster.block_rank(); e < 16; e += ctas) {
+    double re = 0.0, im = 0.0;
+    for (int r = 0; r < ctas; r++) {
+      const float2 v = *cluster.map_shared_rank(&sums[e * Sh::kThreads + threadIdx.x], r);
+      re += (double)v.x;
+      im += (double)v.y;
+    }
+    add_out(e / 4, e % 4, make_float2((float)re, (float)im));
+  }
+  cluster.sync();  // they have been read
 }
 
 template <int TM, bool PAIRS>
@@ -173,42 +202,76 @@ int cgemm_part(const float2* A, int n, const float2* X, int m, int first, int gr
     BEM_CUDA_TRY(cudaFuncSetAttribute(cgemm_kernel<TM, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
     attr.store(true, std::memory_order_release);
   }
-  const long long rows = (n + Sh::kRows - 1) / Sh::kRows;
-  // Cut of the columns: least time for whole rounds of the CTAs that fit (a
-  // CTA's start and end cost about 48 columns), around sqrt(32 n) columns, where
-  // the roundings of the CTA's sums and of the atomics are least together.
-  const double best = std::sqrt(32.0 * n);
-  const long long places = (long long)sms * Sh::kPerSm, widest = std::min(1024LL, (long long)(2.0 * best) + kCgRun);
-  long long span = 0, cost = 0;
-  for (long long cuts = (n + widest - 1) / widest; cuts <= (long long)(3.0 * n / best) + 1; cuts++) {
-    const long long w = ((n + cuts - 1) / cuts + kCgRun - 1) / kCgRun * kCgRun;
-    const long long rounds = (rows * groups * ((n + w - 1) / w) + places - 1) / places;
-    if (!span || rounds * (w + 48) < cost) {
-      span = w;
-      cost = rounds * (w + 48);
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(Sh::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = Sh::kSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  // CTAs that fit as clusters of 4 and of 8
+  static std::atomic<int> fit[2];
+  auto places = [&](int c) -> long long {
+    std::atomic<int>& known = fit[c == 8];
+    int k = known.load(std::memory_order_relaxed);
+    if (k == 0) {
+      at[0].val.clusterDim.y = (unsigned)c;
+      cfg.gridDim = dim3(1, (unsigned)c, 1);
+      if (cudaOccupancyMaxActiveClusters(&k, cgemm_kernel<TM, PAIRS>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        k = 0;
+      }
+      if (k < 1) k = -1;  // none
+      known.store(k, std::memory_order_relaxed);
     }
-  }
-  const long long cuts = (n + span - 1) / span;
-  (cgemm_kernel<TM, PAIRS><<<dim3((unsigned)rows, (unsigned)cuts, (unsigned)groups), Sh::kThreads, Sh::kSmem, s>>>(
-       A, n, X, m, first, Y),
-   count_launch());
-  BEM_CUDA_TRY(cudaGetLastError());
+    return k > 0 ? (long long)k * c : 0;
+  };
+  // Cut of the columns: least time for whole rounds of the CTAs that fit (a
+  // CTA's start and end cost about 48 columns), at most 1024 columns per CTA, at
+  // least 1024 per cluster.
+  const long long rows = (n + Sh::kRows - 1) / Sh::kRows;
+  int best = (n + 4095) / 4096 * 4, ctas = 4;
+  long long cost = 0;
+  for (int cuts = best; 128 * cuts <= n; cuts += 4)
+    for (int c = 4; c <= 8; c *= 2) {
+      if (cuts % c || 1024LL * cuts > (long long)c * n) continue;
+      const long long fits = places(c);
+      if (!fits) continue;
+      const long long w = ((n + cuts - 1) / cuts + kCgCols - 1) / kCgCols * kCgCols;
+      const long long time = (rows * groups * cuts + fits - 1) / fits * (w + 48);
+      if (!cost || time < cost) {
+        best = cuts;
+        ctas = c;
+        cost = time;
+      }
+    }
+  at[0].val.clusterDim.y = (unsigned)ctas;
+  cfg.gridDim = dim3((unsigned)rows, (unsigned)best, (unsigned)groups);
+  BEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, cgemm_kernel<TM, PAIRS>, A, n, X, m, first, Y));
+  count_launch();
   return BEM_OK;
 }
 
 // Y += A X.
 template <bool PAIRS>
 int cgemm_all(const float2* A, int n, const float2* X, int m, float2* Y, int sms, cudaStream_t s) {
-  // remainders of up to 32 right-hand sides in a tile of their own
-  const int wide = m % 64 > 32 ? (m + 63) / 64 : m / 64, first = 64 * wide, left = m - first;
+  // a remainder of up to 48 right-hand sides goes 16 at a time: three reads of A
+  // take less time than a tile of 64 (10 242 unknowns: 0.32 ms each, 1.2 ms)
+  const int wide = m % 64 > 48 ? (m + 63) / 64 : m / 64, first = 64 * wide;
   if (wide) {
     const int rc = cgemm_part<64, PAIRS>(A, n, X, m, 0, wide, Y, sms, s);
     if (rc) return rc;
   }
-  if (left > 16) return cgemm_part<32, PAIRS>(A, n, X, m, first, 1, Y, sms, s);
-  if (left > 0) return cgemm_part<16, PAIRS>(A, n, X, m, first, 1, Y, sms, s);
-  return BEM_OK;
+  return m > first ? cgemm_part<16, PAIRS>(A, n, X, m, first, (m - first + 15) / 16, Y, sms, s) : BEM_OK;
 }
+
+// Where it is used.  Up to 8192 unknowns it would still take 0.80 to 0.86 of the
+// time with 9 to 16 right-hand sides (2562 unknowns 42 and 34 us), but single
+// layers times smooth fields come out up to 1.15 times as far off 64 bits (642
+// to 5002 unknowns), and with 17 to 56 it is no faster.
+inline bool cgemm_takes(int n, int m) { return m > 8 && n > 8192; }
 
 int launch_cgemm(const float2* A, int n, const float2* X, int m, float2* Y, int sms, cudaStream_t s) {
   const bool pairs = (n & 1) == 0 && ((uintptr_t)A & 15) == 0;

@@ -3459,7 +3459,7 @@ int launch_block(const GmPtrs& P, const BkPtrs& K, const BkShape& sh, int group,
 
 int cmatmul(const float2* A, int n, const float2* X, int m, float2* Y, cudaStream_t s) {
   BEM_CUDA_TRY(cudaMemsetAsync(Y, 0, sizeof(float2) * (size_t)n * m, s));
-  if (m > kCgSides && n > kCgLeast) return launch_cgemm(A, n, X, m, Y, device_sms(), s);
+  if (cgemm_takes(n, m)) return launch_cgemm(A, n, X, m, Y, device_sms(), s);
   return launch_cgemv(A, n, X, m, Y, nullptr, s);
 }
 
