@@ -469,12 +469,14 @@ namespace {
 // nothing is gained: 4096 listeners x 64 on 20 480 triangles 2.6 ms, with runs
 // of 800 2.68 ms).
 //
-// An output takes one FP32 addition per run.  Where these are more than 64, the
+// An output takes one FP32 addition per run.  Where these are more than 64 (a
+// fortieth of the triangles on small meshes, 8 at the least: as many as the
+// chunks of 256 points that the point-by-point kernel added one by one), the
 // runs of a cluster (`most` CTAs at the most) are added up first, and there are
 // no more than 512 runs while that leaves at most 400 triangles in each: 20
 // listeners, one right-hand side, 20 480 triangles at 200 Hz 6.4e-7 -> 2.2e-7 off
-// 64 bits, in the same time.  Where they are fewer, a cluster gains nothing and
-// costs 2 us of a 46 us call.
+// 64 bits, in the same time; 100 listeners x 5 on 1280 triangles 2.3e-7 -> 1.9e-7.
+// Where they are fewer, a cluster gains nothing and costs 2 us of a 46 us call.
 struct ListenRuns {
   int run, parts, cluster;
 };
@@ -490,7 +492,8 @@ ListenRuns listen_runs(int groups, int nt, long long slots, int least, int most)
   r.run = (int)std::max<long long>(least, (nt + splits - 1) / splits);
   r.parts = (nt + r.run - 1) / r.run;
   r.cluster = 1;
-  while (r.cluster < most && r.parts > 64 * r.cluster) r.cluster *= 2;
+  const int limit = std::min(64, std::max(8, nt / 40));
+  while (r.cluster < most && r.parts > limit * r.cluster) r.cluster *= 2;
   return r;
 }
 
