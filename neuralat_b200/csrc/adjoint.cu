@@ -977,7 +977,8 @@ extern "C" int bem_vertex_gradient(const void* geom, float k, const void* lambda
   BEM_CUDA_TRY(cudaGetDevice(&dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int smem = (int)(kAdjWarps * sizeof(AdjWarp));
-  BEM_CUDA_TRY(cudaFuncSetAttribute(grad_regular_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  static DeviceOnce once;
+  if ((rc = once.shared_memory(grad_regular_kernel, smem))) return rc;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, grad_regular_kernel, kAdjThreads, smem));
   const long long n_steps = strip_steps(g.nblocks), warps = (long long)sms * (occ > 0 ? occ : 1) * kAdjWarps;
   const long long chunk = std::max(2LL, strip_part(n_steps, warps, kStripRounds));

@@ -829,11 +829,8 @@ int sm_count() {
 template <bool DO_V, bool DO_K>
 int launch_regular(const GeomView& g, float k, float2* V, float2* K, float v_scale, float k_scale, cudaStream_t s) {
   const int smem = (int)sizeof(RegSmem<DO_V, DO_K>);
-  static std::atomic<bool> attr_set{false};
-  if (!attr_set.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(regular_vk_kernel<DO_V, DO_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr_set.store(true, std::memory_order_release);
-  }
+  static DeviceOnce once;
+  if (const int rc = once.shared_memory(regular_vk_kernel<DO_V, DO_K>, smem)) return rc;
   const int n_groups = (g.nt + kTestTris - 1) / kTestTris;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, regular_vk_kernel<DO_V, DO_K>, kRegThreads, smem));
@@ -864,14 +861,11 @@ int launch_touch(const GeomView& g, float k, float2* V, float2* K, float v_scale
 }  // namespace
 
 namespace {
-// Persistent grid of a strip kernel (shared-memory attribute set once).
+// Persistent grid of a strip kernel.
 template <typename KernelT>
-int strip_grid(KernelT kernel, std::atomic<bool>& attr, int most_per_sm, long long* grid) {
+int strip_grid(KernelT kernel, DeviceOnce& once, int most_per_sm, long long* grid) {
   const int smem = (int)(kStripWarps * sizeof(VkWarp));
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr.store(true, std::memory_order_release);
-  }
+  if (const int rc = once.shared_memory(kernel, smem)) return rc;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kStripThreads, smem));
   if (most_per_sm > 0 && most_per_sm < occ) occ = most_per_sm;
@@ -880,9 +874,9 @@ int strip_grid(KernelT kernel, std::atomic<bool>& attr, int most_per_sm, long lo
 }
 
 int launch_strip_vk(const GeomView& g, float k, float2* V, float2* K, float v_scale, float k_scale, cudaStream_t s) {
-  static std::atomic<bool> attr{false};
+  static DeviceOnce once;
   long long grid = 0;
-  int rc = strip_grid(regular_strip_vk_kernel, attr, 0, &grid);
+  int rc = strip_grid(regular_strip_vk_kernel, once, 0, &grid);
   if (rc) return rc;
   const StripItems P = strip_items(g.nv, g.nblocks, grid * kStripWarps, kStripRounds, 2, g_tune_chunk, 0, 0);
   const long long blocks = (P.items + kStripWarps - 1) / kStripWarps;
@@ -1015,9 +1009,9 @@ int assemble_vk_batch(const GeomView* views, const float* ks, float2* const* Vs,
                       float mass_coeff, float k_coeff, void* ws, size_t ws_bytes, cudaStream_t s) {
   if (np <= 0) return BEM_ERR_INVALID_ARGUMENT;
   if (!ws || ws_bytes < batch_workspace_bytes(np)) return BEM_ERR_WORKSPACE;
-  static std::atomic<bool> attr{false};
+  static DeviceOnce once;
   long long grid = 0;
-  const int rc = strip_grid(regular_strip_vk_batch_kernel, attr, g_tune_ctas_per_sm, &grid);
+  const int rc = strip_grid(regular_strip_vk_batch_kernel, once, g_tune_ctas_per_sm, &grid);
   if (rc) return rc;
   // host descriptors
   const size_t hbytes = al256b(sizeof(BatchHeader)), pbytes = sizeof(BatchProblem) * (size_t)np;

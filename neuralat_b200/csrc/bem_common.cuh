@@ -337,13 +337,15 @@ unsigned long long launch_count();
   } while (0)
 
 namespace bemb {
-// Set-up of a kernel once on each device (one static object per kernel).  The
+// Set-up of a kernel once on each device (one static object per kernel or per
+// group of kernels set up together).  The
 // limit of a kernel's dynamic shared memory belongs to the kernel on the current
 // device and to all host threads: it is set once, to the largest size that any
 // launch asks for, since a thread that set its own call's size could lower it
 // between another thread's call and that call's launch.
 class DeviceOnce {
  public:
+  // set(): a bem_status
   template <typename F>
   int operator()(F&& set) {
     int dev = 0;
@@ -353,6 +355,14 @@ class DeviceOnce {
     const int rc = set();
     if (rc == BEM_OK) done_.fetch_or(bit, std::memory_order_release);
     return rc;
+  }
+  // the limit of dynamic shared memory
+  template <typename Kernel>
+  int shared_memory(Kernel kernel, size_t bytes) {
+    return (*this)([&]() -> int {
+      BEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      return BEM_OK;
+    });
   }
 
  private:

@@ -576,14 +576,11 @@ int bm_check(float k, const float2* L, const float2* R) {
   return BEM_OK;
 }
 
-// Persistent grid of a regular kernel (shared-memory attribute set once).
+// Persistent grid of a regular kernel.
 template <int TN, typename KernelT>
-int bm_grid(KernelT kernel, std::atomic<bool>& attr, long long* grid) {
+int bm_grid(KernelT kernel, DeviceOnce& once, long long* grid) {
   const int smem = (int)(kStripWarps * sizeof(BmWarp<TN>));
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr.store(true, std::memory_order_release);
-  }
+  if (const int rc = once.shared_memory(kernel, smem)) return rc;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kStripThreads, smem));
   *grid = (long long)bm_sm_count() * (occ > 0 ? occ : 1);
@@ -600,14 +597,14 @@ namespace {
 
 template <int TN>
 int bm_single_grid(long long* grid) {
-  static std::atomic<bool> attr{false};
-  return bm_grid<TN>(regular_bm_kernel<TN>, attr, grid);
+  static DeviceOnce once;
+  return bm_grid<TN>(regular_bm_kernel<TN>, once, grid);
 }
 
 template <int TN>
 int bm_batch_grid(long long* grid) {
-  static std::atomic<bool> attr{false};
-  return bm_grid<TN>(regular_bm_batch_kernel<TN>, attr, grid);
+  static DeviceOnce once;
+  return bm_grid<TN>(regular_bm_batch_kernel<TN>, once, grid);
 }
 
 int bm_rule(int order, int* tn) {

@@ -197,11 +197,8 @@ template <int TM, bool PAIRS>
 int cgemm_part(const float2* A, int n, const float2* X, int m, int first, int groups, float2* Y, int sms,
                cudaStream_t s) {
   using Sh = CgShape<TM>;
-  static std::atomic<bool> attr{false};
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(cgemm_kernel<TM, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
-    attr.store(true, std::memory_order_release);
-  }
+  static DeviceOnce once;
+  if (const int rc = once.shared_memory(cgemm_kernel<TM, PAIRS>, Sh::kSmem)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(Sh::kThreads, 1, 1);
   cfg.dynamicSmemBytes = Sh::kSmem;

@@ -388,12 +388,8 @@ template <int LAYER, int TN>
 int launch_regular_generic(const GeomView& g, float k, const float* normals, const float* curls, float2* out,
                            cudaStream_t s) {
   const int smem = (int)sizeof(GenSmem);
-  static std::atomic<bool> attr{false};
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(regular_generic_kernel<LAYER, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem));
-    attr.store(true, std::memory_order_release);
-  }
+  static DeviceOnce once;
+  if (const int rc = once.shared_memory(regular_generic_kernel<LAYER, TN>, smem)) return rc;
   int dev = 0, sms = 148, occ = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

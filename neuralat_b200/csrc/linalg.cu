@@ -440,13 +440,11 @@ int launch_resid_f64(const float2* A, int n, const double2* X, int m, double2* R
   if (n & 1) return launch_cmatmul<double, 1>(A, n, X, m, m, R, m, B, m, norm2, nullptr, s);
   BEM_CUDA_TRY(cudaMemsetAsync(R, 0, sizeof(double2) * (size_t)n * m, s));
   if (err && ((uintptr_t)A & 15) == 0) {
-    static std::atomic<bool> attr{false};
-    if (!attr.load(std::memory_order_acquire)) {
-      BEM_CUDA_TRY(cudaFuncSetAttribute(resid_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRtSmem));
-      attr.store(true, std::memory_order_release);
-    }
+    static DeviceOnce once;
+    int rc = once.shared_memory(resid_tma_kernel, kRtSmem);
+    if (rc) return rc;
     CUtensorMap map;
-    int rc = encode_map_2d_f32_sw128(&map, A, 2ull * n, (unsigned long long)n, 8ull * n, 2 * kRtTileCols, kRtRows);
+    rc = encode_map_2d_f32_sw128(&map, A, 2ull * n, (unsigned long long)n, 8ull * n, 2 * kRtTileCols, kRtRows);
     if (rc) return rc;
     const int n_cg = (n + kRtMaxCols - 1) / kRtMaxCols;
     const int cb = ((n + n_cg - 1) / n_cg + kRtTileCols - 1) / kRtTileCols * kRtTileCols;
@@ -696,12 +694,9 @@ __global__ void __launch_bounds__(kGtThreads, 1)
 
 template <int MR>
 int launch_cgemv_mr(const float2* A, int n, const float2* X, int m, float2* Y, const int* active, cudaStream_t s) {
-  static std::atomic<bool> attr{false};
+  static DeviceOnce once;
   const int smem = (int)(sizeof(float2) * MR * kGvChunk);
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(cgemv_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr.store(true, std::memory_order_release);
-  }
+  if (const int rc = once.shared_memory(cgemv_kernel<MR>, smem)) return rc;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cgemv_kernel<MR>, kGvThreads, smem));
   const int kc = (n + kGvChunk - 1) / kGvChunk;
@@ -721,14 +716,12 @@ int launch_cgemv_mr(const float2* A, int n, const float2* X, int m, float2* Y, c
 template <int MR>
 int launch_cgemv_tma(const float2* A, int n, const float2* X, int m, float2* Y, const int* active, int* err,
                      cudaStream_t s) {
-  static std::atomic<bool> attr{false};
+  static DeviceOnce once;
   const int smem = (int)gt_smem_bytes<MR>();
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(cgemv_tma_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr.store(true, std::memory_order_release);
-  }
+  int rc = once.shared_memory(cgemv_tma_kernel<MR>, smem);
+  if (rc) return rc;
   CUtensorMap map;
-  int rc = encode_map_2d_f32(&map, A, 2ull * n, (unsigned long long)n, 8ull * n, 2 * kGtTileCols, kGtBlockRows);
+  rc = encode_map_2d_f32(&map, A, 2ull * n, (unsigned long long)n, 8ull * n, 2 * kGtTileCols, kGtBlockRows);
   if (rc) return rc;
   const int kc = (n + kGvChunk - 1) / kGvChunk;
   const int groups = (m + MR - 1) / MR;
@@ -3182,15 +3175,16 @@ int sm_count_linalg() {
 }
 
 int arnoldi_shape(int n, int m, ArnShape* out) {
-  static std::atomic<bool> attr{false};
+  static DeviceOnce once;
   int dev = 0, smem_optin = 0;
   BEM_CUDA_TRY(cudaGetDevice(&dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (!attr.load(std::memory_order_acquire)) {
+  const int rc = once([&]() -> int {
     BEM_CUDA_TRY(cudaFuncSetAttribute(gm_arnoldi_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     BEM_CUDA_TRY(cudaFuncSetAttribute(gm_arnoldi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin));
-    attr.store(true, std::memory_order_release);
-  }
+    return BEM_OK;
+  });
+  if (rc) return rc;
   const int max_cl = g_arn_max_cluster > 0 && g_arn_max_cluster < kArnMaxCluster ? g_arn_max_cluster : kArnMaxCluster;
   int cl = 1;
   while (cl < max_cl && (long long)cl * 2 * kArnThreads < n) cl++;
@@ -3258,12 +3252,7 @@ int cycle_shape(int n, int R, CyShape* out) {
   const size_t smem = cy_layout(n, rows, R).total;
   if (smem + 1024 > (size_t)smem_optin) return BEM_ERR_UNSUPPORTED;  // 1 KB for the static shared memory
   static DeviceOnce once;
-  const int rc = once([&]() -> int {
-    BEM_CUDA_TRY(
-        cudaFuncSetAttribute(gm_single_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-    return BEM_OK;
-  });
-  if (rc) return rc;
+  if (const int rc = once.shared_memory(gm_single_kernel, smem_optin - 1024)) return rc;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gm_single_kernel, kCyThreads, smem));
   out->rows = rows;
@@ -3309,7 +3298,7 @@ int solve_single(const GmPtrs& P, const CyShape& shape, const float2* A, const f
 }
 
 int coop_shape(int n, int m, int R, CoShape* out) {
-  static std::atomic<bool> attr{false};
+  static DeviceOnce once;
   int dev = 0, coop_ok = 0, smem_optin = 0;
   BEM_CUDA_TRY(cudaGetDevice(&dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&coop_ok, cudaDevAttrCooperativeLaunch, dev));
@@ -3327,11 +3316,7 @@ int coop_shape(int n, int m, int R, CoShape* out) {
   while (slots > 2 && co_layout(m, npc, R, cpc, slots).total > (size_t)smem_optin / 2) slots--;
   const size_t smem = co_layout(m, npc, R, cpc, slots).total;
   if (smem > (size_t)smem_optin / 2) return BEM_ERR_UNSUPPORTED;
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(gm_arnoldi_coop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      smem_optin / 2));
-    attr.store(true, std::memory_order_release);
-  }
+  if (const int rc = once.shared_memory(gm_arnoldi_coop_kernel, smem_optin / 2)) return rc;
   int occ = 0;
   BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, gm_arnoldi_coop_kernel, kCoThreads, smem));
   if (occ < 1 || grid > occ * sms) return BEM_ERR_UNSUPPORTED;
@@ -3368,8 +3353,7 @@ int block_dispatch(int pp, int tile, F&& f) {
 }
 
 int block_shape(int n, int m, int R, BkShape* out) {
-  static std::mutex mu;
-  static bool attr_set[2][3] = {};
+  static DeviceOnce once[2][3];
   int dev = 0, coop_ok = 0, smem_optin = 0;
   BEM_CUDA_TRY(cudaGetDevice(&dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&coop_ok, cudaDevAttrCooperativeLaunch, dev));
@@ -3409,19 +3393,11 @@ int block_shape(int n, int m, int R, BkShape* out) {
     sh.vbase[g] = row;
     row += (sh.nb + 1) * sh.p[g];
     const int pi = sh.g[g].pp == 4 ? 0 : sh.g[g].pp == 8 ? 1 : 2, ti = sh.g[g].tile == 32 ? 0 : 1;
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      if (!attr_set[ti][pi]) {
-        int rc = block_dispatch(sh.g[g].pp, sh.g[g].tile, [&](auto kern) -> int {
-          BEM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_optin - 1024));
-          return BEM_OK;
-        });
-        if (rc) return rc;
-        attr_set[ti][pi] = true;
-      }
-    }
+    int rc = block_dispatch(sh.g[g].pp, sh.g[g].tile,
+                            [&](auto kern) -> int { return once[ti][pi].shared_memory(kern, smem_optin - 1024); });
+    if (rc) return rc;
     int occ = 0;
-    int rc = block_dispatch(sh.g[g].pp, sh.g[g].tile, [&](auto kern) -> int {
+    rc = block_dispatch(sh.g[g].pp, sh.g[g].tile, [&](auto kern) -> int {
       BEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBkThreads, sh.smem[g]));
       return BEM_OK;
     });
@@ -3622,14 +3598,10 @@ extern "C" int bem_gmres_solve(const void* A, int n, const void* B, int m, void*
   const int st_nb = (npairs_all + st_span - 1) / st_span;
   const int st_grid = std::min(m * st_nb, 3 * sm_count_linalg());  // persistent: up to 3 blocks per SM
   if (streamed) {
-    static std::atomic<bool> st_attr{false};
-    if (!st_attr.load(std::memory_order_acquire)) {
-      BEM_CUDA_TRY(cudaFuncSetAttribute(gm_st_dots_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(sizeof(double4) * 4096)));
-      BEM_CUDA_TRY(cudaFuncSetAttribute(gm_st_dots_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(sizeof(double4) * 4096)));
-      st_attr.store(true, std::memory_order_release);
-    }
+    static DeviceOnce once[2];
+    int rc0 = once[0].shared_memory(gm_st_dots_kernel<0>, sizeof(double4) * 4096);
+    if (!rc0) rc0 = once[1].shared_memory(gm_st_dots_kernel<1>, sizeof(double4) * 4096);
+    if (rc0) return rc0;
   }
   // one Arnoldi step: the matvec reads the operand that gm_arnoldi_kernel (or
   // gm_start_norm_kernel) wrote and accumulates into Y, which

@@ -545,15 +545,11 @@ int listen_few(const GeomView& g, const float* pts, int np, float k, const float
 
 template <int J>
 int listen_many(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
-                int rhs0, float2* out, int dev, int sms, cudaStream_t s) {
+                int rhs0, float2* out, int sms, cudaStream_t s) {
   const int smem = (int)sizeof(ListenSmem<J>);
   static std::atomic<int> clusters[3];
-  static std::atomic<unsigned long long> attr{0};  // devices whose attribute is set
-  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
-  if (!(attr.load(std::memory_order_acquire) & bit)) {
-    BEM_CUDA_TRY(cudaFuncSetAttribute(listen_many_kernel<J>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr.fetch_or(bit, std::memory_order_release);
-  }
+  static DeviceOnce once;
+  if (const int rc = once.shared_memory(listen_many_kernel<J>, smem)) return rc;
   return listen_launch(listen_many_kernel<J>, (np + kLsThreads - 1) / kLsThreads, g.nt, sms, J == 8 ? 2 : 3, 12, 4,
                        (size_t)smem, s, clusters, g, pts, np, k, neu, dir, nrhs, rhs0, out);
 }
@@ -579,10 +575,10 @@ int b2p_enqueue(const GeomView& g, const float* points, int np, float k, const v
   } else {
     for (int r0 = 0; r0 < nrhs; r0 += 64) {
       const int left = nrhs - r0;
-      const int rc = left > 32   ? listen_many<8>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s)
-                     : left > 16 ? listen_many<4>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s)
-                     : left > 8  ? listen_many<2>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s)
-                                 : listen_many<1>(g, points, np, k, neu, dir, nrhs, r0, o, dev, sms, s);
+      const int rc = left > 32   ? listen_many<8>(g, points, np, k, neu, dir, nrhs, r0, o, sms, s)
+                     : left > 16 ? listen_many<4>(g, points, np, k, neu, dir, nrhs, r0, o, sms, s)
+                     : left > 8  ? listen_many<2>(g, points, np, k, neu, dir, nrhs, r0, o, sms, s)
+                                 : listen_many<1>(g, points, np, k, neu, dir, nrhs, r0, o, sms, s);
       if (rc) return rc;
     }
   }

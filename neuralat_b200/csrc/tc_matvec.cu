@@ -682,14 +682,10 @@ TcLayout tc_layout(int n, int m, int precision) {
 template <int NB, bool X3, bool F16>
 int launch_tc(const TcLayout& L, char* ws, int n, const int* active, int nact, float* Y, int m2, cudaStream_t s) {
   using S = TcSmem<NB, X3>;
-  static std::atomic<bool> attr{false};
-  if (!attr.load(std::memory_order_acquire)) {
-    BEM_CUDA_TRY(
-        cudaFuncSetAttribute(tc_gemm_kernel<NB, X3, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes));
-    attr.store(true, std::memory_order_release);
-  }
+  static DeviceOnce once;
+  int rc = once.shared_memory(tc_gemm_kernel<NB, X3, F16>, S::kBytes);
+  if (rc) return rc;
   CUtensorMap mah, mal, mbh, mbl;
-  int rc;
   if ((rc = make_map(&mah, ws + L.ah, 2 * n, n, L.ld, kBM))) return rc;
   if ((rc = make_map(&mal, ws + (X3 ? L.alo : L.ah), 2 * n, n, L.ld, kBM))) return rc;
   if ((rc = make_map(&mbh, ws + L.bh, 2 * n, NB, L.ld, NB))) return rc;
@@ -738,12 +734,8 @@ int tc_operator_prepare(const float2* A, int n, int precision, void* ws, cudaStr
     const size_t row_bytes = sizeof(float4) * (size_t)(n / 2);
     const bool staged = (n & 1) == 0 && (L.ld & 3) == 0 && ((uintptr_t)A & 15) == 0 && row_bytes <= 96 * 1024;
     if (staged) {
-      static std::atomic<bool> attr{false};
-      if (!attr.load(std::memory_order_acquire)) {
-        BEM_CUDA_TRY(cudaFuncSetAttribute(tc_split_a_f16_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          96 * 1024));
-        attr.store(true, std::memory_order_release);
-      }
+      static DeviceOnce once;
+      if (const int rc = once.shared_memory(tc_split_a_f16_smem_kernel, 96 * 1024)) return rc;
       int dev = 0, sms = 148;
       cudaGetDevice(&dev);
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
