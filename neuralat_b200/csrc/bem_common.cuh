@@ -329,11 +329,15 @@ void count_launches(unsigned long long n);
 unsigned long long launch_count();
 }  // namespace bemb
 
-// error-checking helper for host code inside the library
+// error-checking helper for host code inside the library; a reported error is
+// cleared, or the next call's check of its launches would report it once more
 #define BEM_CUDA_TRY(expr)                          \
   do {                                              \
     cudaError_t _e = (expr);                        \
-    if (_e != cudaSuccess) return BEM_ERR_CUDA;     \
+    if (_e != cudaSuccess) {                        \
+      cudaGetLastError();                           \
+      return BEM_ERR_CUDA;                          \
+    }                                               \
   } while (0)
 
 namespace bemb {

@@ -543,7 +543,7 @@ int geom_view(const void* geom, GeomView* v, GeomHeader* out_hdr) {
     }
   }
   if (!hit) {
-    if (cudaMemcpy(&h, geom, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return BEM_ERR_CUDA;
+    BEM_CUDA_TRY(cudaMemcpy(&h, geom, sizeof(h), cudaMemcpyDeviceToHost));
     if (h.magic == kGeomMagic) cache_put(geom, h);
   }
   if (h.magic != kGeomMagic) return BEM_ERR_WORKSPACE;

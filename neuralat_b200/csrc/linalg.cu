@@ -2905,7 +2905,7 @@ int capture_graph(const std::function<int(cudaStream_t)>& body, cudaGraphExec_t*
   }
   const cudaError_t ei = cudaGraphInstantiate(exec, graph, 0);
   cudaGraphDestroy(graph);
-  if (ei != cudaSuccess) return BEM_ERR_CUDA;
+  BEM_CUDA_TRY(ei);
   *nkern = launch_count() - l0;
   return BEM_OK;
 }

@@ -113,3 +113,26 @@ def test_second_device(cuda, calls):
         large = {k for k in cuda.launched}
         cuda.launched.clear()
     assert any("strip_vk" in k for k in large) or any("cgemm" in k for k in large)
+
+
+@pytest.mark.parametrize("event", ["launch", "copy", "occupancy"])
+def test_a_reported_error_is_gone(cuda, event):
+    """An error of the runtime ends the call that met it and no later one."""
+    A, X, Y = array((600, 600)), array((600, 8)), array((600, 8))
+    calls = [lambda: cuda.solve(600), lambda: cuda.solve(600, 8, use_x0=1),
+             lambda: cuda.lib.bem_cmatmul(at(A), 600, at(X), 8, at(Y), None)]
+    for first in calls:
+        failed = []
+
+        def on(name, kernel, pointer, value):
+            if name == event and not failed:
+                failed.append(kernel)
+                return 1  # cudaErrorInvalidValue
+            return 0
+
+        cuda.on = on
+        status = first()
+        cuda.on = None
+        assert status in (L.BEM_OK, L.BEM_ERR_CUDA)  # where there is another way, it is taken
+        for call in calls:
+            assert call() == L.BEM_OK, failed
