@@ -181,8 +181,10 @@ int bem_assembly_status(bem_stream_t stream);
 /* Launch-shape knobs of the assembly kernels, set by the autotuner
  * (0 = automatic).  Process-wide. */
 enum {
-  BEM_TUNE_ASSEMBLY_CHUNK = 1,      /* trial blocks (32 triangles) per work item */
-  BEM_TUNE_ASSEMBLY_CTAS_PER_SM = 2, /* persistent CTAs per SM (<= occupancy limit) */
+  BEM_TUNE_ASSEMBLY_CHUNK = 1,      /* trial blocks (32 triangles) per work item of the V and K assemblies:
+                                        both, one alone, batched */
+  BEM_TUNE_ASSEMBLY_CTAS_PER_SM = 2, /* persistent CTAs per SM (<= occupancy limit) of the batched V and K
+                                        assembly and of one operator alone */
   BEM_TUNE_TC_PROMOTE = 3,           /* tensor-core matvec: K blocks (64 reals) accumulated in tensor
                                         memory before the partial sum leaves it (0: automatic) */
   BEM_TUNE_GMRES_REORTH = 4,         /* Arnoldi Gram-Schmidt passes: 0 automatic (one), 1 one, 2 two */

@@ -839,7 +839,7 @@ int launch_regular(const GeomView& g, float k, float2* V, float2* K, float v_sca
   // chunk of trial tiles per work item: enough items to balance the grid
   int chunk = (int)((long long)n_groups * g.ntiles / (8LL * grid));
   chunk = chunk < 1 ? 1 : (chunk > 64 ? 64 : chunk);
-  if (g_tune_chunk > 0) chunk = g_tune_chunk;
+  if (g_tune_chunk > 0) chunk = 2 * std::min(g_tune_chunk, g.ntiles);  // the knob counts blocks of 32
   const int n_chunks = (g.ntiles + chunk - 1) / chunk;
   const int n_items = n_groups * n_chunks;
   (regular_vk_kernel<DO_V, DO_K><<<grid < n_items ? grid : n_items, kRegThreads, smem, s>>>(
@@ -927,8 +927,8 @@ int assemble_mass(const GeomView& g, float2* M, float coeff, bool zero, cudaStre
 namespace bemb {
 
 namespace {
-int g_tune_chunk = 0;        // trial tiles per regular work item (0: automatic)
-int g_tune_ctas_per_sm = 0;  // persistent CTAs per SM (0: occupancy limit)
+int g_tune_chunk = 0;        // trial blocks (32 triangles) per regular work item (0: automatic)
+int g_tune_ctas_per_sm = 0;  // persistent CTAs per SM (0: occupancy limit; not for V and K of one problem)
 
 struct PinnedStage {
   void* buf = nullptr;

@@ -136,3 +136,35 @@ def test_a_reported_error_is_gone(cuda, event):
         assert status in (L.BEM_OK, L.BEM_ERR_CUDA)  # where there is another way, it is taken
         for call in calls:
             assert call() == L.BEM_OK, failed
+
+
+@pytest.mark.parametrize("blocks", [1, 3, 4, 100, (1 << 31) - 1])
+def test_chunk_knob_means_blocks(cuda, blocks):
+    """The chunk knob counts 32-triangle trial blocks in every V and K assembly:
+    chunk is argument 6 of the one-operator kernel, in 16-triangle tiles, and
+    number 2 (behind two 64-bit counts) of the strip kernel's items, in steps of a
+    triangle."""
+    from neuralat_b200.bem import meshes as M
+
+    v, t = M.icosphere(3, 0.1)
+    g, X, Y = cuda.geometry(v, t), array((len(v), len(v))), array((len(v), len(v)))
+    seen = {}
+
+    def on(event, name, pointer, value):
+        if event == "launch" and "regular" in name:
+            argument = ctypes.cast(pointer, ctypes.POINTER(ctypes.POINTER(ctypes.c_int)))[6]
+            seen["strip" if "strip" in name else "tiles"] = argument[4] if "strip" in name else 16 * argument[0]
+        return 0
+
+    L.check(cuda.lib.bem_set_tuning(L.TUNE_ASSEMBLY_CHUNK, blocks))
+    try:
+        cuda.on = on
+        for a, b in ((at(X), at(Y)), (at(X), None), (None, at(Y))):
+            assert cuda.lib.bem_boundary_matrices_vk(at(g), 1.0, a, b, 0.5, -1.0, None) == L.BEM_OK
+            if len(seen) == 2:
+                assert min(seen["strip"], len(t)) == min(seen["tiles"], len(t)) == min(32 * blocks, len(t))
+                del seen["tiles"]
+        assert "strip" in seen
+    finally:
+        cuda.on = None
+        L.check(cuda.lib.bem_set_tuning(L.TUNE_ASSEMBLY_CHUNK, 0))
