@@ -851,51 +851,62 @@ __global__ void conj_transpose_kernel(const float2* __restrict__ A, int n, float
 }
 
 // S^H pbar and D^H pbar: `lanes` lanes (a power of two, 32 at most) per trial
-// quadrature point, each over every lanes-th listener.  Their sums meet in
-// registers, so that a vertex takes one FP32 addition per point of its triangles
-// however many lanes share the point.  (With a grid of listener parts, each
-// added on its own, the velocity gradient of 144 triangles and 615 listeners was
-// 8.0e-7 off 64 bits; it is 2.2e-7 so, and 2.6e-7 with one lane per point.)
-__global__ void b2p_adjoint_kernel(GeomView g, const float* __restrict__ pts, int np, int lanes, float k,
-                                   const float2* __restrict__ pbar, float2* __restrict__ out_s,
-                                   float2* __restrict__ out_d) {
-  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long at = id / lanes;
-  const int jq = (int)min(at, 6LL * g.nt - 1);  // past the end: for the shuffles only
-  const int j = jq / 6, q = jq - 6 * j;
-  const TriRec& r = g.rec_orig[j];
-  float zsr = 0.f, zsi = 0.f, zdr = 0.f, zdi = 0.f;
+// triangle, each over every lanes-th listener.  A listener's six points are
+// summed onto the triangle's vertices in FP32, the listeners and lanes in FP64,
+// so that a vertex takes one FP32 addition per triangle however many lanes share
+// it.  (With a thread per point and a grid of listener parts, each added on its
+// own, the velocity gradient of 144 triangles and 615 listeners was 8.0e-7 off
+// 64 bits; it is 1.9e-7 so, and 2.6e-7 with one thread per point and no parts.
+// 2000 listeners x 80 triangles 79 us, 128 x 5120 27 us; in parts 261 and 27 us.)
+__global__ void __launch_bounds__(128)
+    b2p_adjoint_kernel(GeomView g, const float* __restrict__ pts, int np, int lanes, float k,
+                       const float2* __restrict__ pbar, float2* __restrict__ out_s, float2* __restrict__ out_d) {
+  const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x, at = id / lanes;
+  const TriRec& r = g.rec_orig[at < g.nt ? at : g.nt - 1];  // past the end: for the shuffles only
+  float y[18];
+#pragma unroll
+  for (int e = 0; e < 18; e++) y[e] = r.qp[e];
+  const float n0 = r.n[0], n1 = r.n[1], n2 = r.n[2];
+  double sum[12];  // S^H and D^H pbar at the vertices, (re, im)
+#pragma unroll
+  for (int e = 0; e < 12; e++) sum[e] = 0.0;
   for (int p = (int)(id & (lanes - 1)); p < np; p += lanes) {
-    const float dx = r.qp[3 * q] - pts[3 * p], dy = r.qp[3 * q + 1] - pts[3 * p + 1], dz = r.qp[3 * q + 2] - pts[3 * p + 2];
-    float rr = sqrtf(dx * dx + dy * dy + dz * dz);
-    rr = fmaxf(rr, kEps);
-    float s, c;
-    sincosf(k * rr, &s, &c);
-    const float u = 1.f / rr;
-    const float gr = c * u, gi = s * u;
-    const float dn = dx * r.n[0] + dy * r.n[1] + dz * r.n[2];
-    const float f = -dn * u * u * u, kr = k * rr;
-    const float dr = (c + kr * s) * f, di = (s - kr * c) * f;
+    const float x0 = pts[3 * p], x1 = pts[3 * p + 1], x2 = pts[3 * p + 2];
     const float2 pb = pbar[p];
-    // conj(kernel) * pbar
-    zsr += gr * pb.x + gi * pb.y;
-    zsi += gr * pb.y - gi * pb.x;
-    zdr += dr * pb.x + di * pb.y;
-    zdi += dr * pb.y - di * pb.x;
+    float t[12];
+#pragma unroll
+    for (int e = 0; e < 12; e++) t[e] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      const float dx = y[3 * q] - x0, dy = y[3 * q + 1] - x1, dz = y[3 * q + 2] - x2;
+      float rr = sqrtf(dx * dx + dy * dy + dz * dz);
+      rr = fmaxf(rr, kEps);
+      float s, c;
+      sincosf(k * rr, &s, &c);
+      const float u = 1.f / rr;
+      const float gr = c * u, gi = s * u;
+      const float dn = dx * n0 + dy * n1 + dz * n2;
+      const float f = -dn * u * u * u, kr = k * rr;
+      const float dr = (c + kr * s) * f, di = (s - kr * c) * f;
+      // conj(kernel) * pbar
+      const float z[4] = {gr * pb.x + gi * pb.y, gr * pb.y - gi * pb.x, dr * pb.x + di * pb.y, dr * pb.y - di * pb.x};
+#pragma unroll
+      for (int b = 0; b < 3; b++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) t[4 * b + e] = fmaf((float)(tri6_w(q) * tri6_phi(q, b)), z[e], t[4 * b + e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 12; e++) sum[e] += (double)t[e];
   }
-  for (int o = lanes >> 1; o > 0; o >>= 1) {
-    zsr += __shfl_xor_sync(0xffffffffu, zsr, o);
-    zsi += __shfl_xor_sync(0xffffffffu, zsi, o);
-    zdr += __shfl_xor_sync(0xffffffffu, zdr, o);
-    zdi += __shfl_xor_sync(0xffffffffu, zdi, o);
-  }
-  if ((id & (lanes - 1)) != 0 || at >= 6LL * g.nt) return;
-  const float w = (float)tri6_w(q) * r.area * kInv4Pi;
+  for (int o = lanes >> 1; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < 12; e++) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], o);
+  if ((id & (lanes - 1)) != 0 || at >= g.nt) return;
+  const double w = (double)r.area * (double)kInv4Pi;
 #pragma unroll
   for (int b = 0; b < 3; b++) {
-    const float f = w * (float)tri6_phi(q, b);
-    if (out_s) atomicAdd(&out_s[r.v[b]], make_float2(f * zsr, f * zsi));
-    if (out_d) atomicAdd(&out_d[r.v[b]], make_float2(f * zdr, f * zdi));
+    if (out_s) atomicAdd(&out_s[r.v[b]], make_float2((float)(w * sum[4 * b]), (float)(w * sum[4 * b + 1])));
+    if (out_d) atomicAdd(&out_d[r.v[b]], make_float2((float)(w * sum[4 * b + 2]), (float)(w * sum[4 * b + 3])));
   }
 }
 
@@ -948,10 +959,10 @@ extern "C" int bem_boundary2potential_adjoint(const void* geom, const float* poi
   int dev = 0, sms = 148;
   BEM_CUDA_TRY(cudaGetDevice(&dev));
   BEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // lanes until every SM holds about 1024 threads, at least 8 listeners in each
+  // lanes until every SM holds about 1024 threads, at least 2 listeners in each
   int lanes = 1;
-  while (lanes < 32 && 6LL * g.nt * lanes < 1024LL * sms && np >= 16 * lanes) lanes *= 2;
-  const long long threads = 6LL * g.nt * lanes;
+  while (lanes < 32 && (long long)g.nt * lanes < 1024LL * sms && np >= 4 * lanes) lanes *= 2;
+  const long long threads = (long long)g.nt * lanes;
   (b2p_adjoint_kernel<<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(
        g, points, np, lanes, k, (const float2*)pbar, (float2*)out_s, (float2*)out_d),
    count_launch());
