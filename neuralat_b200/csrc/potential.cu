@@ -129,7 +129,7 @@ constexpr int kLsChunk = 16;  // triangles staged per warp
 // (blockIdx.y) for 32 listeners, up to M <= 4 right-hand sides: the products
 // with the vertex densities stay in the listener's own registers.  Each warp
 // walks a quarter of the run; their sums meet in shared memory and those of a
-// cluster's runs in its first CTA, so that few FP32 terms are added to an output
+// cluster's runs in its first CTA (FP64, rounded once), so that few FP32 terms are added to an output
 // one after the other.
 //
 // Bound by the FP32 and sincos units (about 125 instructions for the 6 points
@@ -212,9 +212,13 @@ __global__ void __launch_bounds__(kLsThreads)
   cluster.sync();  // every CTA's sums are complete
   if (cluster.block_rank() == 0 && p < np)
     for (int s = warp; s < M && s < nrhs; s += kLsWarps) {
-      float2 t = sum_s[0][s][lane];
-      for (unsigned r = 1; r < cluster.num_blocks(); r++) t = f2_add(t, *cluster.map_shared_rank(&sum_s[0][s][lane], r));
-      atomicAdd(&out[(size_t)p * nrhs + s], t);
+      double re = 0.0, im = 0.0;
+      for (unsigned r = 0; r < cluster.num_blocks(); r++) {
+        const float2 t = *cluster.map_shared_rank(&sum_s[0][s][lane], r);
+        re += (double)t.x;
+        im += (double)t.y;
+      }
+      atomicAdd(&out[(size_t)p * nrhs + s], make_float2((float)re, (float)im));
     }
   cluster.sync();  // the sums have been read
 }
@@ -392,19 +396,18 @@ __global__ void __launch_bounds__(kLsThreads, J == 8 ? 2 : 3)
       for (int j = 0; j < J; j++) add_out(l, j, sm.sum[l * J + j][tid]);
     return;
   }
-  // the cluster's sums, an equal part of them per CTA
+  // the cluster's sums, a part of them per CTA
   cluster.sync();  // every CTA's sums are complete
-  const int mine = 4 * J / ctas, q0 = (int)cluster.block_rank() * mine;
-  for (int q = q0; q < q0 + mine; q++) {
-    float4 t = *cluster.map_shared_rank(&sm.sum[q][tid], 0);
-    for (int r = 1; r < ctas; r++) {
+  for (int q = (int)cluster.block_rank(); q < 4 * J; q += ctas) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int r = 0; r < ctas; r++) {
       const float4 v = *cluster.map_shared_rank(&sm.sum[q][tid], r);
-      t.x += v.x;
-      t.y += v.y;
-      t.z += v.z;
-      t.w += v.w;
+      t[0] += (double)v.x;
+      t[1] += (double)v.y;
+      t[2] += (double)v.z;
+      t[3] += (double)v.w;
     }
-    add_out(q / J, q % J, t);
+    add_out(q / J, q % J, make_float4((float)t[0], (float)t[1], (float)t[2], (float)t[3]));
   }
   cluster.sync();  // the sums have been read
 }
@@ -472,7 +475,7 @@ namespace {
 // An output takes one FP32 addition per run.  Where these are more than 64 (a
 // fortieth of the triangles on small meshes, 8 at the least: as many as the
 // chunks of 256 points that the point-by-point kernel added one by one), the
-// runs of a cluster (`most` CTAs at the most) are added up first, and there are
+// runs of a cluster (up to 8 CTAs) are added up first, and there are
 // no more than 512 runs while that leaves at most 400 triangles in each: 20
 // listeners, one right-hand side, 20 480 triangles at 200 Hz 6.4e-7 -> 2.2e-7 off
 // 64 bits, in the same time; 100 listeners x 5 on 1280 triangles 2.3e-7 -> 1.9e-7.
@@ -481,7 +484,7 @@ struct ListenRuns {
   int run, parts, cluster;
 };
 
-ListenRuns listen_runs(int groups, int nt, long long slots, int least, int most) {
+ListenRuns listen_runs(int groups, int nt, long long slots, int least) {
   long long splits = 1;
   for (int waves = 1; waves <= 64; waves++) {
     splits = std::max<long long>(1, waves * slots / groups);
@@ -493,7 +496,7 @@ ListenRuns listen_runs(int groups, int nt, long long slots, int least, int most)
   r.parts = (nt + r.run - 1) / r.run;
   r.cluster = 1;
   const int limit = std::min(64, std::max(8, nt / 40));
-  while (r.cluster < most && r.parts > limit * r.cluster) r.cluster *= 2;
+  while (r.cluster < 8 && r.parts > limit * r.cluster) r.cluster *= 2;
   return r;
 }
 
@@ -501,9 +504,9 @@ ListenRuns listen_runs(int groups, int nt, long long slots, int least, int most)
 // that an SM holds; clusters: how many clusters of 2, 4 and 8 the GPU holds (0:
 // not known yet).
 template <typename Kernel, typename... Args>
-int listen_launch(Kernel kernel, int groups, int nt, int sms, int per_sm, int least, int most, size_t smem,
+int listen_launch(Kernel kernel, int groups, int nt, int sms, int per_sm, int least, size_t smem,
                   cudaStream_t s, std::atomic<int>* clusters, Args... args) {
-  ListenRuns r = listen_runs(groups, nt, (long long)per_sm * sms, least, most);
+  ListenRuns r = listen_runs(groups, nt, (long long)per_sm * sms, least);
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kLsThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
@@ -525,7 +528,7 @@ int listen_launch(Kernel kernel, int groups, int nt, int sms, int per_sm, int le
       known.store(n, std::memory_order_relaxed);
     }
     const int c = r.cluster;
-    r = listen_runs(groups, nt, (long long)n * c, least, most);
+    r = listen_runs(groups, nt, (long long)n * c, least);
     r.cluster = c;
     r.parts = (r.parts + c - 1) / c * c;  // the last runs may be empty
   }
@@ -539,7 +542,7 @@ template <int M>
 int listen_few(const GeomView& g, const float* pts, int np, float k, const float2* neu, const float2* dir, int nrhs,
                float2* out, int sms, cudaStream_t s) {
   static std::atomic<int> clusters[3];
-  return listen_launch(listen_few_kernel<M>, (np + 31) / 32, g.nt, sms, 8, 16, 8, 0, s, clusters, g, pts, np, k, neu, dir,
+  return listen_launch(listen_few_kernel<M>, (np + 31) / 32, g.nt, sms, 8, 16, 0, s, clusters, g, pts, np, k, neu, dir,
                        nrhs, out);
 }
 
@@ -550,7 +553,7 @@ int listen_many(const GeomView& g, const float* pts, int np, float k, const floa
   static std::atomic<int> clusters[3];
   static DeviceOnce once;
   if (const int rc = once.shared_memory(listen_many_kernel<J>, smem)) return rc;
-  return listen_launch(listen_many_kernel<J>, (np + kLsThreads - 1) / kLsThreads, g.nt, sms, J == 8 ? 2 : 3, 12, 4,
+  return listen_launch(listen_many_kernel<J>, (np + kLsThreads - 1) / kLsThreads, g.nt, sms, J == 8 ? 2 : 3, 12,
                        (size_t)smem, s, clusters, g, pts, np, k, neu, dir, nrhs, rhs0, out);
 }
 }  // namespace
