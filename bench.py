@@ -47,7 +47,7 @@ sys.path.insert(0, ROOT)
 METRIC = "assemble+solve+eval s/problem @20k tris (icosphere s5, 8 RHS, 4 kHz, 256 listeners), 1 B200"
 WORKLOAD = ("icosphere s5 N=10242 T=20480, r=0.15 m axes*U[0.7,1.3] (seed 1), k=2pi*4000/343, "
             "8 smoothed complex Gaussian Neumann RHS (seed 2), 256 listeners r=0.5 m (seed 0), CBIE rtol 1e-6")
-F_VK = 63.0  # FP32 flops per regular quadrature-point pair, fused V+K (algorithmic count)
+F_VK = 74.0  # FP32 pipe work per unordered regular quadrature-point pair, V and K: 37 operations, an FMA's 2 flop each
 
 
 def parse():
@@ -563,7 +563,7 @@ def run_ours(args):
     # ---- roofline of the dominant kernel (fused regular V+K assembly) ----------
     clocks = clk.summary()
     peak = fp32_peak_tflops(clocks.get("sm_max_mhz"))
-    achieved = F_VK * n_eval / (asm_ms / 1e3) / 1e12
+    achieved = F_VK * (n_eval / 2) / (asm_ms / 1e3) / 1e12  # each unordered pair is evaluated once
     # DRAM traffic of regular_strip_vk_kernel: 9.43 GB per launch measured by ncu
     # at icosphere s5 (N = 10 242: the atomic read-modify-write of the two output
     # matrices), scaled by the units processed to this mesh
@@ -571,9 +571,9 @@ def run_ours(args):
     roofline = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": traffic,
                 "kernel": "bem_boundary_matrices_vk (regular_strip_vk_kernel + touching + memset, timed as one stage), "
-                          f"63 flop x {n_eval:.4e} ordered regular quadrature-point pairs per launch (the kernel "
-                          "evaluates each unordered pair once, and the rule's symmetry takes it fewer operations "
-                          "than these); peak = nominal FP32 (SMs x 128 FMA x 2 x max SM "
+                          f"37 FP32 pipe operations (2 flop each, as the peak counts an FMA) x {n_eval / 2:.4e} "
+                          "unordered regular quadrature-point pairs per launch, as the kernel executes them; "
+                          "peak = nominal FP32 (SMs x 128 FMA x 2 x max SM "
                           "clock; no measured FP32 peak available); traffic scaled from an s5 ncu capture"}
 
     # ---- roofline of the solve's dominant kernel (tensor-core matvec) ----------

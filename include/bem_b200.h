@@ -92,9 +92,9 @@ int bem_geometry_build(const float* vertices, int nv, const int* triangles, int 
 /* Copies the per-triangle unit normals (nt,3) and surface curls (nt,3,3)
  * (rows b: n x grad phi_b), solver.py:40-58.  Either output may be NULL. */
 int bem_geometry_normals(const void* geom, float* normals, float* curls, bem_stream_t stream);
-/* BEM_OK, or BEM_ERR_CUDA if a bounded wait of an assembly kernel (the bulk
- * copies of trial tiles) expired while assembling on this geometry since the
- * last call; a matrix assembled meanwhile may be wrong.  The status word lives
+/* BEM_OK, or BEM_ERR_CUDA if a bounded wait of an assembly kernel or of the
+ * vertex gradient's (the bulk copies of trial triangles) expired on this geometry
+ * since the last call; a matrix or gradient computed meanwhile may be wrong.  The status word lives
  * in the geometry workspace (assembly kernels write it although the geometry
  * is passed as const); this call clears it and synchronises `stream`.  No
  * counterpart in the reference, whose kernels report no errors. */
@@ -129,8 +129,8 @@ int bem_boundary_matrices_vk(const void* geom, float k, void* v_out, void* k_out
 
 /* Batched fused assembly: many problems (meshes of any size, each with its
  * own wavenumber) in one persistent launch whose warps drain a single queue of
- * (problem, run of triangle pairs) work items, plus one launch
- * per touching-pair type over all problems.  `problems` is a HOST array;
+ * (problem, run of triangle pairs) work items, plus one launch for the
+ * touching pairs of all problems.  `problems` is a HOST array;
  * every v_out / k_out must be non-NULL (nv x nv complex64, overwritten with V
  * and mass_coeff M + k_coeff K).  Workspace: bem_batch_workspace_bytes.
  * No counterpart in the reference (one mesh, one wavenumber per call). */
@@ -228,7 +228,8 @@ int bem_potential_matrix(const void* geom, int layer, const float* points, int n
  *   out(:, s) = -S neumann(:, s) + D dirichlet(:, s),   s = 0..nrhs-1
  * (src/bem/solver.py:140-147).  neumann/dirichlet are (nv, nrhs) complex64
  * row-major (either may be NULL = zero); out is (np, nrhs) complex64,
- * overwritten.  scratch: bem_boundary2potential_scratch_bytes() bytes. */
+ * overwritten.  scratch: bem_boundary2potential_scratch_bytes() bytes, still
+ * required although the sums stay in registers and shared memory. */
 size_t bem_boundary2potential_scratch_bytes(int nt, int nrhs);
 int bem_boundary2potential(const void* geom, const float* points, int np, float k, const void* neumann,
                            const void* dirichlet, int nrhs, void* out, void* scratch,

@@ -10,8 +10,9 @@ batch runner changes how the work reaches the GPU:
 * the assembly of a whole wave is ONE persistent launch of the regular-pair
   kernel (its warps drain a single queue of (problem, run of triangle
   pairs) items, so a 320-triangle mesh and a 20 480-triangle mesh share the GPU
-  without launch-per-problem overhead) plus one launch per touching-pair
-  type (``bem_batch_matrices_vk``);
+  without launch-per-problem overhead) plus one launch for the touching pairs
+  (``bem_batch_matrices_vk``; one per type of them in
+  ``bem_batch_matrices_bm``);
 * the solves of a wave run concurrently, one CUDA stream per worker thread,
   each Arnoldi step replayed from a captured CUDA graph; the concurrency
   follows the problem size (a 10k-unknown solve already keeps every SM busy,

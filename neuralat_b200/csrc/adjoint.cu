@@ -33,17 +33,6 @@ int geom_view(const void* geom, GeomView* v, GeomHeader* out_hdr);
 
 namespace {
 
-template <typename R>
-__device__ __forceinline__ void sincos_a(R x, R* s, R* c);
-template <>
-__device__ __forceinline__ void sincos_a<double>(double x, double* s, double* c) {
-  sincos(x, s, c);
-}
-template <>
-__device__ __forceinline__ void sincos_a<float>(float x, float* s, float* c) {
-  sincosf(x, s, c);
-}
-
 // sine and cosine of a phase k r in the regular pairs
 __device__ __forceinline__ void sincos_phase(float x, float* s, float* c) { __sincosf(x, s, c); }
 
@@ -51,42 +40,37 @@ __device__ __forceinline__ void sincos_phase(float x, float* s, float* c) { __si
 //   F  += Re(a (bV G + bK K))
 //   gy += grad_y Re(...)     (grad_x is its negative)
 //   gn += grad_n Re(...)
-template <typename R>
-__device__ __forceinline__ void point_grad(const R d[3], const R n[3], R k, R ar, R ai, R bvr, R bvi, R bkr, R bki,
-                                           R W, R& F, R gy[3], R gn[3]) {
-  R r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-  const bool clamped = r < R(kEps);
-  if (clamped) r = R(kEps);
-  const R u = R(1) / r;
-  R s, c;
-  sincos_a<R>(k * r, &s, &c);
-  const R Gr = u * c, Gi = u * s;                                     // G (without 1/4pi)
-  const R Gpr = u * (-u * c - k * s), Gpi = u * (-u * s + k * c);     // G'
-  const R fr = Gpr * u, fi = Gpi * u;                                 // f = G'/r
-  const R t1 = R(2) * u * u - k * k, t2 = R(-2) * k * u;
-  const R Gppr = Gr * t1 - Gi * t2, Gppi = Gr * t2 + Gi * t1;         // G''
-  const R fpr = (Gppr - Gpr * u) * u, fpi = (Gppi - Gpi * u) * u;     // f'
-  const R dn = d[0] * n[0] + d[1] * n[1] + d[2] * n[2];
-  const R aVr = ar * bvr - ai * bvi, aVi = ar * bvi + ai * bvr;       // a bV
-  const R aKr = ar * bkr - ai * bki, aKi = ar * bki + ai * bkr;       // a bK
-  const R ReG = aVr * Gr - aVi * Gi;
-  const R ReK = (aKr * fr - aKi * fi) * dn;
+__device__ __forceinline__ void point_grad(const float d[3], const float n[3], float k, float ar, float ai, float bvr,
+                                           float bvi, float bkr, float bki, float W, float& F, float gy[3],
+                                           float gn[3]) {
+  float r = sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+  const bool clamped = r < kEps;
+  if (clamped) r = kEps;
+  const float u = 1.f / r;
+  float s, c;
+  sincosf(k * r, &s, &c);
+  const float Gr = u * c, Gi = u * s;                                     // G (without 1/4pi)
+  const float Gpr = u * (-u * c - k * s), Gpi = u * (-u * s + k * c);     // G'
+  const float fr = Gpr * u, fi = Gpi * u;                                 // f = G'/r
+  const float t1 = 2.f * u * u - k * k, t2 = -2.f * k * u;
+  const float Gppr = Gr * t1 - Gi * t2, Gppi = Gr * t2 + Gi * t1;         // G''
+  const float fpr = (Gppr - Gpr * u) * u, fpi = (Gppi - Gpi * u) * u;     // f'
+  const float dn = d[0] * n[0] + d[1] * n[1] + d[2] * n[2];
+  const float aVr = ar * bvr - ai * bvi, aVi = ar * bvi + ai * bvr;       // a bV
+  const float aKr = ar * bkr - ai * bki, aKi = ar * bki + ai * bkr;       // a bK
+  const float ReG = aVr * Gr - aVi * Gi;
+  const float ReK = (aKr * fr - aKi * fi) * dn;
   F += W * (ReG + ReK);
-  const R ReAVf = clamped ? R(0) : (aVr * fr - aVi * fi);
-  const R ReAKfp = clamped ? R(0) : (aKr * fpr - aKi * fpi);
-  const R c1 = W * (ReAVf + ReAKfp * dn * u);
-  const R c2 = W * (aKr * fr - aKi * fi);
+  const float ReAVf = clamped ? 0.f : (aVr * fr - aVi * fi);
+  const float ReAKfp = clamped ? 0.f : (aKr * fpr - aKi * fpi);
+  const float c1 = W * (ReAVf + ReAKfp * dn * u);
+  const float c2 = W * (aKr * fr - aKi * fi);
 #pragma unroll
   for (int e = 0; e < 3; e++) {
     gy[e] += c1 * d[e] + c2 * n[e];
     gn[e] += c2 * d[e];
   }
 }
-
-template <typename R>
-struct V3R {
-  R x[3];
-};
 
 // d(area)/d(v_c) = 1/2 n x (v_{c+2} - v_{c+1});   normal chain:
 // d(E)/d(v_c) += (v_{c+1} - v_{c+2}) x t,  t = (I - n n^T) dE/dn / |c|.
@@ -141,8 +125,11 @@ __device__ __forceinline__ double2 lerp3(const float2* vec, int v0, int v1, int 
 //
 // Bound by the FP32 pipe: about 64 operations per unordered point pair, on
 // packed pairs (the two points of a trial vertex).  Measured on B200 with 5120
-// triangles: 1.44 ms, against 12.0 ms for ordered pairs with the densities
-// interpolated in FP64 for every pair and library sincos calls.
+// triangles: 1.43 ms (FP32 pipe 71 % of its cycles), against 12.0 ms for ordered
+// pairs with the densities interpolated in FP64 for every pair and library sincos
+// calls.  Vertex gradients, 300 to 8000 triangles at 130 to 1300 Hz, are 0.1 to
+// 0.7 times as far off 64 bits as those (FP64 sums over the blocks outweigh the
+// hardware's sincos).
 // ---------------------------------------------------------------------------
 constexpr int kAdjThreads = 128;
 constexpr int kAdjWarps = kAdjThreads / 32;
@@ -768,7 +755,7 @@ __global__ void grad_listener_kernel(GeomView g, float k, const float* __restric
       const float d[3] = {rj.qp[3 * q] - x0, rj.qp[3 * q + 1] - x1, rj.qp[3 * q + 2] - x2};
       float gy[3] = {0, 0, 0};
       const float W = rj.area * kInv4Pi * (float)tri6_w(q);
-      point_grad<float>(d, n, k, ar, ai, bvr[q], bvi[q], bkr[q], bki[q], W, F, gy, N);
+      point_grad(d, n, k, ar, ai, bvr[q], bvi[q], bkr[q], bki[q], W, F, gy, N);
 #pragma unroll
       for (int e = 0; e < 3; e++) U[q][e] += gy[e];
     }

@@ -313,12 +313,12 @@ __global__ void __launch_bounds__(kRegThreads, 2)
 // runs on packed pairs (the two points of a trial vertex): the same rounding
 // as scalar operations in fewer issued instructions.
 //
-// Measured on B200 with 20 480 triangles: 12.8 ms (both operators; FP32 pipe
-// 61 % of its cycles, issue 61 %), of which 1.6 ms are the column reductions,
+// Measured on B200 with 20 480 triangles: 12.6 ms (both operators; FP32 pipe
+// 64 % of its cycles, issue 63 %), of which 1.6 ms are the column reductions,
 // against 19.0 ms for 16 x 16-triangle tiles whose 3 x 3 blocks all went
 // through shared memory between block barriers.  Two CTAs of four warps per SM
-// with everything unrolled (no spills) take 14.6 ms for the whole assembly,
-// three CTAs at 168 registers 15.1 ms, four at 128 registers 18.2 ms (spills).
+// with everything unrolled (no spills) took 14.6 ms for the whole assembly with
+// one item per warp (13.5 in rounds), three CTAs at 168 registers 15.1 ms, four at 128 registers 18.2 ms (spills).
 // ---------------------------------------------------------------------------
 constexpr float kRho = (float)(tri6_w_own(3) / tri6_w_own(0));
 constexpr float kSigma = (float)(tri6_w_common(3) / tri6_w_common(0));
