@@ -218,7 +218,7 @@ int cgemm_part(const float2* A, int n, const float2* X, int m, int first, int gr
       cfg.gridDim = dim3(1, (unsigned)c, 1);
       if (cudaOccupancyMaxActiveClusters(&k, cgemm_kernel<TM, PAIRS>, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        k = 0;
+        return 0;
       }
       if (k < 1) k = -1;  // none
       known.store(k, std::memory_order_relaxed);
@@ -229,9 +229,9 @@ int cgemm_part(const float2* A, int n, const float2* X, int m, int first, int gr
   // CTA's start and end cost about 48 columns), at most 1024 columns per CTA, at
   // least 1024 per cluster.
   const long long rows = (n + Sh::kRows - 1) / Sh::kRows;
-  int best = (n + 4095) / 4096 * 4, ctas = 4;
+  int best = (n + 1023) / 1024, ctas = 1;
   long long cost = 0;
-  for (int cuts = best; 128 * cuts <= n; cuts += 4)
+  for (int cuts = (best + 3) / 4 * 4; 128 * cuts <= n; cuts += 4)
     for (int c = 4; c <= 8; c *= 2) {
       if (cuts % c || 1024LL * cuts > (long long)c * n) continue;
       const long long fits = places(c);

@@ -524,13 +524,15 @@ int listen_launch(Kernel kernel, int groups, int nt, int sms, int per_sm, int le
     if (n == 0) {
       cfg.gridDim = dim3(1, (unsigned)r.cluster, 1);
       BEM_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
-      if (n < 1) return BEM_ERR_CUDA;
+      if (n < 1) n = -1;  // none of this size
       known.store(n, std::memory_order_relaxed);
     }
-    const int c = r.cluster;
-    r = listen_runs(groups, nt, (long long)n * c, least);
+    const int c = n > 0 ? r.cluster : 1;
+    if (n > 0) r = listen_runs(groups, nt, (long long)n * c, least);
     r.cluster = c;
     r.parts = (r.parts + c - 1) / c * c;  // the last runs may be empty
+    at[0].val.clusterDim.y = (unsigned)c;
+    cfg.numAttrs = c > 1 ? 1 : 0;
   }
   cfg.gridDim = dim3((unsigned)groups, (unsigned)r.parts, 1);
   BEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args..., r.run));
